@@ -162,8 +162,9 @@ int lfts_step_fwd_noalloc(const lfts_params *p, const double *q_in, double *q_ou
 /* ---- timing / integration helpers -------------------------------------- */
 /* The CUDA stream every call of this context runs on (a cudaStream_t). */
 void *lfts_stream(lfts_ctx *ctx);
-/* Time the contour chain of one calc_concs: mean ms of a yz-plane step
- * kernel and of an x-pencil kernel (one stream, events around every launch),
+/* Time the contour chain of one calc_concs: mean ms per contour step spent in
+ * kernels over yz planes (y and z lines) and in kernels over x lines (one
+ * stream, events around every launch; by 3-D transforms: of one such kernel),
  * and ms of the whole production chain (leaves the current fields' propagators). */
 int lfts_profile_chain(lfts_ctx *ctx, double *ms_plane, double *ms_pencil, double *ms_chain);
 /* Mean ms over `reps` back-to-back runs of each part of one Anderson
@@ -175,31 +176,35 @@ int lfts_profile_chain(lfts_ctx *ctx, double *ms_plane, double *ms_pencil, doubl
 int lfts_profile_iteration(lfts_ctx *ctx, int reps, double *ms_chain, double *ms_concs, double *ms_update);
 /* Number of kernels this context has launched so far. */
 long long lfts_kernel_launches(const lfts_ctx *ctx);
-/* The free choices of a context's contour chain.  None changes what is
- * computed: pencil_cw changes no value at all, the others change FP32-mixed
- * results only within that path's stated error (and FP64 ones not at all:
- * two_streams only reorders independent launches). */
+/* The free choices of a context's contour chain.  A context applies the bond
+ * one axis at a time; lfts_create picks its pencil_cw, two_streams and
+ * phi_in_chain by timing.  FP64: these change no value at all.  FP32-mixed: a
+ * choice installed by lfts_set_tiles selects the chain by 3-D transforms, the
+ * one that ensemble replicas run, with these tiles; its results agree with
+ * the axis-by-axis chain's within that path's stated error. */
 typedef struct lfts_tiles {
-    int pencil_cw;     /* x-pencil columns per CTA: 8, 16 or 32 */
-    int plane_stages;  /* yz-plane transform stages per axis: 2, or 3 (FP32-mixed, 64/96/128 square planes) */
-    int h_in_pencil;   /* FP32-mixed: h and the propagator stores in the x-pencil kernel and g in the
+    int pencil_cw;     /* columns per CTA of the x kernels (and y, axis by axis): 8, 16 or 32 */
+    int plane_stages;  /* 3-D transforms: yz-plane transform stages per axis: 2, or 3 (FP32-mixed, 64/96/128 square
+                          planes) */
+    int h_in_pencil;   /* 3-D transforms: h and the propagator stores in the x-pencil kernel and g in the
                           yz-plane kernel (1; 96- and 128-point x lines, 3 stages), or all in the yz-plane (0) */
     int two_streams;   /* FP64: each chain on its own stream (1) or both chains in every launch (0) */
-    int phi_in_chain;  /* with h_in_pencil: the concentration sums formed in the x-pencil from the
-                          middle of the chain on (each new slot times its already stored partner,
+    int phi_in_chain;  /* with h_in_pencil: the concentration sums formed in the chain from its
+                          middle on (each new slot times its already stored partner,
                           FP32 sums; the later slots are then not stored) (1), or by a separate
                           pass over all N stored slots (0) */
-    int plane_split;   /* FP32-mixed 128 x 128 planes with h_in_pencil: CTAs per x-plane in the yz-plane
-                          kernel, 8 (the plane split over a thread-block cluster, its transposes through
+    int plane_split;   /* 3-D transforms, FP32-mixed 128 x 128 planes with h_in_pencil: CTAs per x-plane in the
+                          yz-plane kernel, 8 (the plane split over a thread-block cluster, its transposes through
                           distributed shared memory; bitwise the same values) or 1; 0 reads as 1 */
 } lfts_tiles;
 /* lfts_create picks the tiles by timing the whole contour chain for every
- * valid combination on the context's own buffers and keeping the fastest,
- * once per precision and mesh in a process (the counterpart of the
- * reference's FFTW_PATIENT planning, src/step.cc:15-16).  Environment:
- * LFTS_AUTOTUNE=0 skips the timing (built-in choice); LFTS_PENCIL_CW=8|16|32,
- * LFTS_XH_CHAIN=0|1, LFTS_PHI_IN_CHAIN=0|1, LFTS_PLANE_SPLIT=1|8 and
- * LFTS_ONE_STREAM=1 fix one choice each. */
+ * combination on the context's own buffers and keeping the fastest, once per
+ * precision and mesh in a process (the counterpart of the reference's
+ * FFTW_PATIENT planning, src/step.cc:15-16); lfts_get_tiles gives them, with
+ * plane_stages, h_in_pencil and plane_split of a transform chain that has such
+ * tiles.  Environment: LFTS_AUTOTUNE=0 skips the timing (built-in choice);
+ * LFTS_PENCIL_CW=8|16|32, LFTS_PHI_IN_CHAIN=0|1 and LFTS_ONE_STREAM=1 fix one
+ * choice each, LFTS_XH_CHAIN=0 leaves the sums to the separate pass. */
 int lfts_get_tiles(const lfts_ctx *ctx, lfts_tiles *out);
 /* Installs a tile choice (LFTS_ERR_ARG / LFTS_ERR_UNSUPPORTED for an
  * invalid one), e.g. to make a context compute exactly what an ensemble

@@ -1,0 +1,35 @@
+// The compiled axis kernels (axis_conv.cuh) of one mesh, looked up by size:
+// axis_fp64.cu and axis_fp32.cu instantiate them.
+#pragma once
+#include "axis_conv.cuh"
+
+namespace lfts {
+
+template <typename T>
+struct AxisFn {
+    void (*fn)(AxisArgs<T>);  // null: not compiled
+    int nt;
+    size_t smem;
+    int per;  // x, y: columns per CTA; z: lines per CTA; plane: 1 (the plane)
+};
+
+template <typename T>
+struct AxisSet {
+    AxisFn<T> x[kAxisModes], y, z[kAxisModes], plane[kAxisModes];
+    bool planes;  // [Cy Cz h Cz Cy] in one kernel; else z lines and y lines apart
+    int cw;
+};
+
+// fills *o for an mx x my x mz mesh with x and y tiles of cw columns (8, 16, 32);
+// false without kernels for it
+bool axis_kernels(int mx, int my, int mz, int cw, AxisSet<double> *o);
+bool axis_kernels(int mx, int my, int mz, int cw, AxisSet<float> *o);
+
+// Columns per CTA of the x-line kernel that ends a chain, whatever the tile
+// choice: its CTAs' partial sums for Q then do not depend on the tiles.
+constexpr int kLastCw = 16;
+
+// Whether y and z lines share a kernel, one CTA per x-plane.
+constexpr bool axis_planes(int my, int mz) { return my * mz <= 48 * 48; }
+
+}  // namespace lfts

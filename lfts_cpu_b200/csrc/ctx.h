@@ -7,10 +7,14 @@
 #include <cuda_runtime.h>
 
 #include "../../include/lfts_b200.h"
+#include "axis_dispatch.h"
 #include "fft_dispatch.h"
 #include "field_kernels.cuh"
 
 using namespace lfts;
+
+// most CTAs of a chain's last kernel (128 x 128 lines, 16 a CTA)
+constexpr int kMaxQparts = 4096;
 
 struct lfts_ctx {
     lfts_params p{};
@@ -27,10 +31,11 @@ struct lfts_ctx {
 
     double *w = nullptr;       // 4M: W-, w+, phi-, phi+
     void *q = nullptr;         // N slots x 2M, slot i at (i-1)*2M
-    void *spec = nullptr;      // 2 x mx x my x KZ complex
+    void *field = nullptr;     // the contour chain's field (2M); half spectra of the adjoint and FP64 S(k)
     void *tw[3] = {};          // exp(-2 pi i t/m) per dimension
     void *gtab[3] = {};        // gx[mx], gy[my], gz[KZ] (gz carries 1/M)
-    double *qpart = nullptr;   // mx per-plane sums of q_N
+    double *qpart = nullptr;   // per-CTA sums of q_N
+    unsigned *ticket = nullptr;  // CTAs of the chain's last kernel that are done
     double *Qd = nullptr;      // Q, ln Q
     double *partials = nullptr;
     double *red = nullptr;     // kRedWidth reduced values (device)
@@ -63,20 +68,23 @@ struct lfts_ctx {
     int adj_buf_slots = 0;
     AdjKernel adj{};
 
-    PlaneKernels<double> pl64{};
-    PencilKernels<double> pe64{};
+    AxisSet<double> ax64{};    // the contour chain's kernels (one of the two by precision)
+    AxisSet<float> ax32{};
+    PlaneKernel fwd_yz{};      // FP64 forward transforms: S(k), the adjoint
+    PencilKernel power_x{};
+    lfts_tiles tiles{};        // the choice in use
+    // FP32: the chain by 3-D transforms, once lfts_set_tiles asked for it
+    bool transform_chain = false;
     PlaneKernels<float> pl32{};
     PencilKernels<float> pe32{};
-    int plane_stages = 2;     // yz-plane transform stages per axis (3: fft_plane3.cuh)
     int plane_split = 1;      // CTAs per x-plane of PLANE_G (8: the cluster kernel, fft_plane3c.cuh)
     int pf_ctas = 0;          // PLANE_G ahead of a summing pencil: prefetching CTAs past the planes
     PlaneSplitKernel psplit{};
+    bool xh_chain = false;    // h and the q stores in the x-pencil (enqueue_transform_chain)
 
     bool fields_set = false;
     bool have_concs = false;
-    bool packed = false;      // FP32: both chains as one complex field (fft_packed.cuh)
-    bool xh_chain = false;    // FP32 128^3: h and the q stores in the x-pencil (enqueue_chain_launches)
-    bool phi_in_chain = false;  // with xh_chain: the concentration sums formed in the chain (PENCIL_HA)
+    bool phi_in_chain = false;  // FP32: the concentration sums formed in the chain (AX_HA)
     void *acc = nullptr;      // their (A, B) sums per mesh point, FP32 pairs
     bool use_graph = true;    // LFTS_NO_GRAPH=1: launch the chain kernel by kernel
     cudaGraph_t chain_graph = nullptr;

@@ -1,5 +1,6 @@
-// Lookup of the compiled FFT kernels by mesh size (one translation unit per
-// precision instantiates them: fft_fp64.cu, fft_fp32.cu).
+// Lookup of the compiled 3-D transform kernels by mesh size: FP64 forward
+// transforms (fft_fp64.cu: S(k) samples, the adjoint) and the FP32-mixed
+// transform chain (fft_fp32.cu).
 #pragma once
 #include <cstddef>
 
@@ -23,11 +24,17 @@ struct PencilKernels {
     int cw;
 };
 
-// false when (ny, nz) / nx has no compiled instantiation
-// packed-chain plane kernels (fft_packed.cuh), FP32
-bool plane_c_kernels(int ny, int nz, PlaneKernels<float> *out);
-// three-stage packed-chain plane kernels (fft_plane3.cuh), FP32: 64, 96, 128 square planes
-bool plane3_kernels(int ny, int nz, PlaneKernels<float> *out);
+struct PlaneKernel {
+    void (*fn)(PlaneArgs<double>);
+    int nt;
+    size_t smem;
+};
+struct PencilKernel {
+    void (*fn)(PencilArgs<double>);
+    int nt;
+    size_t smem;
+    int cw;
+};
 // PLANE_G with each x-plane split over a thread-block cluster of cl CTAs
 // (fft_plane3c.cuh), FP32: 128 x 128 planes
 struct PlaneSplitKernel {
@@ -35,22 +42,25 @@ struct PlaneSplitKernel {
     int cl, nt;
     size_t smem;
 };
-bool plane_split_kernel(int ny, int nz, PlaneSplitKernel *out);
-bool plane_kernels(int ny, int nz, PlaneKernels<double> *out);
-bool pencil_kernels(int nx, PencilKernels<double> *out);
-bool pencil_kernels(int nx, PencilKernels<float> *out);
-// x-pencil kernels of tile width cw (columns per CTA: 8, 16 or 32); the tile
-// width changes only the work split, not any column's arithmetic
-bool pencil_kernels(int nx, int cw, PencilKernels<double> *out);
-bool pencil_kernels(int nx, int cw, PencilKernels<float> *out);
 struct AdjKernel {
     void (*fn)(AdjArgs);
     int nt;
     size_t smem;
     int cw;
 };
-// adjoint x-pencil (FP64) for line length nx
+
+// false when (ny, nz) / nx has no compiled instantiation
+bool fwd_plane_kernel(int ny, int nz, PlaneKernel *out);
+bool power_pencil_kernel(int nx, PencilKernel *out);
 bool adjoint_kernel(int nx, AdjKernel *out);
+// packed-chain plane kernels (fft_packed.cuh), FP32
+bool plane_c_kernels(int ny, int nz, PlaneKernels<float> *out);
+// three-stage packed-chain plane kernels (fft_plane3.cuh), FP32: 64, 96, 128 square planes
+bool plane3_kernels(int ny, int nz, PlaneKernels<float> *out);
+bool plane_split_kernel(int ny, int nz, PlaneSplitKernel *out);
+// x-pencil kernels of tile width cw (columns per CTA: 8, 16 or 32), FP32; the
+// width changes only the work split, not any column's arithmetic
+bool pencil_kernels(int nx, int cw, PencilKernels<float> *out);
 
 // line lengths with a two-stage plan
 bool fft_length_supported(int n);

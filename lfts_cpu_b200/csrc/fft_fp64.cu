@@ -1,38 +1,35 @@
-// FP64 instantiations of the contour-step FFT kernels.
-#include "fft_inst.cuh"
+// FP64 forward-transform kernels: S(k) samples and the adjoint.
+#include "fft_dispatch.h"
+#include "fft_lengths.h"
 
-#define LFTS_PLANE_CASE_double(a, b) \
-    if (ny == a && nz == b) { fill_plane<double, a, b>(o); return true; }
-#define LFTS_PENCIL_CASE_double(a) \
-    if (nx == a) { fill_pencil<double, a>(o); return true; }
-#define LFTS_PENCIL_CW_CASE_double(a)                                   \
-    if (nx == a) {                                                   \
-        if (cw == 8) { fill_pencil<double, a, 8>(o); return true; }      \
-        if (cw == 16) { fill_pencil<double, a, 16>(o); return true; }    \
-        if (cw == 32) { fill_pencil<double, a, 32>(o); return true; }    \
-        return false;                                                \
+namespace lfts {
+
+bool fwd_plane_kernel(int ny, int nz, PlaneKernel *o)
+{
+#define LFTS_PLANE_CASE(a, b)                                                                  \
+    if (ny == a && nz == b) {                                                                  \
+        *o = {fwd_plane_kernel_t<a, b>, PlaneCfg<double, a, b>::NT, PlaneCfg<double, a, b>::SMEM}; \
+        return true;                                                                           \
     }
-LFTS_DEFINE_PLANE_DISPATCH(double)
-LFTS_DEFINE_DISPATCH(double)
-
-namespace lfts {
-bool fft_length_supported(int n)
-{
-#define LFTS_LEN_CASE(a) if (n == a) return true;
-    LFTS_FOR_EACH_LEN(LFTS_LEN_CASE)
-#undef LFTS_LEN_CASE
+    LFTS_FOR_EACH_PAIR(LFTS_PLANE_CASE)
+#undef LFTS_PLANE_CASE
     return false;
 }
-bool plane_pair_supported(int ny, int nz)
+
+bool power_pencil_kernel(int nx, PencilKernel *o)
 {
-#define LFTS_PAIR_CASE(a, b) if (ny == a && nz == b) return true;
-    LFTS_FOR_EACH_PAIR(LFTS_PAIR_CASE)
-#undef LFTS_PAIR_CASE
+    constexpr int CW = 32;
+#define LFTS_POWER_CASE(a)                                                                \
+    if (nx == a) {                                                                        \
+        using C = PencilCfg<double, a, CW>;                                               \
+        *o = {pencil_kernel<double, a, CW, PENCIL_POWER>, C::NT, C::SMEM, CW};            \
+        return true;                                                                      \
+    }
+    LFTS_FOR_EACH_LEN(LFTS_POWER_CASE)
+#undef LFTS_POWER_CASE
     return false;
 }
-}  // namespace lfts
 
-namespace lfts {
 bool adjoint_kernel(int nx, AdjKernel *o)
 {
     constexpr int CW = 16;
@@ -48,4 +45,20 @@ bool adjoint_kernel(int nx, AdjKernel *o)
 #undef LFTS_ADJ_CASE
     return false;
 }
+
+bool fft_length_supported(int n)
+{
+#define LFTS_LEN_CASE(a) if (n == a) return true;
+    LFTS_FOR_EACH_LEN(LFTS_LEN_CASE)
+#undef LFTS_LEN_CASE
+    return false;
+}
+bool plane_pair_supported(int ny, int nz)
+{
+#define LFTS_PAIR_CASE(a, b) if (ny == a && nz == b) return true;
+    LFTS_FOR_EACH_PAIR(LFTS_PAIR_CASE)
+#undef LFTS_PAIR_CASE
+    return false;
+}
+
 }  // namespace lfts

@@ -1,38 +1,36 @@
-// Fused contour-step kernels for sm_100a.
+// 3-D transform kernels for sm_100a.
 //
-// One contour step of the reference (step::fwd, src/step.cc:35-65) is
-//     q_{i+1} = h .* IFFT3( g .* FFT3(q_i) )
-// for two chains at once.  Here a 3-D transform is split into
-//   * a yz-plane pass (one CTA per x-plane per chain): inverse y, inverse z
-//     (complex-to-real), multiply by h, store q_{i+1}, forward z
-//     (real-to-complex), forward y -- i.e. the end of step i and the start of
-//     step i+1 fused, with the whole plane's half spectrum resident in shared
-//     memory (my x (mz/2+1) complex values);
-//   * an x-pencil pass (one CTA per tile of (ky,kz) columns per chain):
-//     forward x, multiply by g(k), inverse x.
+// FP64 forward transforms (S(k) samples, the adjoint), and the x-pencil of the
+// FP32-mixed transform chain, which the replica ensemble runs: one contour step
+// of the reference (step::fwd, src/step.cc:35-65) as q_{i+1} = h .* IFFT3( g .*
+// FFT3(q_i) ).  A 3-D transform is split into
+//   * a yz-plane pass (one CTA per x-plane per field) with the whole plane
+//     resident in shared memory: here the FP64 forward one, z (real-to-complex)
+//     then y; the chain's, inverse and forward with h between, are in
+//     fft_packed.cuh and fft_plane3.cuh;
+//   * an x-pencil pass (one CTA per tile of (ky,kz) columns): forward x, and in
+//     the chain g(k) (or h) and inverse x.
 // Each 1-D transform of length n = R1*R2 runs as two in-register radix
 // stages separated by one shared-memory exchange: stage "A" works on the
 // strided sets {j2 + R2 t}, stage "B" on the contiguous blocks {R2 k1 + u}.
 // Running A then B leaves the data "transposed" (index k1 + R1 k2 stored at
 // R2 k1 + k2); running B then A takes it back to natural order.  Every stage
 // therefore works in place, and the order in between is only ever seen by
-// code that knows the mapping (ymap below).
+// code that knows the mapping.
 //
-// Two real rows of a plane are packed into one complex line (a + i b) for
-// the z transforms; the half spectra are separated / recombined with the
-// Hermitian symmetry X[n-k] = conj X[k].  As in FFTW's c2r, the imaginary
-// parts of the k=0 and k=n/2 coefficients are ignored on the way back.
+// Two real rows of an FP64 plane are packed into one complex line (a + i b) for
+// the z transforms; the half spectra are separated with the Hermitian symmetry
+// X[n-k] = conj X[k].
 #pragma once
 #include "dft.cuh"
 
 namespace lfts {
 
-// Programmatic dependent launch: the chain's kernels are launched with
-// programmatic stream serialisation, so a kernel's CTAs may start while the
-// previous kernel drains.  Each kernel loads its constant tables first, then
-// waits for the previous grid's results (griddepcontrol.wait) before touching
-// the spectrum, h, q or w, and lets its dependent launch as soon as all of its
-// own CTAs are running.  Launched without the attribute, both are no-ops.
+// Programmatic dependent launch: the contour chain's kernels (axis_conv.cuh) are
+// launched with programmatic stream serialisation, so a kernel's CTAs may start
+// while the previous kernel drains.  Each kernel loads its constant tables
+// first, then waits for the previous grid's results (griddepcontrol.wait) before
+// touching the field, h, q or w.  Launched without the attribute, both are no-ops.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" :::); }
 // pull one 128-byte line into L2 (a hint: L2 is the point of coherence, so a
@@ -99,17 +97,8 @@ struct PlaneCfg {
     static constexpr size_t SMEM = sizeof(cpx<T>) * (size_t)(NY * KZP + 2 * NY + NTA + NTB);
     static __device__ __forceinline__ int ta(int j2, int k1) { return j2 * TAP + k1; }
     static __device__ __forceinline__ int tb(int k1, int u) { return k1 * TBP + u; }
-    // resident CTAs per SM the register budget is sized for (FP32 planes are
-    // small enough for two)
-    static constexpr int MINB = (sizeof(T) == 4 && 2 * SMEM < 200 * 1024 && NT <= 512) ? 2 : 1;
     static_assert(NZ % 2 == 0 && NY % 2 == 0, "plane kernels need even my and mz");
-    static __device__ __forceinline__ int ymap(int p) { return p / RY2 + RY1 * (p % RY2); }
     static __device__ __forceinline__ int zpos(int s) { return s + s / RZ2; }
-};
-
-template <int TASKS, int NT>
-struct Tpt {
-    static constexpr int v = (TASKS + NT - 1) / NT;
 };
 
 // The z-line phases are warp-local: warp w owns row pairs
@@ -129,60 +118,6 @@ struct WarpPairs {
 };
 
 // ---------------------------------------------------------------- y phases --
-// inverse, natural -> transposed, stage A reading the global half spectrum.
-// KC * RY2 <= NT, so every thread has at most one task; the loads are issued
-// by y_invA_load (before the barrier that publishes the twiddle tables) and
-// consumed by y_invA_finish.
-template <typename C, typename T>
-__device__ __forceinline__ void y_invA_load(const cpx<T> *__restrict__ Sg, cpx<T> (&v)[C::RY1])
-{
-    constexpr int KZ = C::KZ, KC = C::KC, R1 = C::RY1, R2 = C::RY2;
-    static_assert(KC * R2 <= C::NT, "one stage-A task per thread");
-    const int t = threadIdx.x;
-    if (t < KC * R2) {
-        const int col = t % KC, j2 = t / KC;
-#pragma unroll
-        for (int a = 0; a < R1; a++) {
-            v[a] = Sg[(j2 + R2 * a) * KZ + col];
-            if (col == 0) {  // Y0 + i Y_{NZ/2}
-                const cpx<T> n2 = Sg[(j2 + R2 * a) * KZ + KC];
-                v[a] = {v[a].x - n2.y, v[a].y + n2.x};
-            }
-        }
-    }
-}
-
-template <typename C, typename T>
-__device__ __forceinline__ void y_invA_finish(cpx<T> *P, cpx<T> (&v)[C::RY1], const cpx<T> *twy)
-{
-    constexpr int KC = C::KC, KZP = C::KZP, R1 = C::RY1, R2 = C::RY2, NY = R1 * R2;
-    const int t = threadIdx.x;
-    if (t < KC * R2) {
-        const int col = t % KC, j2 = t / KC;
-        Dft<R1, 1, T>::run(v);
-#pragma unroll
-        for (int k1 = 0; k1 < R1; k1++)
-            P[(j2 + R2 * k1) * KZP + col] = ctw<1>(v[k1], twy[(j2 * k1) % NY]);
-    }
-}
-
-// stage B in place with sign S; TW: apply exp(S 2pi i j2 k1/n) after the DFT
-template <typename C, int S, bool TW, typename T>
-__device__ __forceinline__ void y_B(cpx<T> *P, const cpx<T> *twy)
-{
-    constexpr int KC = C::KC, KZP = C::KZP, R1 = C::RY1, R2 = C::RY2, NY = R1 * R2;
-    for (int t = threadIdx.x; t < KC * R1; t += C::NT) {
-        const int col = t % KC, k1 = t / KC;
-        cpx<T> v[R2];
-#pragma unroll
-        for (int u = 0; u < R2; u++) v[u] = P[(R2 * k1 + u) * KZP + col];
-        Dft<R2, S, T>::run(v);
-#pragma unroll
-        for (int u = 0; u < R2; u++)
-            P[(R2 * k1 + u) * KZP + col] = TW ? ctw<S>(v[u], twy[(u * k1) % NY]) : v[u];
-    }
-}
-
 // forward, stage A in smem with twiddles (natural -> transposed start)
 template <typename C, typename T>
 __device__ __forceinline__ void y_fwdA_tw(cpx<T> *P, const cpx<T> *twy)
@@ -221,27 +156,6 @@ __device__ __forceinline__ void y_fwdB_global(const cpx<T> *P, cpx<T> *__restric
     }
 }
 
-// forward stage A -> global, natural order (end of transposed -> natural forward)
-template <typename C, typename T>
-__device__ __forceinline__ void y_fwdA_global(const cpx<T> *P, cpx<T> *__restrict__ Sg, cpx<T> *colbuf)
-{
-    constexpr int KZ = C::KZ, KC = C::KC, KZP = C::KZP, R1 = C::RY1, R2 = C::RY2;
-    for (int t = threadIdx.x; t < KC * R2; t += C::NT) {
-        const int col = t % KC, j2 = t / KC;
-        cpx<T> v[R1];
-#pragma unroll
-        for (int k1 = 0; k1 < R1; k1++) v[k1] = P[(j2 + R2 * k1) * KZP + col];
-        Dft<R1, -1, T>::run(v);
-#pragma unroll
-        for (int j1 = 0; j1 < R1; j1++) {
-            if (col == 0)
-                colbuf[j2 + R2 * j1] = v[j1];
-            else
-                Sg[(j2 + R2 * j1) * KZ + col] = v[j1];
-        }
-    }
-}
-
 // Separate the packed column Y = Y0 + i Y_{NZ/2} (natural ky order in colbuf)
 // into the kz = 0 and kz = NZ/2 columns of the global half spectrum.
 template <typename C, typename T>
@@ -258,137 +172,6 @@ __device__ __forceinline__ void y_unpack0(const cpx<T> *colbuf, cpx<T> *__restri
 // ---------------------------------------------------------------- z phases --
 // Row pair q occupies the 2*KZP slots starting at P + 2q*KZP ("region");
 // the packed line's slot s lives at region[zpos(s)], the rows' k at row[k].
-
-// Build Z = A + iB (Hermitian-extended) and run inverse stage A.  Permuting
-// inside each pair region: the warp reads everything before __syncwarp, then
-// writes.
-template <typename C, typename T>
-__device__ __forceinline__ void z_build_invA(cpx<T> *P, const cpx<T> *twa)
-{
-    using WP = WarpPairs<C>;
-    constexpr int KZP = C::KZP, R1 = C::RZ1, R2 = C::RZ2, NZ = R1 * R2;
-    constexpr int RND = WP::template Rounds<R2>::v;
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int q0 = WP::first(w), ntask = WP::count(w) * R2;
-    cpx<T> hold[RND][R1];
-#pragma unroll
-    for (int s = 0; s < RND; s++) {
-        const int t = lane + 32 * s;
-        if (t < ntask) {
-            const int q = q0 + t / R2, j2 = t % R2;
-            const cpx<T> *A = P + 2 * q * KZP, *B = A + KZP;
-#pragma unroll
-            for (int a = 0; a < R1; a++) {
-                const int k = j2 + R2 * a;
-                cpx<T> z;
-                if (k == 0) {
-                    z = {A[0].x, B[0].x};
-                } else if (2 * k == NZ) {
-                    z = {A[0].y, B[0].y};  // packed kz = NZ/2 (real part only, as c2r)
-                } else if (2 * k < NZ) {
-                    const cpx<T> av = A[k], bv = B[k];
-                    z = {av.x - bv.y, av.y + bv.x};
-                } else {
-                    const cpx<T> av = A[NZ - k], bv = B[NZ - k];
-                    z = {av.x + bv.y, bv.x - av.y};
-                }
-                hold[s][a] = z;
-            }
-            Dft<R1, 1, T>::run(hold[s]);
-#pragma unroll
-            for (int k1 = 0; k1 < R1; k1++) hold[s][k1] = ctw<1>(hold[s][k1], twa[C::ta(j2, k1)]);
-        }
-    }
-    __syncwarp();
-#pragma unroll
-    for (int s = 0; s < RND; s++) {
-        const int t = lane + 32 * s;
-        if (t < ntask) {
-            const int q = q0 + t / R2, j2 = t % R2;
-            cpx<T> *Z = P + 2 * q * KZP;
-#pragma unroll
-            for (int k1 = 0; k1 < R1; k1++) Z[C::zpos(j2 + R2 * k1)] = hold[s][k1];
-        }
-    }
-}
-
-// Inverse stage B -> real rows (transposed z order), times h, store q;
-// STEP: then forward stage B with twiddles back into smem.
-// LAST: accumulate chain-0 values into *qsum instead.
-// All of a lane's h values are loaded before its first task (they do not
-// depend on shared memory), and q goes out with evict-first stores: it is
-// read again only by the concentration pass.
-template <typename C, int MODE, typename T>
-__device__ __forceinline__ void z_invB_h(cpx<T> *P, const cpx<T> *twb, const T *__restrict__ h,
-                                         T *__restrict__ qrow, double &qsum)
-{
-    using WP = WarpPairs<C>;
-    constexpr int KZP = C::KZP, R1 = C::RZ1, R2 = C::RZ2, NZ = R1 * R2;
-    constexpr int RND = WP::template Rounds<R1>::v;
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int q0 = WP::first(w), ntask = WP::count(w) * R1;
-    T hv[RND][R2][2];
-#pragma unroll
-    for (int s = 0; s < RND; s++) {
-        const int t = lane + 32 * s;
-        if (t < ntask) {
-            const int q = q0 + t / R1, k1 = t % R1;
-            const int ya = C::ymap(2 * q), yb = C::ymap(2 * q + 1);
-#pragma unroll
-            for (int k2 = 0; k2 < R2; k2++) {
-                hv[s][k2][0] = __ldg(h + ya * NZ + k1 + R1 * k2);
-                hv[s][k2][1] = __ldg(h + yb * NZ + k1 + R1 * k2);
-            }
-        }
-    }
-#pragma unroll
-    for (int s = 0; s < RND; s++) {
-        const int t = lane + 32 * s;
-        if (t >= ntask) continue;
-        const int q = q0 + t / R1, k1 = t % R1;
-        cpx<T> *Z = P + 2 * q * KZP;
-        const int ya = C::ymap(2 * q), yb = C::ymap(2 * q + 1);
-        cpx<T> v[R2];
-#pragma unroll
-        for (int u = 0; u < R2; u++) v[u] = Z[C::zpos(R2 * k1 + u)];
-        Dft<R2, 1, T>::run(v);
-#pragma unroll
-        for (int k2 = 0; k2 < R2; k2++) {
-            const int z = k1 + R1 * k2;
-            const T a = v[k2].x * hv[s][k2][0];
-            const T b = v[k2].y * hv[s][k2][1];
-            __stcs(qrow + ya * NZ + z, a);
-            __stcs(qrow + yb * NZ + z, b);
-            if (MODE == PLANE_LAST) qsum += (double)a + (double)b;
-            v[k2] = {a, b};
-        }
-        if (MODE == PLANE_STEP) {
-            Dft<R2, -1, T>::run(v);
-#pragma unroll
-            for (int u = 0; u < R2; u++) Z[C::zpos(R2 * k1 + u)] = ctw<-1>(v[u], twb[C::tb(k1, u)]);
-        }
-    }
-}
-
-// forward stage A, transposed -> natural, in place
-template <typename C, typename T>
-__device__ __forceinline__ void z_fwdA(cpx<T> *P)
-{
-    using WP = WarpPairs<C>;
-    constexpr int KZP = C::KZP, R1 = C::RZ1, R2 = C::RZ2;
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int q0 = WP::first(w), ntask = WP::count(w) * R2;
-    for (int t = lane; t < ntask; t += 32) {
-        const int q = q0 + t / R2, j2 = t % R2;
-        cpx<T> *Z = P + 2 * q * KZP;
-        cpx<T> v[R1];
-#pragma unroll
-        for (int k1 = 0; k1 < R1; k1++) v[k1] = Z[C::zpos(j2 + R2 * k1)];
-        Dft<R1, -1, T>::run(v);
-#pragma unroll
-        for (int j1 = 0; j1 < R1; j1++) Z[C::zpos(j2 + R2 * j1)] = v[j1];
-    }
-}
 
 // forward stage A with twiddles, natural -> (start of) transposed, in place
 template <typename C, typename T>
@@ -430,9 +213,9 @@ __device__ __forceinline__ void z_fwdB(cpx<T> *P)
     }
 }
 
-// Separate the packed spectrum Z of rows (a, b) into the half spectra A, B.
-// TRANSPOSED: Z[k] sits at R2*(k % R1) + k / R1, else at k.  Permuting.
-template <typename C, bool TRANSPOSED, typename T>
+// Separate the packed spectrum Z of rows (a, b), Z[k] at R2*(k % R1) + k / R1,
+// into the half spectra A, B.  Permuting.
+template <typename C, typename T>
 __device__ __forceinline__ void z_unpack(cpx<T> *P)
 {
     using WP = WarpPairs<C>;
@@ -448,8 +231,8 @@ __device__ __forceinline__ void z_unpack(cpx<T> *P)
             const int q = q0 + t / KC, k = t % KC;
             const int nk = (k == 0) ? NZ / 2 : NZ - k;  // k = 0 pairs DC with Nyquist
             const cpx<T> *Z = P + 2 * q * KZP;
-            const int pk = TRANSPOSED ? R2 * (k % R1) + k / R1 : k;
-            const int pn = TRANSPOSED ? R2 * (nk % R1) + nk / R1 : nk;
+            const int pk = R2 * (k % R1) + k / R1;
+            const int pn = R2 * (nk % R1) + nk / R1;
             const cpx<T> z = Z[C::zpos(pk)], c = Z[C::zpos(pn)];
             if (k == 0) {
                 // A[0], A[NZ/2], B[0], B[NZ/2] are real: A = Re Z, B = Im Z
@@ -472,12 +255,6 @@ __device__ __forceinline__ void z_unpack(cpx<T> *P)
             P[(2 * q + 1) * KZP + k] = hb[s];
         }
     }
-}
-
-template <typename C, typename T>
-__device__ __forceinline__ void load_tw(cpx<T> *dst, const cpx<T> *__restrict__ src, int n)
-{
-    for (int t = threadIdx.x; t < n; t += C::NT) dst[t] = src[t];
 }
 
 // Both twiddle tables through registers: the global loads go out first (before
@@ -523,132 +300,47 @@ struct TwStage {
     }
 };
 
-// Pull this warp's h rows (used by z_invB_h) towards L1 while the z section
-// starts: one prefetch per 128-byte line.
-template <typename C, typename T>
-__device__ __forceinline__ void prefetch_h_rows(const T *__restrict__ h)
-{
-    using WP = WarpPairs<C>;
-    constexpr int NZ = C::RZ1 * C::RZ2;
-    constexpr int LINES_PER_ROW = (NZ * (int)sizeof(T) + 127) / 128;
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int q0 = WP::first(w), nrows = 2 * WP::count(w);
-    for (int t = lane; t < nrows * LINES_PER_ROW; t += 32) {
-        const int row = t / LINES_PER_ROW, line = t % LINES_PER_ROW;
-        const int p = 2 * q0 + row;
-        const char *addr = reinterpret_cast<const char *>(h + C::ymap(p) * NZ) + 128 * line;
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(addr));
-    }
-}
-
 // ------------------------------------------------------------ plane kernel --
-template <typename T, int NY, int NZ, int MODE>
-__global__ void __launch_bounds__(PlaneCfg<T, NY, NZ>::NT, PlaneCfg<T, NY, NZ>::MINB) plane_kernel(PlaneArgs<T> a)
+template <int NY, int NZ>
+__global__ void __launch_bounds__(PlaneCfg<double, NY, NZ>::NT) fwd_plane_kernel_t(PlaneArgs<double> a)
 {
+    using T = double;
     using C = PlaneCfg<T, NY, NZ>;
     constexpr int KZ = C::KZ, KZP = C::KZP;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cpx<T> *P = reinterpret_cast<cpx<T> *>(smem_raw);
     cpx<T> *twy = P + NY * KZP;
     cpx<T> *twa = twy + NY;            // TA: stage-A z twiddles
-    cpx<T> *twb = twa + C::NTA;        // TB: stage-B z twiddles
-    cpx<T> *colbuf = twb + C::NTB;
+    cpx<T> *colbuf = twa + C::NTA + C::NTB;
 
-    const int x = blockIdx.x, c = blockIdx.y + a.cbase;
+    const int x = blockIdx.x, c = blockIdx.y;
     const int mx = gridDim.x;
-    const long long M = (long long)mx * NY * NZ;
     const long long plane_off = (long long)x * NY * NZ;
     cpx<T> *Sg = a.spec + ((long long)c * mx + x) * NY * KZ;
 
     TwStage<C, T> tws;
     tws.load(a.twy, a.twz);
-    pdl_launch_dependents();
-    pdl_wait();
-
-    if (MODE == PLANE_INIT_W || MODE == PLANE_INIT_Q) {
-        // real rows (natural y order), packed two per complex line; the whole
-        // z section is warp-local (see WarpPairs)
-        tws.store(twy);
-        __syncthreads();  // twiddle tables
-        const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        const int q0 = WarpPairs<C>::first(w), ntask = WarpPairs<C>::count(w) * NZ;
-        for (int t = lane; t < ntask; t += 32) {
-            const int q = q0 + t / NZ, z = t % NZ;
-            const long long ia = plane_off + (2 * q) * NZ + z, ib = ia + NZ;
-            T va, vb;
-            if (MODE == PLANE_INIT_W) {
-                // hA = exp(-(W- + w+)/N), hB = exp(-(-W- + w+)/N)  (src/diblock.cc:64-72)
-                const double sgn = c == 0 ? 1.0 : -1.0;
-                const double da = exp(-(sgn * a.w[ia] + a.w[M + ia]) / a.Nd);
-                const double db = exp(-(sgn * a.w[ib] + a.w[M + ib]) / a.Nd);
-                va = (T)da;
-                vb = (T)db;
-                a.qout[c * M + ia] = va;
-                a.qout[c * M + ib] = vb;
-            } else if (a.src) {
-                va = a.src[c * a.src_stride + ia];
-                vb = a.src[c * a.src_stride + ib];
-            } else {
-                va = (T)a.src64[c * a.src_stride + ia];
-                vb = (T)a.src64[c * a.src_stride + ib];
-            }
-            P[2 * q * KZP + C::zpos(z)] = {va, vb};
-        }
-        __syncwarp();
-        z_fwdA_tw<C>(P, twa);
-        __syncwarp();
-        z_fwdB<C>(P);
-        __syncwarp();
-        z_unpack<C, true>(P);
-        __syncthreads();
-        y_fwdA_tw<C>(P, twy);
-        __syncthreads();
-        y_fwdB_global<C>(P, Sg, colbuf);
-        __syncthreads();
-        y_unpack0<C>(colbuf, Sg);
-        return;
-    }
-
-    // inverse y (natural -> transposed rows), then packed z lines
-    {
-        cpx<T> v[C::RY1];
-        y_invA_load<C>(Sg, v);
-        tws.store(twy);
-        __syncthreads();
-        y_invA_finish<C>(P, v, twy);
-    }
-    __syncthreads();
-    y_B<C, 1, false>(P, twy);
-    __syncthreads();
-    const T *h = a.h + (long long)(c == 0 ? a.hsel0 : a.hsel1) * M + plane_off;
-    z_build_invA<C>(P, twa);
-    __syncwarp();
-    T *qrow = a.qout + c * M + plane_off;
-    double qsum = 0.0;
-    z_invB_h<C, MODE>(P, twb, h, qrow, qsum);
-    if (MODE == PLANE_LAST) {
-        if (c == 0) {
-            // deterministic block reduction of the plane sum
-            __shared__ double red[C::NT / 32];
-            for (int o = 16; o > 0; o >>= 1) qsum += __shfl_xor_sync(0xffffffffu, qsum, o);
-            if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = qsum;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                double s = 0.0;
-                for (int i = 0; i < C::NT / 32; i++) s += red[i];
-                a.qpart[x] = s;
-            }
-        }
-        return;
+    // real rows (natural y order), packed two per complex line; the whole
+    // z section is warp-local (see WarpPairs)
+    tws.store(twy);
+    __syncthreads();  // twiddle tables
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int q0 = WarpPairs<C>::first(w), ntask = WarpPairs<C>::count(w) * NZ;
+    for (int t = lane; t < ntask; t += 32) {
+        const int q = q0 + t / NZ, z = t % NZ;
+        const long long ia = plane_off + (2 * q) * NZ + z, ib = ia + NZ;
+        P[2 * q * KZP + C::zpos(z)] = {a.src[c * a.src_stride + ia], a.src[c * a.src_stride + ib]};
     }
     __syncwarp();
-    z_fwdA<C>(P);
+    z_fwdA_tw<C>(P, twa);
     __syncwarp();
-    z_unpack<C, false>(P);
+    z_fwdB<C>(P);
+    __syncwarp();
+    z_unpack<C>(P);
     __syncthreads();
-    y_B<C, -1, true>(P, twy);
+    y_fwdA_tw<C>(P, twy);
     __syncthreads();
-    y_fwdA_global<C>(P, Sg, colbuf);
+    y_fwdB_global<C>(P, Sg, colbuf);
     __syncthreads();
     y_unpack0<C>(colbuf, Sg);
 }
@@ -726,7 +418,6 @@ __device__ __forceinline__ void pencil_body(const PencilArgs<T> &a, const int ti
         twx[t] = a.twx[t];
         if (MODE == PENCIL_CONV) gxs[t] = a.gx[t];  // POWER mode has no g table
     }
-    pdl_launch_dependents();
     pdl_wait();
 
     // X1: forward stage A from global (strided rows), twiddles, to smem.  At
@@ -862,6 +553,7 @@ __device__ __forceinline__ void pencil_body(const PencilArgs<T> &a, const int ti
     }
     if (MODE == PENCIL_POWER || MODE == PENCIL_H_LAST || MODE == PENCIL_HA_LAST) return;
     __syncthreads();
+    pdl_launch_dependents();
 
     // X3: inverse stage A (strided) -> natural order, to global
     for (int t = threadIdx.x; t < CW * R2; t += C::NT) {

@@ -335,7 +335,6 @@ __device__ __forceinline__ void plane_c_body(const PlaneArgs<T> &a, const int x,
 
     PcTw<C, T> tws;
     tws.load(a.twy, a.twz);
-    pdl_launch_dependents();
     pdl_wait();
 
     if (MODE == PLANE_INIT_W || MODE == PLANE_INIT_Q) {
@@ -373,6 +372,7 @@ __device__ __forceinline__ void plane_c_body(const PlaneArgs<T> &a, const int x,
             pc_y_A<C>(P, v, twy, false);
         }
         __syncthreads();
+        pdl_launch_dependents();
         pc_y_fwdB_global<C, true>(P, Sg);
         return;
     }
@@ -416,6 +416,7 @@ __device__ __forceinline__ void plane_c_body(const PlaneArgs<T> &a, const int x,
     __syncthreads();
     pc_y_B<C, -1, true>(P, twy);
     __syncthreads();
+    pdl_launch_dependents();
     pc_y_fwdA_global<C>(P, Sg);
 }
 

@@ -300,7 +300,6 @@ __device__ __forceinline__ void plane3_body(const PlaneArgs<float> &a, const int
         constexpr int BYTES = 2 * C::NY * C::NZ * (int)sizeof(float);
         for (int o = 128 * threadIdx.x; o < BYTES; o += 128 * C::NT) prefetch_l2(base + o);
     }
-    pdl_launch_dependents();
     pdl_wait();
 
     if (MODE == PLANE_INIT_W || MODE == PLANE_INIT_Q) {
@@ -308,6 +307,7 @@ __device__ __forceinline__ void plane3_body(const PlaneArgs<float> &a, const int
         __syncthreads();
         p3_s2_fwd<C>(P, TY, TZ);
         __syncthreads();
+        pdl_launch_dependents();
         p3_s1_fwd<C>(P, Sg);
         return;
     }
@@ -333,6 +333,7 @@ __device__ __forceinline__ void plane3_body(const PlaneArgs<float> &a, const int
     __syncthreads();
     p3_s2_fwd<C>(P, TY, TZ);
     __syncthreads();
+    pdl_launch_dependents();
     p3_s1_fwd<C>(P, Sg);
 }
 

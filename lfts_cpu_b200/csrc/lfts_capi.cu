@@ -18,7 +18,6 @@
 #include "../../include/lfts_b200.h"
 #include "anderson_device.cuh"
 #include "ctx.h"
-#include "fft_dispatch.h"
 #include "field_kernels.cuh"
 
 using namespace lfts;
@@ -107,26 +106,33 @@ void lfts_internal_set_error(const char *msg) { g_last_error = msg; }
 namespace {
 
 template <typename T>
-PlaneKernels<T> &plane_of(lfts_ctx *c);
+AxisSet<T> &axis_of(lfts_ctx *c);
 template <>
-PlaneKernels<double> &plane_of<double>(lfts_ctx *c) { return c->pl64; }
+AxisSet<double> &axis_of<double>(lfts_ctx *c) { return c->ax64; }
 template <>
-PlaneKernels<float> &plane_of<float>(lfts_ctx *c) { return c->pl32; }
-template <typename T>
-PencilKernels<T> &pencil_of(lfts_ctx *c);
-template <>
-PencilKernels<double> &pencil_of<double>(lfts_ctx *c) { return c->pe64; }
-template <>
-PencilKernels<float> &pencil_of<float>(lfts_ctx *c) { return c->pe32; }
+AxisSet<float> &axis_of<float>(lfts_ctx *c) { return c->ax32; }
 
 template <typename T>
-int set_smem_attrs(const PlaneKernels<T> &pl, const PencilKernels<T> &pe)
+int set_smem(const AxisFn<T> &f)
 {
-    for (int m = 0; m < kPlaneModes; m++)
-        if (pl.fn[m]) CK(cudaFuncSetAttribute(pl.fn[m], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
-    for (int m = 0; m < kPencilModes; m++)
-        if (pe.fn[m]) CK(cudaFuncSetAttribute(pe.fn[m], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pe.smem));
+    if (f.fn) CK(cudaFuncSetAttribute(f.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem));
     return LFTS_OK;
+}
+
+// the axis kernels of this context's mesh with x and y tiles of cw columns
+template <typename T>
+int set_axis(lfts_ctx *c, int cw)
+{
+    AxisSet<T> ax;
+    if (!axis_kernels(c->mx, c->my, c->mz, cw, &ax)) return LFTS_ERR_UNSUPPORTED;
+    int rc = set_smem(ax.y);
+    for (int m = 0; m < kAxisModes && !rc; m++) {
+        rc = set_smem(ax.x[m]);
+        if (!rc) rc = set_smem(ax.z[m]);
+        if (!rc) rc = set_smem(ax.plane[m]);
+    }
+    if (!rc) axis_of<T>(c) = ax;
+    return rc;
 }
 
 template <typename T>
@@ -145,19 +151,18 @@ int upload_tables(lfts_ctx *c, void **tw, void **gt)
     }
     if (!gt) return LFTS_OK;
     // g = exp(-(2 pi)^2 (kx^2/Lx^2 + ky^2/Ly^2 + kz^2/Lz^2)/(6N)) / M, factorised;
-    // the packed (full complex) spectrum needs kz over [0, mz), signed
-    const int n[3] = {c->mx, c->my, c->packed ? c->mz : c->KZ};
+    // over each axis's signed wavenumbers
     for (int d = 0; d < 3; d++) {
-        std::vector<T> g(n[d]);
-        for (int K = 0; K < n[d]; K++) {
-            const int k = (d == 2 && !c->packed) ? K : signed_k(K, m[d]);
+        std::vector<T> g(m[d]);
+        for (int K = 0; K < m[d]; K++) {
+            const int k = signed_k(K, m[d]);
             const double ksq = (double)k * k / (c->p.L[d] * c->p.L[d]);
             double v = std::exp(-kTwoPi * kTwoPi * ksq / (6.0 * c->N));
             if (d == 2) v /= (double)c->M;
             g[K] = (T)v;
         }
-        CK(cudaMalloc(&gt[d], sizeof(T) * n[d]));
-        CK(cudaMemcpy(gt[d], g.data(), sizeof(T) * n[d], cudaMemcpyHostToDevice));
+        CK(cudaMalloc(&gt[d], sizeof(T) * m[d]));
+        CK(cudaMemcpy(gt[d], g.data(), sizeof(T) * m[d], cudaMemcpyHostToDevice));
     }
     return LFTS_OK;
 }
@@ -170,50 +175,39 @@ inline dim3 update_grid(const lfts_ctx *c) { return dim3(c->sms * 8); }
 
 // ---- contour chain ----------------------------------------------------------
 template <typename T>
-PlaneArgs<T> plane_args(lfts_ctx *c)
+AxisArgs<T> axis_args(lfts_ctx *c)
 {
-    PlaneArgs<T> a{};
-    a.w = c->w;
-    a.spec = static_cast<cpx<T> *>(c->spec);
+    AxisArgs<T> a{};
+    a.S = static_cast<T *>(c->field);
+    a.twx = static_cast<const cpx<T> *>(c->tw[0]);
     a.twy = static_cast<const cpx<T> *>(c->tw[1]);
     a.twz = static_cast<const cpx<T> *>(c->tw[2]);
-    a.qpart = c->qpart;
-    a.nchains = 2;
-    a.Nd = (double)c->N;
     a.gx = static_cast<const T *>(c->gtab[0]);
     a.gy = static_cast<const T *>(c->gtab[1]);
     a.gz = static_cast<const T *>(c->gtab[2]);
-    return a;
-}
-
-template <typename T>
-PencilArgs<T> pencil_args(lfts_ctx *c)
-{
-    PencilArgs<T> a{};
-    a.spec = static_cast<cpx<T> *>(c->spec);
-    a.twx = static_cast<const cpx<T> *>(c->tw[0]);
-    a.gx = static_cast<const T *>(c->gtab[0]);
-    a.gy = static_cast<const T *>(c->gtab[1]);
-    a.gz = static_cast<const T *>(c->gtab[2]);
-    a.ncol = c->my * (c->packed ? c->mz : c->KZ);
-    a.KZ = c->packed ? c->mz : c->KZ;
-    a.w = c->w;
-    a.h = static_cast<const T *>(c->q);  // slot 1: the (hA, hB) pairs
+    a.mx = c->mx;
+    a.my = c->my;
+    a.mz = c->mz;
     a.M = c->M;
+    a.w = c->w;
     a.Nd = (double)c->N;
+    a.h = static_cast<const T *>(c->q);  // slot 1
+    a.qpart = c->qpart;
+    a.ticket = c->ticket;
+    a.Qd = c->Qd;
     return a;
 }
 
 // Chain kernels go out with programmatic stream serialisation (see pdl_wait in
 // fft_kernels.cuh): each may be scheduled while its predecessor drains.
 template <typename K, typename A>
-void launch_pdl(lfts_ctx *c, K kernel, dim3 grid, int nt, size_t smem, const A &args, cudaStream_t st = nullptr)
+void launch_pdl(lfts_ctx *c, K kernel, dim3 grid, int nt, size_t smem, const A &args, cudaStream_t st)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(nt);
     cfg.dynamicSmemBytes = smem;
-    cfg.stream = st ? st : c->st;
+    cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = c->use_pdl ? 1 : 0;
@@ -223,27 +217,40 @@ void launch_pdl(lfts_ctx *c, K kernel, dim3 grid, int nt, size_t smem, const A &
     c->launches++;
 }
 
-// In packed mode one launch covers both chains (gridDim.y = 1).
+// The kernels over x lines and over yz planes (one kernel, or z and y lines
+// apart), of the chains from a.cbase on: all of them, or `chains` (FP64)
 template <typename T>
-void launch_plane(lfts_ctx *c, int mode, const PlaneArgs<T> &a, int nchains, cudaStream_t st = nullptr)
+void launch_x(lfts_ctx *c, int mode, const AxisArgs<T> &a, int chains, cudaStream_t st)
 {
-    if constexpr (sizeof(T) == sizeof(float)) {
-        if (mode == PLANE_G && c->plane_split > 1) {
-            launch_pdl(c, c->psplit.fn, dim3(c->mx * c->psplit.cl), c->psplit.nt, c->psplit.smem, a, st);
-            return;
-        }
-    }
-    const PlaneKernels<T> &pl = plane_of<T>(c);
-    const int extra = mode == PLANE_G ? a.pf_ctas : 0;
-    launch_pdl(c, pl.fn[mode], dim3(c->mx + extra, c->packed ? 1 : nchains), pl.nt, pl.smem, a, st);
+    const AxisFn<T> &f = axis_of<T>(c).x[mode];
+    const int ncol = c->my * c->mz / kChains<T>;
+    launch_pdl(c, f.fn, dim3((ncol + f.per - 1) / f.per, 1, chains), f.nt, f.smem, a, st);
 }
 
+// y lines on their own, for the meshes without plane kernels
 template <typename T>
-void launch_pencil(lfts_ctx *c, int mode, const PencilArgs<T> &a, int nchains, cudaStream_t st = nullptr)
+void launch_y(lfts_ctx *c, const AxisArgs<T> &a, int chains, cudaStream_t st)
 {
-    const PencilKernels<T> &pe = pencil_of<T>(c);
-    launch_pdl(c, pe.fn[mode], dim3((a.ncol + pe.cw - 1) / pe.cw, c->packed ? 1 : nchains), pe.nt, pe.smem, a,
-               st);
+    const AxisSet<T> &ax = axis_of<T>(c);
+    if (ax.planes) return;
+    const int ncol = c->mz / kChains<T>;
+    launch_pdl(c, ax.y.fn, dim3((ncol + ax.y.per - 1) / ax.y.per, c->mx, chains), ax.y.nt, ax.y.smem, a, st);
+}
+
+// what follows h in a yz kernel's mode ends with the z convolution only where
+// the y lines have a kernel of their own: launch_y comes before and after it
+template <typename T>
+void launch_yz(lfts_ctx *c, int mode, const AxisArgs<T> &a, int chains, cudaStream_t st)
+{
+    const AxisSet<T> &ax = axis_of<T>(c);
+    if (ax.planes) {
+        const AxisFn<T> &f = ax.plane[mode];
+        launch_pdl(c, f.fn, dim3(c->mx, 1, chains), f.nt, f.smem, a, st);
+        return;
+    }
+    const AxisFn<T> &f = ax.z[mode];
+    const int nlines = c->mx * c->my / kChains<T>;
+    launch_pdl(c, f.fn, dim3((nlines + f.per - 1) / f.per, 1, chains), f.nt, f.smem, a, st);
 }
 
 inline int hsel_chain0(const lfts_ctx *c, int i) { return i < c->NA ? 0 : 1; }  // src/step.cc:53-57
@@ -299,114 +306,217 @@ void enqueue_chain(lfts_ctx *c)
     c->launches += c->chain_kernels;
 }
 
-// propagators of both chains for all N monomers, then Q (src/diblock.cc:36-48).
-// The two chains (q and q^) are independent until the concentrations, so
-// each runs its own launch sequence on its own stream (st: q, st1: q^) and
-// one chain's kernels fill the other's tails; with one stream both chains
-// share every launch.
+// ---- FP32-mixed chain by 3-D transforms ---------------------------------------
+// What a context runs once lfts_set_tiles has been called on it, and what the
+// ensemble's replicas run (lfts_ensemble.cu): fft_packed.cuh, fft_plane3.cuh.
+PlaneArgs<float> plane_args(lfts_ctx *c)
+{
+    PlaneArgs<float> a{};
+    a.w = c->w;
+    a.spec = static_cast<cpx<float> *>(c->field);
+    a.twy = static_cast<const cpx<float> *>(c->tw[1]);
+    a.twz = static_cast<const cpx<float> *>(c->tw[2]);
+    a.qpart = c->qpart;
+    a.nchains = 2;
+    a.Nd = (double)c->N;
+    a.gx = static_cast<const float *>(c->gtab[0]);
+    a.gy = static_cast<const float *>(c->gtab[1]);
+    a.gz = static_cast<const float *>(c->gtab[2]);
+    return a;
+}
+
+PencilArgs<float> pencil_args(lfts_ctx *c)
+{
+    PencilArgs<float> a{};
+    a.spec = static_cast<cpx<float> *>(c->field);
+    a.twx = static_cast<const cpx<float> *>(c->tw[0]);
+    a.gx = static_cast<const float *>(c->gtab[0]);
+    a.gy = static_cast<const float *>(c->gtab[1]);
+    a.gz = static_cast<const float *>(c->gtab[2]);
+    a.ncol = c->my * c->mz;
+    a.KZ = c->mz;
+    a.w = c->w;
+    a.h = static_cast<const float *>(c->q);  // slot 1: the (hA, hB) pairs
+    a.M = c->M;
+    a.Nd = (double)c->N;
+    return a;
+}
+
+void launch_plane(lfts_ctx *c, int mode, const PlaneArgs<float> &a)
+{
+    if (mode == PLANE_G && c->plane_split > 1) {
+        launch_pdl(c, c->psplit.fn, dim3(c->mx * c->psplit.cl), c->psplit.nt, c->psplit.smem, a, c->st);
+        return;
+    }
+    const int extra = mode == PLANE_G ? a.pf_ctas : 0;
+    launch_pdl(c, c->pl32.fn[mode], dim3(c->mx + extra), c->pl32.nt, c->pl32.smem, a, c->st);
+}
+
+void launch_pencil(lfts_ctx *c, int mode, const PencilArgs<float> &a)
+{
+    launch_pdl(c, c->pe32.fn[mode], dim3((a.ncol + c->pe32.cw - 1) / c->pe32.cw), c->pe32.nt, c->pe32.smem, a, c->st);
+}
+
+void enqueue_transform_chain(lfts_ctx *c)
+{
+    float *q = static_cast<float *>(c->q);
+    const long long M = c->M;
+    PlaneArgs<float> a = plane_args(c);
+    PencilArgs<float> pa = pencil_args(c);
+    if (c->xh_chain) {
+        // One step is q_{i+1} = h . F^-1[g . F[q_i]].  g is even in every
+        // wavenumber, so F^-1[g F[q]] = F[g F^-1[q]]; with D_i = F_x^-1[q_i]
+        // in the spectrum buffer a step is
+        //   yz-plane (PLANE_G):  E_i = F_yz[g . F_yz^-1[D_i]]  (the STEP flow, g for h)
+        //   x-pencil (PENCIL_H): q_{i+1} = h . F_x[E_i], stored; D_{i+1} = F_x^-1[q_{i+1}]
+        // which puts the h loads and q stores in the pencil's several CTAs
+        // per SM instead of the plane kernel's one.
+        PencilArgs<float> pi = pa;
+        pi.qout = q;  // slot 1 = (hA, hB)
+        launch_pencil(c, PENCIL_INIT_W, pi);
+        // With phi in the chain, the concentration sums are formed as the
+        // slots are made: slot i+1 = (q_{i+1}, q^_{N-i}) pairs with slot
+        // N-i = (q_{N-i}, q^_{i+1}).  From the middle of the chain on that
+        // partner is already stored, so the pencil adds the two products
+        // into acc and slot i+1 need not be stored (except slot N, for Q);
+        // the middle slot of an odd chain pairs with itself.
+        const bool acc = c->phi_in_chain;
+        bool first_acc = true;
+        for (int i = 1; i < c->N; i++) {
+            PlaneArgs<float> ag = a;
+            if (acc && c->N - i < i + 1) {
+                ag.pf = q + (long long)(c->N - i - 1) * 2 * M;  // the partner slot
+                if (c->plane_split == 1) ag.pf_ctas = c->pf_ctas;
+            }
+            launch_plane(c, PLANE_G, ag);
+            PencilArgs<float> ph = pa;
+            ph.qout = q + (long long)i * 2 * M;  // slot i+1
+            ph.hsel0 = hsel_chain0(c, i);
+            ph.hsel1 = hsel_chain1(c, i);
+            const int p = c->N - i;  // partner slot
+            if (!acc || p > i + 1) {
+                launch_pencil(c, i + 1 < c->N ? PENCIL_H : PENCIL_H_LAST, ph);
+                continue;
+            }
+            ph.partner = p < i + 1 ? q + (long long)(p - 1) * 2 * M : nullptr;
+            ph.acc = static_cast<float *>(c->acc);
+            ph.acc_init = first_acc ? 1 : 0;
+            ph.a_is_A = i + 1 <= c->NA;
+            ph.b_is_A = p <= c->NA;
+            first_acc = false;
+            launch_pencil(c, i + 1 < c->N ? PENCIL_HA : PENCIL_HA_LAST, ph);
+        }
+        plane_q_sums_kernel<<<c->mx, 256, 0, c->st>>>(
+            reinterpret_cast<const float2 *>(q + (long long)(c->N - 1) * 2 * M), (long long)c->my * c->mz,
+            c->qpart);
+        q_finalize_kernel<<<1, 256, 0, c->st>>>(c->qpart, c->mx, M, c->Qd);
+        c->launches += 2;
+        return;
+    }
+    a.qout = q;  // slot 1 = [hA | hB]
+    launch_plane(c, PLANE_INIT_W, a);
+    a.h = q;
+    for (int i = 1; i < c->N; i++) {
+        launch_pencil(c, PENCIL_CONV, pa);
+        a.qout = q + (long long)i * 2 * M;  // slot i+1
+        a.hsel0 = hsel_chain0(c, i);
+        a.hsel1 = hsel_chain1(c, i);
+        launch_plane(c, i + 1 < c->N ? PLANE_STEP : PLANE_LAST, a);
+    }
+    q_finalize_kernel<<<1, 256, 0, c->st>>>(c->qpart, c->mx, M, c->Qd);
+    c->launches++;
+}
+
+// ---- chain one axis at a time -------------------------------------------------
+// One contour step of the chains from a.cbase on: step i makes slot i+1 from
+// the field that the step before left convolved along z and y (i odd) or
+// along x (i even); a holds what the step's kernel needs.
+template <typename T>
+void launch_step(lfts_ctx *c, int i, int mode, const AxisArgs<T> &a, int chains, cudaStream_t st)
+{
+    launch_y<T>(c, a, chains, st);
+    if (i & 1)
+        launch_x<T>(c, mode, a, chains, st);
+    else
+        launch_yz<T>(c, mode, a, chains, st);
+}
+
+// slot i+1 and the h halves of step i (src/step.cc:53-64)
+template <typename T>
+void set_slot(lfts_ctx *c, AxisArgs<T> &a, int i)
+{
+    a.q[0] = static_cast<T *>(c->q) + (long long)i * 2 * c->M;
+    a.q[1] = a.q[0] + c->M;
+    a.hsel[0] = hsel_chain0(c, i);
+    a.hsel[1] = hsel_chain1(c, i);
+}
+
+// Propagators of both chains for all N monomers, then Q (src/diblock.cc:36-48),
+// one axis at a time (axis_conv.cuh): INIT_W leaves h convolved along z and y;
+// odd steps end along x and begin the next step there, even steps end and begin
+// along z and y.  FP64 chains are independent until the concentrations: with
+// two_streams each runs its own launches on its own stream, else both share
+// every launch.
 template <typename T>
 void enqueue_chain_launches(lfts_ctx *c)
 {
-    T *q = static_cast<T *>(c->q);
-    const long long M = c->M;
-    PlaneArgs<T> a = plane_args<T>(c);
-    PencilArgs<T> pa = pencil_args<T>(c);
-    if constexpr (sizeof(T) == sizeof(float)) {
-        if (c->xh_chain) {
-            // One step is q_{i+1} = h . F^-1[g . F[q_i]].  g is even in every
-            // wavenumber, so F^-1[g F[q]] = F[g F^-1[q]]; with D_i = F_x^-1[q_i]
-            // in the spectrum buffer a step is
-            //   yz-plane (PLANE_G):  E_i = F_yz[g . F_yz^-1[D_i]]  (the STEP flow, g for h)
-            //   x-pencil (PENCIL_H): q_{i+1} = h . F_x[E_i], stored; D_{i+1} = F_x^-1[q_{i+1}]
-            // which puts the h loads and q stores in the pencil's several CTAs
-            // per SM instead of the plane kernel's one.
-            PencilArgs<T> pi = pa;
-            pi.qout = q;  // slot 1 = (hA, hB)
-            launch_pencil<T>(c, PENCIL_INIT_W, pi, 2);
-            // With phi in the chain, the concentration sums are formed as the
-            // slots are made: slot i+1 = (q_{i+1}, q^_{N-i}) pairs with slot
-            // N-i = (q_{N-i}, q^_{i+1}).  From the middle of the chain on that
-            // partner is already stored, so the pencil adds the two products
-            // into acc and slot i+1 need not be stored (except slot N, for Q);
-            // the middle slot of an odd chain pairs with itself.
-            const bool acc = c->phi_in_chain;
-            bool first_acc = true;
-            for (int i = 1; i < c->N; i++) {
-                PlaneArgs<T> ag = a;
-                if (acc && c->N - i < i + 1) {
-                    ag.pf = q + (long long)(c->N - i - 1) * 2 * M;  // the partner slot
-                    if (c->plane_split == 1) ag.pf_ctas = c->pf_ctas;
-                }
-                launch_plane<T>(c, PLANE_G, ag, 2);
-                PencilArgs<T> ph = pa;
-                ph.qout = q + (long long)i * 2 * M;  // slot i+1
-                ph.hsel0 = hsel_chain0(c, i);
-                ph.hsel1 = hsel_chain1(c, i);
-                const int p = c->N - i;  // partner slot
-                if (!acc || p > i + 1) {
-                    launch_pencil<T>(c, i + 1 < c->N ? PENCIL_H : PENCIL_H_LAST, ph, 2);
-                    continue;
-                }
-                ph.partner = p < i + 1 ? q + (long long)(p - 1) * 2 * M : nullptr;
-                ph.acc = static_cast<T *>(c->acc);
-                ph.acc_init = first_acc ? 1 : 0;
-                ph.a_is_A = i + 1 <= c->NA;
-                ph.b_is_A = p <= c->NA;
-                first_acc = false;
-                launch_pencil<T>(c, i + 1 < c->N ? PENCIL_HA : PENCIL_HA_LAST, ph, 2);
-            }
-            plane_q_sums_kernel<<<c->mx, 256, 0, c->st>>>(
-                reinterpret_cast<const float2 *>(q + (long long)(c->N - 1) * 2 * M), (long long)c->my * c->mz,
-                c->qpart);
-            q_finalize_kernel<<<1, 256, 0, c->st>>>(c->qpart, c->mx, M, c->Qd);
-            c->launches += 2;
+    if constexpr (kPairs<T>) {
+        if (c->transform_chain) {
+            enqueue_transform_chain(c);
             return;
         }
     }
-    if (!c->two_streams || c->packed) {
-        a.qout = q;  // slot 1 = [hA | hB]
-        launch_plane<T>(c, PLANE_INIT_W, a, 2);
-        a.h = q;
-        for (int i = 1; i < c->N; i++) {
-            launch_pencil<T>(c, PENCIL_CONV, pa, 2);
-            a.qout = q + (long long)i * 2 * M;  // slot i+1
-            a.hsel0 = hsel_chain0(c, i);
-            a.hsel1 = hsel_chain1(c, i);
-            launch_plane<T>(c, i + 1 < c->N ? PLANE_STEP : PLANE_LAST, a, 2);
-        }
-    } else {
+    const int N = c->N;
+    const AxisArgs<T> a = axis_args<T>(c);
+    const bool two = !kPairs<T> && c->two_streams;
+    const int chains = two ? 1 : kChains<T>;
+    cudaStream_t sc[2] = {c->st, c->st1};
+    AxisArgs<T> ac[2] = {a, a};
+    ac[1].cbase = 1;
+    if (two) {
         cudaEventRecord(c->ev_fork, c->st);
         cudaStreamWaitEvent(c->st1, c->ev_fork, 0);
-        cudaStream_t sc[2] = {c->st, c->st1};
-        PlaneArgs<T> ac[2] = {a, a};
-        PencilArgs<T> pc[2] = {pa, pa};
-        for (int k = 0; k < 2; k++) {
-            ac[k].cbase = k;
-            pc[k].cbase = k;
-            ac[k].qout = q;
-            launch_plane<T>(c, PLANE_INIT_W, ac[k], 1, sc[k]);
-            ac[k].h = q;
-        }
+    }
+    for (int k = 0; k <= (two ? 1 : 0); k++) {
+        set_slot(c, ac[k], 0);
+        launch_yz<T>(c, AX_INIT_W, ac[k], chains, sc[k]);
+    }
+    if (two) {
         // Each stream's INIT_W writes its own half of h (hA from chain 1, hB from
         // chain 2), and each chain's steps read the other half once i >= NA
         // (chain 1) or i >= NB (chain 2): both halves are complete before either
         // chain's first step.
         for (int k = 0; k < 2; k++) cudaEventRecord(c->ev_h[k], sc[k]);
         for (int k = 0; k < 2; k++) cudaStreamWaitEvent(sc[k], c->ev_h[1 - k], 0);
-        for (int i = 1; i < c->N; i++) {
-            for (int k = 0; k < 2; k++) launch_pencil<T>(c, PENCIL_CONV, pc[k], 1, sc[k]);
-            for (int k = 0; k < 2; k++) {
-                ac[k].qout = q + (long long)i * 2 * M;
-                ac[k].hsel0 = hsel_chain0(c, i);
-                ac[k].hsel1 = hsel_chain1(c, i);
-                launch_plane<T>(c, i + 1 < c->N ? PLANE_STEP : PLANE_LAST, ac[k], 1, sc[k]);
+    }
+    bool first_acc = true;
+    for (int i = 1; i < N; i++) {
+        for (int k = 0; k <= (two ? 1 : 0); k++) {
+            set_slot(c, ac[k], i);
+            int mode = i + 1 < N ? AX_H : AX_H_LAST;
+            // With phi in the chain (FP32), the concentration sums are formed as the
+            // slots are made: slot i+1 = (q_{i+1}, q^_{N-i}) pairs with slot
+            // N-i = (q_{N-i}, q^_{i+1}).  From the middle of the chain on that
+            // partner is already stored, so the kernel adds the two products
+            // into acc and slot i+1 need not be stored (except slot N, for Q);
+            // the middle slot of an odd chain pairs with itself.
+            const int p = N - i;  // partner slot
+            if (kPairs<T> && c->phi_in_chain && p <= i + 1) {
+                mode = i + 1 < N ? AX_HA : AX_HA_LAST;
+                ac[k].partner = p < i + 1 ? static_cast<const T *>(c->q) + (long long)(p - 1) * 2 * c->M : nullptr;
+                ac[k].acc = static_cast<T *>(c->acc);
+                ac[k].acc_init = first_acc ? 1 : 0;
+                ac[k].a_is_A = i + 1 <= c->NA;
+                ac[k].b_is_A = p <= c->NA;
+                first_acc = false;
             }
+            launch_step<T>(c, i, mode, ac[k], chains, sc[k]);
         }
+    }
+    if (two) {
         cudaEventRecord(c->ev_join, c->st1);
         cudaStreamWaitEvent(c->st, c->ev_join, 0);
     }
-    q_finalize_kernel<<<1, 256, 0, c->st>>>(c->qpart, c->mx, M, c->Qd);
-    c->launches++;
 }
 
 template <typename T>
@@ -445,34 +555,26 @@ void enqueue_concs_any(lfts_ctx *c, void *Dh0, int nh, const HistPtrs &hist)
 }
 
 // ---- tile choices and their autotuner ------------------------------------------
-// A context's contour chain has these free choices, none of which changes what
-// is computed (each is tested against the others at the precision's tolerance;
-// the x-pencil width changes no column's arithmetic at all):
-//   pencil_cw     x-pencil columns per CTA (8, 16, 32)
-//   plane_stages  FP32-mixed yz-plane transform stages per axis: 3 (fft_plane3.cuh,
-//                 64 / 96 / 128 square planes) or 2 (fft_packed.cuh)
-//   h_in_pencil   FP32-mixed: h and the propagator stores in the x-pencil and g in
-//                 the yz-plane kernel (96- and 128-point x lines, three-stage planes),
-//                 or both in the yz-plane kernel
+// The axis-by-axis chain has these free choices, none of which changes what is
+// computed (phi_in_chain within the FP32-mixed tolerance, the others not at all):
+//   pencil_cw     columns per CTA of the x- and y-line kernels (8, 16, 32)
+//   phi_in_chain  FP32-mixed, 96- and 128-point lines: concentration sums formed
+//                 in the chain
 //   two_streams   FP64: each chain on its own stream, or both chains per launch
-// autotune() times the whole chain for every valid combination on the
-// context's own buffers (a tile's cost depends on how it overlaps its
-// neighbours in the chain, so it is timed in place) and keeps the fastest,
-// once per (precision, mesh) per process -- the reference's analogue is
-// planning its FFTs with FFTW_PATIENT (src/step.cc:15-16).
+// autotune() times the whole chain for every combination on the context's own
+// buffers (a tile's cost depends on how it overlaps its neighbours in the chain,
+// so it is timed in place) and keeps the fastest, once per (precision, mesh) per
+// process -- the reference's analogue is planning its FFTs with FFTW_PATIENT
+// (src/step.cc:15-16).
+// lfts_set_tiles on an FP32-mixed context installs the transform chain instead,
+// whose choices change how values are rounded:
+//   plane_stages  yz-plane transform stages per axis: 3 (fft_plane3.cuh, 64 / 96 /
+//                 128 square planes) or 2 (fft_packed.cuh)
+//   h_in_pencil   h and the propagator stores in the x-pencil and g in the
+//                 yz-plane kernel (96- and 128-point x lines, three-stage planes),
+//                 or both in the yz-plane kernel
 std::mutex g_tune_mu;
 std::map<std::tuple<int, int, int, int>, lfts_tiles> g_tuned;
-
-template <typename T>
-int set_pencil(lfts_ctx *c, int cw)
-{
-    PencilKernels<T> pk{};
-    if (!pencil_kernels(c->mx, cw, &pk)) return LFTS_ERR_UNSUPPORTED;
-    for (int m = 0; m < kPencilModes; m++)
-        if (pk.fn[m]) CK(cudaFuncSetAttribute(pk.fn[m], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pk.smem));
-    pencil_of<T>(c) = pk;
-    return LFTS_OK;
-}
 
 // the captured chain and the Anderson-loop graph that holds it (rebuilt on
 // the next use with the new tiles)
@@ -489,78 +591,108 @@ void drop_chain_graph(lfts_ctx *c)
     if (c->mix_graph_state == 1) c->mix_graph_state = 0;
 }
 
-// installs a tile choice (validated); the chain graph is captured anew
+// FP32-mixed meshes that an ensemble runs with one layout of the transform chain
+// only: a context runs it there too, so that a replica computes what a context
+// of its mesh does.  (16^3 ... 48^3: as replicas' Anderson loops amplify
+// rounding, the ensemble keeps the arithmetic of its chain.)
+bool transform_by_default(const lfts_ctx *c)
+{
+    auto ens = [](int n) { return n == 16 || n == 24 || n == 32 || n == 48; };
+    return c->prec == LFTS_FP32_MIXED && c->my == c->mz && ens(c->my) && (ens(c->mx) || c->mx == 64 || c->mx == 96);
+}
+
+bool has_three_stages(const lfts_ctx *c) { return c->my == c->mz && (c->my == 64 || c->my == 96 || c->my == 128); }
+bool has_h_in_pencil(const lfts_ctx *c)
+{
+    return has_three_stages(c) && c->my != 64 && (c->mx == 96 || c->mx == 128);
+}
+
+// the (A, B) concentration sums, FP32 pairs per mesh point
+int alloc_sums(lfts_ctx *c)
+{
+    if (c->acc) return LFTS_OK;
+    if (cudaMalloc(&c->acc, sizeof(float) * 2 * (size_t)c->M) == cudaSuccess) return LFTS_OK;
+    cudaGetLastError();
+    c->acc = nullptr;
+    g_last_error = "device allocation of the concentration sums failed";
+    return LFTS_ERR_NOMEM;
+}
+
+// the axis-by-axis chain with the choices of t (autotune's, so valid)
+int apply_axis_tiles(lfts_ctx *c, const lfts_tiles &t)
+{
+    int rc = t.phi_in_chain ? alloc_sums(c) : LFTS_OK;
+    if (!rc) rc = c->prec == LFTS_FP64 ? set_axis<double>(c, t.pencil_cw) : set_axis<float>(c, t.pencil_cw);
+    if (rc) return rc;
+    c->transform_chain = false;
+    c->two_streams = t.two_streams == 1;
+    c->phi_in_chain = t.phi_in_chain == 1;
+    c->tiles = t;
+    drop_chain_graph(c);
+    return LFTS_OK;
+}
+
+// lfts_set_tiles' choice, validated first; the chain graph is captured anew
 int apply_tiles(lfts_ctx *c, const lfts_tiles &t)
 {
     if (t.pencil_cw != 8 && t.pencil_cw != 16 && t.pencil_cw != 32) return LFTS_ERR_ARG;
     const int split = t.plane_split == 0 ? 1 : t.plane_split;
     if (split != 1 && split != 8) return LFTS_ERR_ARG;
+    lfts_tiles now = t;
+    now.plane_split = split;
     if (c->prec == LFTS_FP64) {
         if (t.plane_stages != 2 || t.h_in_pencil != 0 || (t.two_streams != 0 && t.two_streams != 1) ||
             t.phi_in_chain != 0 || split != 1)
             return LFTS_ERR_ARG;
-        int rc = set_pencil<double>(c, t.pencil_cw);
-        if (rc) return rc;
-        c->two_streams = t.two_streams == 1;
-    } else {
-        if ((t.plane_stages != 2 && t.plane_stages != 3) || (t.h_in_pencil != 0 && t.h_in_pencil != 1) ||
-            t.two_streams != 0 || (t.phi_in_chain != 0 && t.phi_in_chain != 1) || (t.phi_in_chain && !t.h_in_pencil))
-            return LFTS_ERR_ARG;
-        PlaneKernels<float> pl{};
-        const bool ok = t.plane_stages == 3 ? plane3_kernels(c->my, c->mz, &pl) : plane_c_kernels(c->my, c->mz, &pl);
-        if (!ok) return LFTS_ERR_UNSUPPORTED;
-        PencilKernels<float> pk{};
-        if (!pencil_kernels(c->mx, t.pencil_cw, &pk)) return LFTS_ERR_UNSUPPORTED;
-        if (t.h_in_pencil && !(pl.fn[PLANE_G] && pk.fn[PENCIL_H])) return LFTS_ERR_UNSUPPORTED;
-        if (t.phi_in_chain && !(pk.fn[PENCIL_HA] && pk.fn[PENCIL_HA_LAST])) return LFTS_ERR_UNSUPPORTED;
-        PlaneSplitKernel ps{};
-        if (split > 1) {
-            // the cluster kernel replaces PLANE_G of the three-stage plane
-            if (!(t.h_in_pencil && t.plane_stages == 3 && plane_split_kernel(c->my, c->mz, &ps) && ps.cl == split))
-                return LFTS_ERR_UNSUPPORTED;
-            CK(cudaFuncSetAttribute(ps.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ps.smem));
-        }
-        if (t.phi_in_chain && !c->acc) {
-            // the (A, B) concentration sums, FP32 pairs per mesh point
-            cudaError_t e = cudaMalloc(&c->acc, sizeof(float) * 2 * (size_t)c->M);
-            if (e != cudaSuccess) {
-                cudaGetLastError();
-                c->acc = nullptr;
-                g_last_error = "device allocation of the concentration sums failed";
-                return LFTS_ERR_NOMEM;
-            }
-        }
-        for (int m = 0; m < kPlaneModes; m++)
-            if (pl.fn[m]) CK(cudaFuncSetAttribute(pl.fn[m], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
-        int rc = set_pencil<float>(c, t.pencil_cw);
-        if (rc) return rc;
-        c->pl32 = pl;
-        c->psplit = ps;
-        c->plane_split = split;
-        c->plane_stages = t.plane_stages;
-        c->xh_chain = t.h_in_pencil == 1;
-        c->phi_in_chain = t.phi_in_chain == 1;
+        return apply_axis_tiles(c, now);
     }
+    if ((t.plane_stages != 2 && t.plane_stages != 3) || (t.h_in_pencil != 0 && t.h_in_pencil != 1) ||
+        t.two_streams != 0 || (t.phi_in_chain != 0 && t.phi_in_chain != 1) || (t.phi_in_chain && !t.h_in_pencil))
+        return LFTS_ERR_ARG;
+    PlaneKernels<float> pl{};
+    const bool ok = t.plane_stages == 3 ? plane3_kernels(c->my, c->mz, &pl) : plane_c_kernels(c->my, c->mz, &pl);
+    if (!ok) return LFTS_ERR_UNSUPPORTED;
+    PencilKernels<float> pk{};
+    if (!pencil_kernels(c->mx, t.pencil_cw, &pk)) return LFTS_ERR_UNSUPPORTED;
+    if (t.h_in_pencil && !(pl.fn[PLANE_G] && pk.fn[PENCIL_H])) return LFTS_ERR_UNSUPPORTED;
+    if (t.phi_in_chain && !(pk.fn[PENCIL_HA] && pk.fn[PENCIL_HA_LAST])) return LFTS_ERR_UNSUPPORTED;
+    PlaneSplitKernel ps{};
+    if (split > 1) {
+        // the cluster kernel replaces PLANE_G of the three-stage plane
+        if (!(t.h_in_pencil && t.plane_stages == 3 && plane_split_kernel(c->my, c->mz, &ps) && ps.cl == split))
+            return LFTS_ERR_UNSUPPORTED;
+        CK(cudaFuncSetAttribute(ps.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ps.smem));
+    }
+    if (t.phi_in_chain) {
+        int rc = alloc_sums(c);
+        if (rc) return rc;
+    }
+    for (int m = 0; m < kPlaneModes; m++)
+        if (pl.fn[m]) CK(cudaFuncSetAttribute(pl.fn[m], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
+    for (int m = 0; m < kPencilModes; m++)
+        if (pk.fn[m]) CK(cudaFuncSetAttribute(pk.fn[m], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pk.smem));
+    c->transform_chain = true;
+    c->pl32 = pl;
+    c->pe32 = pk;
+    c->psplit = ps;
+    c->plane_split = split;
+    c->xh_chain = t.h_in_pencil == 1;
+    c->phi_in_chain = t.phi_in_chain == 1;
+    c->tiles = now;
     drop_chain_graph(c);
     return LFTS_OK;
 }
 
-lfts_tiles current_tiles(const lfts_ctx *c)
+// a choice of tile_candidates, for the chain that the context runs by default
+int apply_default_tiles(lfts_ctx *c, const lfts_tiles &t)
 {
-    lfts_tiles t{};
-    const bool fp64 = c->prec == LFTS_FP64;
-    t.pencil_cw = fp64 ? c->pe64.cw : c->pe32.cw;
-    t.plane_stages = fp64 ? 2 : c->plane_stages;
-    t.h_in_pencil = (!fp64 && c->xh_chain) ? 1 : 0;
-    t.two_streams = (fp64 && c->two_streams) ? 1 : 0;
-    t.phi_in_chain = (!fp64 && c->phi_in_chain) ? 1 : 0;
-    t.plane_split = fp64 ? 1 : c->plane_split;
-    return t;
+    return transform_by_default(c) ? apply_tiles(c, t) : apply_axis_tiles(c, t);
 }
 
-// every valid combination for this context, restricted by the environment
-// (LFTS_PENCIL_CW, LFTS_XH_CHAIN, LFTS_ONE_STREAM, LFTS_PHI_IN_CHAIN fix one
-// choice each)
+// every combination of the default chain, restricted by the environment
+// (LFTS_PENCIL_CW, LFTS_ONE_STREAM, LFTS_PHI_IN_CHAIN fix one choice each;
+// LFTS_XH_CHAIN=0 leaves the sums out).  plane_stages and h_in_pencil name the
+// transform chain that such a choice belongs to.
 std::vector<lfts_tiles> tile_candidates(const lfts_ctx *c)
 {
     std::vector<lfts_tiles> out;
@@ -568,10 +700,6 @@ std::vector<lfts_tiles> tile_candidates(const lfts_ctx *c)
     const char *fxh = std::getenv("LFTS_XH_CHAIN");
     const char *fone = std::getenv("LFTS_ONE_STREAM");
     const char *fphi = std::getenv("LFTS_PHI_IN_CHAIN");
-    const char *fsplit = std::getenv("LFTS_PLANE_SPLIT");
-    const int split_forced = fsplit ? std::atoi(fsplit) : 0;
-    PlaneSplitKernel ps{};
-    const bool has_split = c->prec != LFTS_FP64 && plane_split_kernel(c->my, c->mz, &ps);
     const int cw_forced = fcw ? std::atoi(fcw) : 0;
     for (int cw : {8, 16, 32}) {
         if (cw_forced > 0 && cw != cw_forced) continue;
@@ -582,35 +710,18 @@ std::vector<lfts_tiles> tile_candidates(const lfts_ctx *c)
             }
             continue;
         }
-        PlaneKernels<float> p3{};
-        PencilKernels<float> pk{};
-        const bool has3 = plane3_kernels(c->my, c->mz, &p3);
-        const bool hasx = has3 && p3.fn[PLANE_G] && pencil_kernels(c->mx, cw, &pk) && pk.fn[PENCIL_H];
-        const bool hasa = hasx && pk.fn[PENCIL_HA] && pk.fn[PENCIL_HA_LAST];
-        for (int st : {3, 2}) {
-            if (st == 3 && !has3) continue;
-            for (int xh : {1, 0}) {
-                if (xh && (st != 3 || !hasx)) continue;
-                if (fxh && ((fxh[0] != '0') != (xh == 1))) continue;
-                for (int phi : {0, 1}) {
-                    if (phi && (!xh || !hasa)) continue;
-                    if (fphi && ((fphi[0] != '0') != (phi == 1))) continue;
-                    // LFTS_PLANE_SPLIT applies where the cluster kernel does
-                    const bool can_split = xh && has_split && ps.cl == 8;
-                    for (int split : {1, 8}) {
-                        if (split > 1 && !can_split) continue;
-                        if (split_forced > 0 && can_split && split != split_forced) continue;
-                        out.push_back({cw, st, xh, 0, phi, split});
-                    }
-                }
-            }
+        const int xh = has_h_in_pencil(c) && !(fxh && fxh[0] == '0') ? 1 : 0;
+        for (int phi : {0, 1}) {
+            if (phi && !xh) continue;
+            if (fphi && xh && ((fphi[0] != '0') != (phi == 1))) continue;
+            out.push_back({cw, has_three_stages(c) ? 3 : 2, xh, 0, phi, 1});
         }
     }
     return out;
 }
 
-// the choice used when autotuning is off: three-stage planes and h in the
-// x-pencil where compiled, the usual pencil winners, two FP64 streams
+// the choice used when autotuning is off: the usual tile winners, two FP64
+// streams, the separate concentration pass
 lfts_tiles default_tiles(const lfts_ctx *c)
 {
     std::vector<lfts_tiles> cand = tile_candidates(c);
@@ -661,7 +772,7 @@ int tune_tiles(lfts_ctx *c, lfts_tiles *best)
     bool found = false;
     int rc = LFTS_OK;
     for (const lfts_tiles &t : tile_candidates(c)) {
-        if (apply_tiles(c, t) != LFTS_OK) continue;
+        if (apply_default_tiles(c, t) != LFTS_OK) continue;
         float ms = 0.f;
         rc = c->prec == LFTS_FP64 ? time_chain<double>(c, e0, e1, &ms) : time_chain<float>(c, e0, e1, &ms);
         if (rc) break;
@@ -696,60 +807,58 @@ int autotune(lfts_ctx *c)
             g_tuned[key] = t;
         }
     }
-    return apply_tiles(c, t);
+    return apply_default_tiles(c, t);
 }
 
 // One chain on one stream with CUDA events around every contour-step kernel
 // (mean duration of a yz-plane STEP and an x-pencil CONV launch, both chains
 // per launch), then the production chain timed as a whole (first launch to Q).
-template <typename T>
-int profile_chain(lfts_ctx *c, double *ms_plane, double *ms_pencil, double *ms_chain)
+int profile_transform_chain(lfts_ctx *c, double *ms_plane, double *ms_pencil, double *ms_chain)
 {
     const int n = c->N - 1;
     std::vector<cudaEvent_t> ev(4 * n + 2);
     for (auto &e : ev) CK(cudaEventCreate(&e));
-    T *q = static_cast<T *>(c->q);
+    float *q = static_cast<float *>(c->q);
     const long long M = c->M;
-    PlaneArgs<T> a = plane_args<T>(c);
-    PencilArgs<T> pa = pencil_args<T>(c);
+    PlaneArgs<float> a = plane_args(c);
+    PencilArgs<float> pa = pencil_args(c);
     // per step j: pencil between ev[4j] and ev[4j+1], plane between ev[4j+2] and ev[4j+3]
     CK(cudaEventRecord(ev[4 * n], c->st));
     if (c->xh_chain) {
-        // the chain of enqueue_chain_launches: pencil INIT_W, (N-1) x (plane G, pencil H)
-        PencilArgs<T> pi = pa;
+        // the chain of enqueue_transform_chain: pencil INIT_W, (N-1) x (plane G, pencil H)
+        PencilArgs<float> pi = pa;
         pi.qout = q;
-        launch_pencil<T>(c, PENCIL_INIT_W, pi, 2);
+        launch_pencil(c, PENCIL_INIT_W, pi);
         for (int i = 1; i < c->N; i++) {
             const int j = i - 1;
             CK(cudaEventRecord(ev[4 * j + 2], c->st));
-            launch_plane<T>(c, PLANE_G, a, 2);
+            launch_plane(c, PLANE_G, a);
             CK(cudaEventRecord(ev[4 * j + 3], c->st));
-            PencilArgs<T> ph = pa;
+            PencilArgs<float> ph = pa;
             ph.qout = q + (long long)i * 2 * M;
             ph.hsel0 = hsel_chain0(c, i);
             ph.hsel1 = hsel_chain1(c, i);
             CK(cudaEventRecord(ev[4 * j], c->st));
-            launch_pencil<T>(c, i + 1 < c->N ? PENCIL_H : PENCIL_H_LAST, ph, 2);
+            launch_pencil(c, i + 1 < c->N ? PENCIL_H : PENCIL_H_LAST, ph);
             CK(cudaEventRecord(ev[4 * j + 1], c->st));
         }
-        if constexpr (sizeof(T) == sizeof(float))
-            plane_q_sums_kernel<<<c->mx, 256, 0, c->st>>>(
-                reinterpret_cast<const float2 *>(q + (long long)(c->N - 1) * 2 * M), (long long)c->my * c->mz,
-                c->qpart);
+        plane_q_sums_kernel<<<c->mx, 256, 0, c->st>>>(
+            reinterpret_cast<const float2 *>(q + (long long)(c->N - 1) * 2 * M), (long long)c->my * c->mz,
+            c->qpart);
     } else {
         a.qout = q;
-        launch_plane<T>(c, PLANE_INIT_W, a, 2);
+        launch_plane(c, PLANE_INIT_W, a);
         a.h = q;
         for (int i = 1; i < c->N; i++) {
             const int j = i - 1;
             CK(cudaEventRecord(ev[4 * j], c->st));
-            launch_pencil<T>(c, PENCIL_CONV, pa, 2);
+            launch_pencil(c, PENCIL_CONV, pa);
             CK(cudaEventRecord(ev[4 * j + 1], c->st));
             a.qout = q + (long long)i * 2 * M;
             a.hsel0 = hsel_chain0(c, i);
             a.hsel1 = hsel_chain1(c, i);
             CK(cudaEventRecord(ev[4 * j + 2], c->st));
-            launch_plane<T>(c, i + 1 < c->N ? PLANE_STEP : PLANE_LAST, a, 2);
+            launch_plane(c, i + 1 < c->N ? PLANE_STEP : PLANE_LAST, a);
             CK(cudaEventRecord(ev[4 * j + 3], c->st));
         }
     }
@@ -775,7 +884,7 @@ int profile_chain(lfts_ctx *c, double *ms_plane, double *ms_pencil, double *ms_c
     }
     // the production chain (both streams, PDL), timed as a whole
     CK(cudaEventRecord(ev[0], c->st));
-    enqueue_chain<T>(c);
+    enqueue_chain<float>(c);
     CK(cudaEventRecord(ev[1], c->st));
     CK(cudaEventSynchronize(ev[1]));
     float tc = 0.f;
@@ -783,6 +892,53 @@ int profile_chain(lfts_ctx *c, double *ms_plane, double *ms_pencil, double *ms_c
     for (auto &e : ev) cudaEventDestroy(e);
     *ms_pencil = npe ? pe / npe : 0.0;
     *ms_plane = npl ? pl / npl : 0.0;
+    *ms_chain = tc;
+    return LFTS_OK;
+}
+
+// The chain on one stream with CUDA events around its launches: mean duration
+// per contour step of the kernels over yz planes (y and z lines) and over x
+// lines, both chains per launch; then the production chain timed as a whole.
+template <typename T>
+int profile_chain(lfts_ctx *c, double *ms_plane, double *ms_pencil, double *ms_chain)
+{
+    const int n = c->N - 1;
+    std::vector<cudaEvent_t> ev(3 * n + 2);
+    for (auto &e : ev) CK(cudaEventCreate(&e));
+    AxisArgs<T> a = axis_args<T>(c);
+    set_slot(c, a, 0);
+    launch_yz<T>(c, AX_INIT_W, a, kChains<T>, c->st);
+    for (int i = 1; i <= n; i++) {
+        set_slot(c, a, i);
+        const int mode = i < n ? AX_H : AX_H_LAST;
+        CK(cudaEventRecord(ev[3 * i - 3], c->st));
+        launch_y<T>(c, a, kChains<T>, c->st);
+        CK(cudaEventRecord(ev[3 * i - 2], c->st));
+        if (i & 1)
+            launch_x<T>(c, mode, a, kChains<T>, c->st);
+        else
+            launch_yz<T>(c, mode, a, kChains<T>, c->st);
+        CK(cudaEventRecord(ev[3 * i - 1], c->st));
+    }
+    CK(cudaEventSynchronize(ev[3 * n - 1]));
+    double pl = 0.0, pe = 0.0;
+    for (int i = 1; i <= n; i++) {
+        float ty = 0.f, t = 0.f;
+        if (!axis_of<T>(c).planes) CK(cudaEventElapsedTime(&ty, ev[3 * i - 3], ev[3 * i - 2]));
+        CK(cudaEventElapsedTime(&t, ev[3 * i - 2], ev[3 * i - 1]));
+        pl += ty + (i & 1 ? 0.f : t);
+        pe += i & 1 ? t : 0.f;
+    }
+    // the production chain (streams, PDL), timed as a whole
+    CK(cudaEventRecord(ev[3 * n], c->st));
+    enqueue_chain<T>(c);
+    CK(cudaEventRecord(ev[3 * n + 1], c->st));
+    CK(cudaEventSynchronize(ev[3 * n + 1]));
+    float tc = 0.f;
+    CK(cudaEventElapsedTime(&tc, ev[3 * n], ev[3 * n + 1]));
+    for (auto &e : ev) cudaEventDestroy(e);
+    *ms_pencil = pe / n;
+    *ms_plane = pl / n;
     *ms_chain = tc;
     return LFTS_OK;
 }
@@ -1046,22 +1202,19 @@ int anderson_mix(lfts_ctx *c, int maxIter, double errTol, int *k_out)
 int sk_sample(lfts_ctx *c)
 {
     PlaneArgs<double> a{};
-    a.src64 = c->w;  // W-
-    a.src_stride = 0;
+    a.src = c->w;  // W-
     a.spec = static_cast<cpx<double> *>(c->skspec);
     const bool fp64 = c->prec == LFTS_FP64;
     a.twy = static_cast<const cpx<double> *>(fp64 ? c->tw[1] : c->sktw[1]);
     a.twz = static_cast<const cpx<double> *>(fp64 ? c->tw[2] : c->sktw[2]);
-    a.Nd = (double)c->N;
-    c->pl64.fn[PLANE_INIT_Q]<<<dim3(c->mx, 1), c->pl64.nt, c->pl64.smem, c->st>>>(a);
+    c->fwd_yz.fn<<<dim3(c->mx, 1), c->fwd_yz.nt, c->fwd_yz.smem, c->st>>>(a);
     PencilArgs<double> pa{};
     pa.spec = a.spec;
     pa.twx = static_cast<const cpx<double> *>(fp64 ? c->tw[0] : c->sktw[0]);
     pa.S = c->S;
     pa.ncol = c->my * c->KZ;
-    pa.KZ = c->KZ;
     const int ncol = pa.ncol;
-    c->pe64.fn[PENCIL_POWER]<<<dim3((ncol + c->pe64.cw - 1) / c->pe64.cw, 1), c->pe64.nt, c->pe64.smem, c->st>>>(pa);
+    c->power_x.fn<<<(ncol + c->power_x.cw - 1) / c->power_x.cw, c->power_x.nt, c->power_x.smem, c->st>>>(pa);
     c->launches += 2;
     CK(cudaGetLastError());
     c->nsamples++;
@@ -1123,8 +1276,10 @@ int ctx_alloc(lfts_ctx *c)
     CK(cudaMalloc(&c->w, sizeof(double) * 4 * M));
     CK(cudaMemset(c->w, 0, sizeof(double) * 4 * M));
     CK(cudaMalloc(&c->q, c->tsize * 2 * M * (size_t)c->N));
-    CK(cudaMalloc(&c->spec, c->tsize * 2 * 2 * (size_t)c->mx * c->my * c->KZ));
-    CK(cudaMalloc(&c->qpart, sizeof(double) * c->mx));
+    CK(cudaMalloc(&c->field, c->tsize * 2 * 2 * (size_t)c->mx * c->my * c->KZ));
+    CK(cudaMalloc(&c->qpart, sizeof(double) * kMaxQparts));
+    CK(cudaMalloc(&c->ticket, sizeof(unsigned)));
+    CK(cudaMemset(c->ticket, 0, sizeof(unsigned)));
     CK(cudaMalloc(&c->Qd, sizeof(double) * 2));
     CK(cudaMalloc(&c->partials, sizeof(double) * kRedWidth * c->red_blocks));
     CK(cudaMalloc(&c->red, sizeof(double) * kRedWidth));
@@ -1145,7 +1300,7 @@ int ctx_alloc(lfts_ctx *c)
     CK(cudaMalloc(&c->S, sizeof(double) * c->Mk));
     CK(cudaMemset(c->S, 0, sizeof(double) * c->Mk));
     if (c->prec == LFTS_FP64) {
-        c->skspec = c->spec;
+        c->skspec = c->field;
     } else {
         CK(cudaMalloc(&c->skspec, sizeof(cpx<double>) * (size_t)c->Mk));
         c->sk_own_spec = true;
@@ -1158,13 +1313,14 @@ void ctx_free(lfts_ctx *c)
     if (c->st) cudaStreamSynchronize(c->st);
     cudaFree(c->w);
     cudaFree(c->q);
-    cudaFree(c->spec);
+    cudaFree(c->field);
     for (int d = 0; d < 3; d++) {
         cudaFree(c->tw[d]);
         cudaFree(c->gtab[d]);
         cudaFree(c->sktw[d]);
     }
     cudaFree(c->qpart);
+    cudaFree(c->ticket);
     cudaFree(c->Qd);
     cudaFree(c->partials);
     cudaFree(c->red);
@@ -1225,22 +1381,22 @@ int step_fwd_impl(lfts_ctx *c, const double *q_in, double *q_out, const double *
     T *dst = reinterpret_cast<T *>(dout);
     if (sizeof(T) != sizeof(double)) {
         convert_kernel<double, T><<<stream_grid(c), 256, 0, c->st>>>(dq, tq, 2 * M);
-        to_pairs_kernel<double, T><<<stream_grid(c), 256, 0, c->st>>>(dh, th, M);  // packed-path layout
+        to_pairs_kernel<double, T><<<stream_grid(c), 256, 0, c->st>>>(dh, th, M);  // pairs, as slot 1
         c->launches += 2;
         src = tq;
         hh = th;
         dst = tout;
     }
-    PlaneArgs<T> a = plane_args<T>(c);
-    a.src = src;
-    a.src_stride = M;
-    launch_plane<T>(c, PLANE_INIT_Q, a, 2);
-    launch_pencil<T>(c, PENCIL_CONV, pencil_args<T>(c), 2);
-    a.qout = dst;
+    AxisArgs<T> a = axis_args<T>(c);
+    a.src[0] = src;
+    a.src[1] = src + M;
     a.h = hh;
-    a.hsel0 = hsel_chain0(c, i);
-    a.hsel1 = hsel_chain1(c, i);
-    launch_plane<T>(c, PLANE_LAST, a, 2);
+    a.q[0] = dst;
+    a.q[1] = dst + M;
+    a.hsel[0] = hsel_chain0(c, i);
+    a.hsel[1] = hsel_chain1(c, i);
+    launch_yz<T>(c, AX_INIT_Q, a, kChains<T>, c->st);
+    launch_step<T>(c, 1, AX_OUT, a, kChains<T>, c->st);
     if (sizeof(T) != sizeof(double)) {
         from_pairs_kernel<T, double><<<stream_grid(c), 256, 0, c->st>>>(tout, dout, M);
         c->launches++;
@@ -1259,12 +1415,16 @@ namespace {
 // (chain 1), then the k^2-weighted products summed into c->adj_partial.
 int adjoint_term(lfts_ctx *c, const double *q_i, const double *qh_ip1)
 {
-    PlaneArgs<double> a = plane_args<double>(c);
+    PlaneArgs<double> a{};
     a.src = q_i;
     a.src_stride = (long long)(qh_ip1 - q_i);
-    launch_plane<double>(c, PLANE_INIT_Q, a, 2);
+    a.spec = static_cast<cpx<double> *>(c->field);
+    a.twy = static_cast<const cpx<double> *>(c->tw[1]);
+    a.twz = static_cast<const cpx<double> *>(c->tw[2]);
+    c->fwd_yz.fn<<<dim3(c->mx, 2), c->fwd_yz.nt, c->fwd_yz.smem, c->st>>>(a);
+    c->launches++;
     AdjArgs aa{};
-    aa.spec = static_cast<const cpx<double> *>(c->spec);
+    aa.spec = static_cast<const cpx<double> *>(c->field);
     aa.twx = static_cast<const cpx<double> *>(c->tw[0]);
     aa.gx = static_cast<const double *>(c->gtab[0]);
     aa.gy = static_cast<const double *>(c->gtab[1]);
@@ -1281,59 +1441,32 @@ int adjoint_term(lfts_ctx *c, const double *q_i, const double *qh_ip1)
 }
 
 // Propagators of both chains with q stored only at monomers 1, 1+K, 1+2K, ...
-// (q^ in full); returns after Q is reduced.  Chains run as separate launches
-// so each output can be placed independently.
+// (q^ in full); returns after Q is reduced.
 int chain_checkpointed(lfts_ctx *c, int K)
 {
-    double *q = static_cast<double *>(c->q);
-    const long long M = c->M;
-    double *discard = c->adj_buf + (long long)K * M;
-    PlaneArgs<double> a = plane_args<double>(c);
-    PencilArgs<double> pa = pencil_args<double>(c);
-    a.qout = q;
-    launch_plane<double>(c, PLANE_INIT_W, a, 2);  // slot 1 = [hA | hB]
-    a.h = q;
-    PlaneArgs<double> a0 = a, a1 = a;
-    PencilArgs<double> p0 = pa, p1 = pa;
-    a0.cbase = 0;
-    a1.cbase = 1;
-    p0.cbase = 0;
-    p1.cbase = 1;
+    AxisArgs<double> a = axis_args<double>(c);
+    set_slot(c, a, 0);
+    launch_yz<double>(c, AX_INIT_W, a, 2, c->st);  // slot 1 = [hA | hB]
     for (int i = 1; i < c->N; i++) {
-        launch_pencil<double>(c, PENCIL_CONV, p0, 1);
-        launch_pencil<double>(c, PENCIL_CONV, p1, 1);
-        const int mode = i + 1 < c->N ? PLANE_STEP : PLANE_LAST;
-        a0.hsel0 = a1.hsel0 = hsel_chain0(c, i);
-        a0.hsel1 = a1.hsel1 = hsel_chain1(c, i);
-        // q_{i+1}: a checkpoint slot or the discard row (chain 0 writes qout + 0)
-        a0.qout = (i % K == 0) ? q + (long long)i * 2 * M : discard;
-        a1.qout = q + (long long)i * 2 * M;  // q^_{N-i}: second half of slot i+1
-        launch_plane<double>(c, mode, a0, 1);
-        launch_plane<double>(c, mode, a1, 1);
+        set_slot(c, a, i);
+        if (i % K) a.q[0] = nullptr;
+        launch_step<double>(c, i, i + 1 < c->N ? AX_H : AX_H_LAST, a, 2, c->st);
     }
-    q_finalize_kernel<<<1, 256, 0, c->st>>>(c->qpart, c->mx, M, c->Qd);
-    c->launches++;
     return LFTS_OK;
 }
 
 // q_{c0+1} .. q_{c0+n} recomputed from the checkpoint q_{c0} into adj_buf rows 1..n
 void recompute_segment(lfts_ctx *c, const double *q_c0, int c0, int n)
 {
-    const long long M = c->M;
-    PlaneArgs<double> a = plane_args<double>(c);
-    PencilArgs<double> pa = pencil_args<double>(c);
-    a.cbase = 0;
-    pa.cbase = 0;
-    a.src = q_c0;
-    a.src_stride = 0;
-    launch_plane<double>(c, PLANE_INIT_Q, a, 1);
-    a.h = static_cast<double *>(c->q);
+    AxisArgs<double> a = axis_args<double>(c);
+    a.src[0] = q_c0;
+    a.ticket = nullptr;
+    launch_yz<double>(c, AX_INIT_Q, a, 1, c->st);
     for (int j = 1; j <= n; j++) {
-        const int i = c0 + j - 1;  // step i makes q_{i+1}
-        launch_pencil<double>(c, PENCIL_CONV, pa, 1);
-        a.hsel0 = hsel_chain0(c, i);
-        a.qout = c->adj_buf + (long long)j * M;
-        launch_plane<double>(c, PLANE_STEP, a, 1);
+        const int i = c0 + j - 1;  // monomer step i makes q_{i+1}
+        a.hsel[0] = hsel_chain0(c, i);
+        a.q[0] = c->adj_buf + (long long)j * c->M;
+        launch_step<double>(c, j, j < n ? AX_H : AX_H_LAST, a, 1, c->st);
     }
 }
 
@@ -1428,21 +1561,13 @@ int lfts_create(const lfts_params *p, int precision, int device, lfts_ctx **out)
         cudaEventCreateWithFlags(&c->ev_h[0], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_h[1], cudaEventDisableTiming) != cudaSuccess)
         return fail(LFTS_ERR_CUDA);
-    if (!plane_kernels(c->my, c->mz, &c->pl64) || !pencil_kernels(c->mx, &c->pe64)) return fail(LFTS_ERR_UNSUPPORTED);
-    if ((rc = set_smem_attrs(c->pl64, c->pe64))) return fail(rc);
-    if (precision == LFTS_FP32_MIXED) {
-        c->packed = true;
-        if (plane3_kernels(c->my, c->mz, &c->pl32))
-            c->plane_stages = 3;
-        else if (!plane_c_kernels(c->my, c->mz, &c->pl32))
-            return fail(LFTS_ERR_UNSUPPORTED);
-        if (!pencil_kernels(c->mx, kDefaultCwFp32, &c->pe32)) return fail(LFTS_ERR_UNSUPPORTED);
-        // h and the stored propagators in the x-pencil where both kernels have
-        // those modes (128^3); LFTS_XH_CHAIN=0 keeps them in the yz-plane kernel
-        const char *xh = getenv("LFTS_XH_CHAIN");
-        c->xh_chain = c->pl32.fn[PLANE_G] && c->pe32.fn[PENCIL_H] && !(xh && xh[0] == '0');
-        if ((rc = set_smem_attrs(c->pl32, c->pe32))) return fail(rc);
-    }
+    if (!fwd_plane_kernel(c->my, c->mz, &c->fwd_yz) || !power_pencil_kernel(c->mx, &c->power_x))
+        return fail(LFTS_ERR_UNSUPPORTED);
+    if (cudaFuncSetAttribute(c->fwd_yz.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->fwd_yz.smem) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(c->power_x.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->power_x.smem) !=
+            cudaSuccess)
+        return fail(LFTS_ERR_CUDA);
     if ((rc = ctx_alloc(c))) return fail(rc == LFTS_ERR_CUDA ? LFTS_ERR_NOMEM : rc);
     if (precision == LFTS_FP64)
         rc = upload_tables<double>(c, c->tw, c->gtab);
@@ -1451,6 +1576,7 @@ int lfts_create(const lfts_params *p, int precision, int device, lfts_ctx **out)
         if (!rc) rc = upload_tables<double>(c, c->sktw, nullptr);
     }
     if (rc) return fail(rc);
+    if (precision == LFTS_FP32_MIXED && (rc = set_axis<float>(c, kDefaultCwFp32))) return fail(rc);  // step_fwd
     if ((rc = autotune(c))) return fail(rc);
     *out = c;
     return LFTS_OK;
@@ -1716,11 +1842,11 @@ int lfts_backward(lfts_ctx *c, int ckpt_every, double *dH_dL, double *dH_dXbN, d
         for (int i = 1; i < N; i++) adjoint_term(c, q + (long long)(i - 1) * 2 * M, qh(i + 1));
     } else {
         const int K = ckpt_every;
-        if (c->adj_buf_slots < K + 1) {
+        if (c->adj_buf_slots < K) {
             cudaFree(c->adj_buf);
             c->adj_buf = nullptr;
-            CK(cudaMalloc(&c->adj_buf, sizeof(double) * (size_t)(K + 1) * M));
-            c->adj_buf_slots = K + 1;
+            CK(cudaMalloc(&c->adj_buf, sizeof(double) * (size_t)K * M));
+            c->adj_buf_slots = K;
         }
         chain_checkpointed(c, K);
         for (int c0 = 1; c0 < N; c0 += K) {
@@ -1767,6 +1893,7 @@ int lfts_profile_chain(lfts_ctx *c, double *ms_plane, double *ms_pencil, double 
     DeviceGuard g(c->dev);
     CK(cudaStreamSynchronize(c->st));
     if (c->prec == LFTS_FP64) return profile_chain<double>(c, ms_plane, ms_pencil, ms_chain);
+    if (c->transform_chain) return profile_transform_chain(c, ms_plane, ms_pencil, ms_chain);
     return profile_chain<float>(c, ms_plane, ms_pencil, ms_chain);
 }
 
@@ -1832,7 +1959,7 @@ int lfts_profile_iteration(lfts_ctx *c, int reps, double *ms_chain, double *ms_c
 int lfts_get_tiles(const lfts_ctx *c, lfts_tiles *out)
 {
     if (!c || !out) return LFTS_ERR_ARG;
-    *out = current_tiles(c);
+    *out = c->tiles;
     return LFTS_OK;
 }
 
@@ -1842,20 +1969,16 @@ int lfts_set_tiles(lfts_ctx *c, const lfts_tiles *t)
     DeviceGuard g(c->dev);
     CK(cudaStreamSynchronize(c->st));
     CK(cudaStreamSynchronize(c->st1));
-    const lfts_tiles old = current_tiles(c);
-    int rc = apply_tiles(c, *t);
-    if (rc) {
-        apply_tiles(c, old);  // leave the context as it was
-        g_last_error = "tile choice not valid for this context's precision and mesh";
-    }
+    int rc = apply_tiles(c, *t);  // an invalid choice leaves the context as it was
+    if (rc) g_last_error = "tile choice not valid for this context's precision and mesh";
     return rc;
 }
 
 int lfts_tuning(const lfts_ctx *c, int *pencil_cw, int *plane_stages)
 {
     if (!c) return LFTS_ERR_ARG;
-    if (pencil_cw) *pencil_cw = c->prec == LFTS_FP64 ? c->pe64.cw : c->pe32.cw;
-    if (plane_stages) *plane_stages = c->prec == LFTS_FP64 ? 2 : c->plane_stages;
+    if (pencil_cw) *pencil_cw = c->tiles.pencil_cw;
+    if (plane_stages) *plane_stages = c->tiles.plane_stages;
     return LFTS_OK;
 }
 

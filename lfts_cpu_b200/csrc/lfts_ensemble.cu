@@ -701,7 +701,7 @@ int lfts_ensemble_create(const lfts_params *params, const unsigned long long *se
         R.seed = seeds[r];
         R.w = c->w;
         R.q = static_cast<float *>(c->q);
-        R.spec = static_cast<cpx<float> *>(c->spec);
+        R.spec = static_cast<cpx<float> *>(c->field);
         for (int d = 0; d < 3; d++) {
             R.tw[d] = static_cast<const cpx<float> *>(c->tw[d]);
             R.g[d] = static_cast<const float *>(c->gtab[d]);

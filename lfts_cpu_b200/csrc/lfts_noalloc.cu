@@ -3,8 +3,8 @@
 // (a host framework that owns every device allocation through its own pool,
 // a real-time loop that may not call into the allocator, or a library layered
 // under an allocator-free API).  The caller passes device inputs and outputs;
-// the step's scratch (the two chains' half spectra, the per-plane Q partial
-// sums and the twiddle / Boltzmann-weight tables) lives in one file-scope
+// the step's scratch (the two chains' fields and the twiddle / Boltzmann-weight
+// tables) lives in one file-scope
 // device array of fixed size, so this path makes no allocation at all.
 //
 // Limits and sharing rules, stated once here and in include/lfts_b200.h:
@@ -15,8 +15,7 @@
 //    kernels overlap on a GPU (different streams, or different host threads)
 //    race on it.  Serialise them (one stream, or events).
 //  * Nothing in the array has to start at zero: every call rewrites the tables
-//    and the spectrum before reading them, and each plane's Q partial is
-//    written before it is read.  The array keeps the last call's contents.
+//    and the fields before reading them.  The array keeps the last call's contents.
 //  * The first call on a device looks up the array's device address (with
 //    that device current); make that first call before any stream capture.
 #include <cmath>
@@ -27,7 +26,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/lfts_b200.h"
-#include "fft_dispatch.h"
+#include "axis_dispatch.h"
 
 using namespace lfts;
 
@@ -43,8 +42,7 @@ struct NoallocLayout {
     static constexpr size_t spec = 0;
     static constexpr size_t tw = spec + sizeof(cpx<double>) * kMaxSpec;      // 3 x kMaxLen complex
     static constexpr size_t g = tw + sizeof(cpx<double>) * 3 * kMaxLen;      // 3 x kMaxLen doubles
-    static constexpr size_t qpart = g + sizeof(double) * 3 * kMaxLen;        // kMaxLen doubles
-    static constexpr size_t bytes = qpart + sizeof(double) * kMaxLen;
+    static constexpr size_t bytes = g + sizeof(double) * 3 * kMaxLen;
 };
 
 // the scratch: one per device, shared by all calls (see the rules above)
@@ -74,9 +72,8 @@ __global__ void noalloc_tables_kernel(cpx<double> *tw, double *g, int mx, int my
             sincospi(-2.0 * t / n[d], &s, &c);
             tw[d * kMaxLen + t] = {c, s};
         }
-        const int len = (d == 2) ? n[2] / 2 + 1 : n[d];
-        for (int K = threadIdx.x; K < len; K += blockDim.x) {
-            const int k = (d == 2 || K <= n[d] / 2) ? K : K - n[d];
+        for (int K = threadIdx.x; K < n[d]; K += blockDim.x) {
+            const int k = K <= n[d] / 2 ? K : K - n[d];
             const double ksq = (double)k * k / (L[d] * L[d]);
             double v = exp(-two_pi * two_pi * ksq / (6.0 * N));
             if (d == 2) v /= M;
@@ -92,9 +89,8 @@ int fail(int code, const char *msg)
 }
 
 // Per-device set-up, done by the first call on each device with that device
-// current: the scratch array's device address.  Then, every call, the
-// dynamic shared-memory limits of the kernels this mesh uses.
-int device_setup(int dev, const PlaneKernels<double> &pl, const PencilKernels<double> &pe)
+// current: the scratch array's device address.
+int device_setup(int dev)
 {
     std::call_once(g_scratch_once[dev], [dev] {
         void *p = nullptr;
@@ -103,13 +99,16 @@ int device_setup(int dev, const PlaneKernels<double> &pl, const PencilKernels<do
     });
     if (g_scratch_err[dev] != cudaSuccess || !g_scratch_addr[dev])
         return fail(LFTS_ERR_CUDA, "cudaGetSymbolAddress(g_step_scratch) failed");
-    for (int m = 0; m < 4; m++)
-        if (cudaFuncSetAttribute(pl.fn[m], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem) != cudaSuccess)
-            return fail(LFTS_ERR_CUDA, "cudaFuncSetAttribute failed");
-    for (int m = 0; m < 2; m++)
-        if (cudaFuncSetAttribute(pe.fn[m], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pe.smem) != cudaSuccess)
-            return fail(LFTS_ERR_CUDA, "cudaFuncSetAttribute failed");
     return LFTS_OK;
+}
+
+// one launch of the step, with the kernel's dynamic shared-memory limit
+bool launch(const AxisFn<double> &f, dim3 grid, cudaStream_t st, const AxisArgs<double> &a)
+{
+    if (cudaFuncSetAttribute(f.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem) != cudaSuccess)
+        return false;
+    f.fn<<<grid, f.nt, f.smem, st>>>(a);
+    return true;
 }
 
 }  // namespace
@@ -132,53 +131,56 @@ int lfts_step_fwd_noalloc(const lfts_params *p, const double *q_in, double *q_ou
     if (2LL * mx * my * KZ > kMaxSpec)
         return fail(LFTS_ERR_ARG, "mesh above the no-alloc scratch limit: 2*mx*my*(mz/2+1) must be <= "
                                   "LFTS_NOALLOC_MAX_SPECTRUM (64^3 meshes fit)");
-    PlaneKernels<double> pl{};
-    PencilKernels<double> pe{};
-    if (!plane_kernels(my, mz, &pl) || !pencil_kernels(mx, &pe))
+    AxisSet<double> ax;
+    if (!axis_kernels(mx, my, mz, kLastCw, &ax))
         return fail(LFTS_ERR_UNSUPPORTED, "mesh size without an FFT kernel");
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices)
         return fail(LFTS_ERR_CUDA, "no current CUDA device");
-    int rc = device_setup(dev, pl, pe);
+    int rc = device_setup(dev);
     if (rc) return rc;
 
     unsigned char *base = g_scratch_addr[dev];
-    cpx<double> *spec = reinterpret_cast<cpx<double> *>(base + NoallocLayout::spec);
     cpx<double> *tw = reinterpret_cast<cpx<double> *>(base + NoallocLayout::tw);
     double *g = reinterpret_cast<double *>(base + NoallocLayout::g);
-    double *qpart = reinterpret_cast<double *>(base + NoallocLayout::qpart);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const long long M = (long long)mx * my * mz;
     const int NB = p->N - p->NA;
 
     noalloc_tables_kernel<<<1, 128, 0, st>>>(tw, g, mx, my, mz, p->L[0], p->L[1], p->L[2], p->N, (double)M);
 
-    PlaneArgs<double> a{};
-    a.src = q_in;
-    a.src_stride = M;
-    a.spec = spec;
+    AxisArgs<double> a{};
+    a.S = reinterpret_cast<double *>(base + NoallocLayout::spec);
+    a.twx = tw;
     a.twy = tw + kMaxLen;
     a.twz = tw + 2 * kMaxLen;
-    a.qpart = qpart;
-    a.nchains = 2;
+    a.gx = g;
+    a.gy = g + kMaxLen;
+    a.gz = g + 2 * kMaxLen;
+    a.mx = mx;
+    a.my = my;
+    a.mz = mz;
+    a.M = M;
     a.Nd = (double)p->N;
-    pl.fn[PLANE_INIT_Q]<<<dim3(mx, 2), pl.nt, pl.smem, st>>>(a);
-
-    PencilArgs<double> pa{};
-    pa.spec = spec;
-    pa.twx = tw;
-    pa.gx = g;
-    pa.gy = g + kMaxLen;
-    pa.gz = g + 2 * kMaxLen;
-    pa.ncol = my * (int)KZ;
-    pa.KZ = (int)KZ;
-    pe.fn[PENCIL_CONV]<<<dim3((pa.ncol + pe.cw - 1) / pe.cw, 2), pe.nt, pe.smem, st>>>(pa);
-
-    a.qout = q_out;
+    a.src[0] = q_in;
+    a.src[1] = q_in + M;
     a.h = h;
-    a.hsel0 = i < p->NA ? 0 : 1;  // src/step.cc:53-57
-    a.hsel1 = i < NB ? 1 : 0;     // src/step.cc:60-64
-    pl.fn[PLANE_LAST]<<<dim3(mx, 2), pl.nt, pl.smem, st>>>(a);
+    a.q[0] = q_out;
+    a.q[1] = q_out + M;
+    a.hsel[0] = i < p->NA ? 0 : 1;  // src/step.cc:53-57
+    a.hsel[1] = i < NB ? 1 : 0;     // src/step.cc:60-64
+    // z and y lines, then x lines and the product with h (axis_conv.cuh)
+    bool ok;
+    if (ax.planes) {
+        ok = launch(ax.plane[AX_INIT_Q], dim3(mx, 1, 2), st, a);
+    } else {
+        const AxisFn<double> &z = ax.z[AX_INIT_Q];
+        ok = launch(z, dim3((mx * my / 2 + z.per - 1) / z.per, 1, 2), st, a) &&
+             launch(ax.y, dim3((mz / 2 + ax.y.per - 1) / ax.y.per, mx, 2), st, a);
+    }
+    const AxisFn<double> &x = ax.x[AX_OUT];
+    ok = ok && launch(x, dim3((my * mz / 2 + x.per - 1) / x.per, 1, 2), st, a);
+    if (!ok) return fail(LFTS_ERR_CUDA, "cudaFuncSetAttribute failed");
 
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(LFTS_ERR_CUDA, cudaGetErrorString(e));
