@@ -86,13 +86,77 @@ template <> struct AxPlan<80> { static constexpr int R1 = 10, R2 = 8; };
 template <> struct AxPlan<96> { static constexpr int R1 = 12, R2 = 8; };
 template <> struct AxPlan<128> { static constexpr int R1 = 16, R2 = 8; };
 
+// z lines apart (zline_kernel): R1, R2 and the lines a warp works on
+template <int N>
+struct AxPlanZ {
+    static constexpr int R1 = AxPlan<N>::R1, R2 = AxPlan<N>::R2, LPW = 32 / R2;
+};
+// 128: 16 lanes of a warp then take 16 neighbouring points, a whole 128-byte row
+// (FP32; Z kernel 11.7 -> 10.0 us with lines of 128^3; at 80 and 96 the wider
+// stage B costs more than the rows give: 4.6 -> 5.2, 6.3 -> 6.5 us)
+template <> struct AxPlanZ<128> { static constexpr int R1 = 8, R2 = 16, LPW = 4; };
+
+// R values of a 16-byte aligned shared-memory row, read 16 bytes at a time (the
+// row is padded to whole 16 bytes)
+template <int R, typename E>
+__device__ __forceinline__ void ax_row(const E *row, E (&out)[R])
+{
+    constexpr int V = 16 / (int)sizeof(E);
+#pragma unroll
+    for (int i = 0; i < (R + V - 1) / V; i++) {
+        const float4 q = reinterpret_cast<const float4 *>(row)[i];
+        const E *e = reinterpret_cast<const E *>(&q);
+#pragma unroll
+        for (int j = 0; j < V; j++)
+            if (V * i + j < R) out[V * i + j] = e[j];
+    }
+}
+
+// Axis tables in shared memory, a row per k1: twiddles exp(-2 pi i k1 u/n) over
+// u, then g(k1 + R1 k2) over k2.  The twiddles are applied in stage B, where a
+// task needs R2 of them for both directions, and not in stage A, which would read
+// R1 for each; rows are an odd number of 16-byte units, so that lanes on
+// different rows read different banks.
+template <typename T, int R1, int R2>
+struct AxTables {
+    static constexpr int N = R1 * R2;
+    static constexpr int TP = (R2 * (int)sizeof(cpx<T>) + 15) / 16 | 1, GP = (R2 * (int)sizeof(T) + 15) / 16 | 1;
+    static constexpr size_t BYTES = 16 * (size_t)R1 * (TP + GP);
+    unsigned char *at;
+    __device__ __forceinline__ cpx<T> *tw(int k1) const { return reinterpret_cast<cpx<T> *>(at + 16 * k1 * TP); }
+    __device__ __forceinline__ T *g(int k1) const { return reinterpret_cast<T *>(at + 16 * (R1 * TP + k1 * GP)); }
+    __device__ __forceinline__ void load(const cpx<T> *__restrict__ twg, const T *__restrict__ gg, int tid, int nt)
+    {
+        for (int i = tid; i < N; i += nt) {
+            const int k1 = i % R1, r = i / R1;
+            tw(k1)[r] = twg[k1 * r];
+            g(k1)[r] = gg[i];
+        }
+    }
+    // stage B of one task: v[u], the inputs of outputs k1 + R1 k2, there and back
+    __device__ __forceinline__ void convolve(cpx<T> (&v)[R2], int k1) const
+    {
+        cpx<T> w[R2];
+        T gk[R2];
+        ax_row(tw(k1), w);
+        ax_row(g(k1), gk);
+#pragma unroll
+        for (int u = 1; u < R2; u++) v[u] = ctw<-1>(v[u], w[u]);
+        Dft<R2, -1, T>::run(v);
+#pragma unroll
+        for (int k2 = 0; k2 < R2; k2++) v[k2] = cscale(v[k2], gk[k2]);
+        Dft<R2, 1, T>::run(v);
+#pragma unroll
+        for (int u = 1; u < R2; u++) v[u] = ctw<1>(v[u], w[u]);
+    }
+};
+
 // One group of threads (a block or a warp) convolving NL lines of N points.
 // LF: neighbouring threads take neighbouring lines (strided axes), else
 // neighbouring points of one line (the contiguous axis).  Idx maps (line,
 // point) to shared memory.
-template <typename T, int N, int NL, int NTG, bool LF, class Idx>
+template <typename T, int R1, int R2, int NL, int NTG, bool LF, class Idx>
 struct LineConv {
-    static constexpr int R1 = AxPlan<N>::R1, R2 = AxPlan<N>::R2;
     static constexpr int RA = (NL * R2 + NTG - 1) / NTG, RB = (NL * R1 + NTG - 1) / NTG;
     static __device__ __forceinline__ bool okA(int t) { return (NL * R2) % NTG == 0 || t < NL * R2; }
     static __device__ __forceinline__ bool okB(int t) { return (NL * R1) % NTG == 0 || t < NL * R1; }
@@ -101,8 +165,8 @@ struct LineConv {
     static __device__ __forceinline__ int lineB(int t) { return LF ? t % NL : t / R1; }
     static __device__ __forceinline__ int ptB(int t) { return LF ? t / NL : t % R1; }
 
-    // stage A: DFT, twiddles, to shared memory.  tw: [j2][k1], pitch R1 + 1
-    static __device__ __forceinline__ void A(cpx<T> (&v)[RA][R1], cpx<T> *sm, const cpx<T> *tw, int tid)
+    // stage A: DFT, to shared memory
+    static __device__ __forceinline__ void A(cpx<T> (&v)[RA][R1], cpx<T> *sm, int tid)
     {
 #pragma unroll
         for (int s = 0; s < RA; s++) {
@@ -111,12 +175,11 @@ struct LineConv {
             const int l = lineA(t), j2 = ptA(t);
             Dft<R1, -1, T>::run(v[s]);
 #pragma unroll
-            for (int k1 = 0; k1 < R1; k1++)
-                sm[Idx::at(l, j2 + R2 * k1)] = k1 ? ctw<-1>(v[s][k1], tw[j2 * (R1 + 1) + k1]) : v[s][k1];
+            for (int k1 = 0; k1 < R1; k1++) sm[Idx::at(l, j2 + R2 * k1)] = v[s][k1];
         }
     }
-    // stage B in place: spectrum times g, and back
-    static __device__ __forceinline__ void B(cpx<T> *sm, const T *g, int tid)
+    // stage B in place: twiddles, spectrum times g, and back
+    static __device__ __forceinline__ void B(cpx<T> *sm, const AxTables<T, R1, R2> &tab, int tid)
     {
 #pragma unroll
         for (int s = 0; s < RB; s++) {
@@ -126,16 +189,13 @@ struct LineConv {
             cpx<T> v[R2];
 #pragma unroll
             for (int u = 0; u < R2; u++) v[u] = sm[Idx::at(l, R2 * k1 + u)];
-            Dft<R2, -1, T>::run(v);
-#pragma unroll
-            for (int k2 = 0; k2 < R2; k2++) v[k2] = cscale(v[k2], g[k1 + R1 * k2]);
-            Dft<R2, 1, T>::run(v);
+            tab.convolve(v, k1);
 #pragma unroll
             for (int u = 0; u < R2; u++) sm[Idx::at(l, R2 * k1 + u)] = v[u];
         }
     }
     // stage A back: v[s][j1] = the line's point j2 + R2 j1
-    static __device__ __forceinline__ void Ainv(cpx<T> (&v)[RA][R1], const cpx<T> *sm, const cpx<T> *tw, int tid)
+    static __device__ __forceinline__ void Ainv(cpx<T> (&v)[RA][R1], const cpx<T> *sm, int tid)
     {
 #pragma unroll
         for (int s = 0; s < RA; s++) {
@@ -143,36 +203,9 @@ struct LineConv {
             if (!okA(t)) continue;
             const int l = lineA(t), j2 = ptA(t);
 #pragma unroll
-            for (int k1 = 0; k1 < R1; k1++) {
-                const cpx<T> x = sm[Idx::at(l, j2 + R2 * k1)];
-                v[s][k1] = k1 ? ctw<1>(x, tw[j2 * (R1 + 1) + k1]) : x;
-            }
+            for (int k1 = 0; k1 < R1; k1++) v[s][k1] = sm[Idx::at(l, j2 + R2 * k1)];
             Dft<R1, 1, T>::run(v[s]);
         }
-    }
-};
-
-// axis tables in shared memory: twiddles [j2][k1] (pitch R1 + 1), then g
-template <typename T, int N>
-struct AxTables {
-    static constexpr int R1 = AxPlan<N>::R1, R2 = AxPlan<N>::R2;
-    static constexpr int NTW = R2 * (R1 + 1);
-    static constexpr size_t BYTES = (sizeof(cpx<T>) * NTW + sizeof(T) * N + 15) / 16 * 16;
-    static __device__ __forceinline__ void load(unsigned char *at, const cpx<T> *__restrict__ tw,
-                                                const T *__restrict__ g, int tid, int nt)
-    {
-        cpx<T> *t = reinterpret_cast<cpx<T> *>(at);
-        T *gs = reinterpret_cast<T *>(t + NTW);
-        for (int i = tid; i < R1 * R2; i += nt) t[(i / R1) * (R1 + 1) + i % R1] = tw[(i / R1) * (i % R1)];
-        for (int i = tid; i < N; i += nt) gs[i] = g[i];
-    }
-    static __device__ __forceinline__ const cpx<T> *tw(const unsigned char *at)
-    {
-        return reinterpret_cast<const cpx<T> *>(at);
-    }
-    static __device__ __forceinline__ const T *g(const unsigned char *at)
-    {
-        return reinterpret_cast<const T *>(reinterpret_cast<const cpx<T> *>(at) + NTW);
     }
 };
 
@@ -391,9 +424,10 @@ struct StridedCfg {
     struct Idx {
         static __device__ __forceinline__ int at(int l, int p) { return (p + PADROW * (p / R2)) * CW + l; }
     };
-    static constexpr size_t TILE = sizeof(cpx<T>) * (size_t)CW * (N + PADROW * (N / R2));
-    static constexpr size_t SMEM = TILE + AxTables<T, N>::BYTES;
-    using Conv = LineConv<T, N, CW, NT, true, Idx>;
+    static constexpr size_t TILE = (sizeof(cpx<T>) * (size_t)CW * (N + PADROW * (N / R2)) + 15) / 16 * 16;
+    using Tables = AxTables<T, R1, R2>;
+    static constexpr size_t SMEM = TILE + Tables::BYTES;
+    using Conv = LineConv<T, R1, R2, CW, NT, true, Idx>;
 };
 
 template <typename T, int N, int CW, int MODE>
@@ -407,9 +441,9 @@ __device__ __forceinline__ void strided_body(const AxisArgs<T> &a, const cpx<T> 
     constexpr bool kLast = MODE == AX_H_LAST || MODE == AX_HA_LAST;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cpx<T> *sm = reinterpret_cast<cpx<T> *>(smem_raw);
-    unsigned char *tab = smem_raw + C::TILE;
     const int tid = threadIdx.x, col0 = tile * CW;
-    AxTables<T, N>::load(tab, twg, gg, tid, C::NT);
+    typename C::Tables tab{smem_raw + C::TILE};
+    tab.load(twg, gg, tid, C::NT);
     pdl_wait();
 
     // complex value of stage-A task t's point j
@@ -424,9 +458,7 @@ __device__ __forceinline__ void strided_body(const AxisArgs<T> &a, const cpx<T> 
         for (int j = 0; j < C::R1; j++) v[s][j] = live(t) ? S[at(t, j)] : cpx<T>{(T)0, (T)0};
     }
     __syncthreads();
-    const cpx<T> *tw = AxTables<T, N>::tw(tab);
-    const T *g = AxTables<T, N>::g(tab);
-    V::A(v, sm, tw, tid);
+    V::A(v, sm, tid);
     // h comes in while stage B works from shared memory: the registers that
     // held the line's points are free until Ainv
     cpx<T> h[kH ? V::RA : 1][C::R1];
@@ -440,9 +472,9 @@ __device__ __forceinline__ void strided_body(const AxisArgs<T> &a, const cpx<T> 
         }
     }
     __syncthreads();
-    V::B(sm, g, tid);
+    V::B(sm, tab, tid);
     __syncthreads();
-    V::Ainv(v, sm, tw, tid);
+    V::Ainv(v, sm, tid);
     if constexpr (kH) {
         double qs = 0.0;
 #pragma unroll
@@ -462,11 +494,11 @@ __device__ __forceinline__ void strided_body(const AxisArgs<T> &a, const cpx<T> 
             return;
         }
         if constexpr (MODE == AX_OUT) return;
-        V::A(v, sm, tw, tid);
+        V::A(v, sm, tid);
         __syncthreads();
-        V::B(sm, g, tid);
+        V::B(sm, tab, tid);
         __syncthreads();
-        V::Ainv(v, sm, tw, tid);
+        V::Ainv(v, sm, tid);
     }
     pdl_launch_dependents();
 #pragma unroll
@@ -508,8 +540,8 @@ __global__ void __launch_bounds__(StridedCfg<T, N, CW>::NT) yline_kernel(AxisArg
 // z lines, LPW whole lines per warp, so the exchanges need no block barrier
 template <typename T, int N>
 struct ZCfg {
-    static constexpr int R1 = AxPlan<N>::R1, R2 = AxPlan<N>::R2;
-    static constexpr int LPW = 32 / R2 < 1 ? 1 : 32 / R2;  // stage A: one task per lane
+    static constexpr int R1 = AxPlanZ<N>::R1, R2 = AxPlanZ<N>::R2;
+    static constexpr int LPW = AxPlanZ<N>::LPW;
     static constexpr int NW = 4, NT = 32 * NW;
     // one pad slot per R2 points: stage B's tasks, R2 apart, start on different banks
     static constexpr int SPAN = N + N / R2;
@@ -517,9 +549,10 @@ struct ZCfg {
     struct Idx {
         static __device__ __forceinline__ int at(int l, int p) { return l * PITCH + p + p / R2; }
     };
-    static constexpr size_t TILE = sizeof(cpx<T>) * (size_t)NW * LPW * PITCH;
-    static constexpr size_t SMEM = TILE + AxTables<T, N>::BYTES;
-    using Conv = LineConv<T, N, LPW, 32, false, Idx>;
+    static constexpr size_t TILE = (sizeof(cpx<T>) * (size_t)NW * LPW * PITCH + 15) / 16 * 16;
+    using Tables = AxTables<T, R1, R2>;
+    static constexpr size_t SMEM = TILE + Tables::BYTES;
+    using Conv = LineConv<T, R1, R2, LPW, 32, false, Idx>;
     static_assert(PITCH >= SPAN, "pitch covers the padded line");
 };
 
@@ -534,10 +567,10 @@ __device__ __forceinline__ void zline_body(const AxisArgs<T> &a, const int cta, 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     cpx<T> *sm = reinterpret_cast<cpx<T> *>(smem_raw) + wid * C::LPW * C::PITCH;
-    unsigned char *tab = smem_raw + C::TILE;
     const int nlines = a.mx * a.my / kChains<T>;
     const int line0 = (cta * C::NW + wid) * C::LPW;
-    AxTables<T, N>::load(tab, a.twz, a.gz, threadIdx.x, C::NT);
+    typename C::Tables tab{smem_raw + C::TILE};
+    tab.load(a.twz, a.gz, threadIdx.x, C::NT);
     pdl_wait();
 
     auto live = [&](int t) { return V::okA(t) && line0 + V::lineA(t) < nlines; };
@@ -561,9 +594,7 @@ __device__ __forceinline__ void zline_body(const AxisArgs<T> &a, const int cta, 
         }
     }
     __syncthreads();
-    const cpx<T> *tw = AxTables<T, N>::tw(tab);
-    const T *g = AxTables<T, N>::g(tab);
-    V::A(v, sm, tw, lane);
+    V::A(v, sm, lane);
     cpx<T> h[kInit ? 1 : V::RA][C::R1];  // as in strided_body
     if constexpr (!kInit) {
 #pragma unroll
@@ -575,9 +606,9 @@ __device__ __forceinline__ void zline_body(const AxisArgs<T> &a, const int cta, 
         }
     }
     __syncwarp();
-    V::B(sm, g, lane);
+    V::B(sm, tab, lane);
     __syncwarp();
-    V::Ainv(v, sm, tw, lane);
+    V::Ainv(v, sm, lane);
     if constexpr (!kInit) {
         double qs = 0.0;
 #pragma unroll
@@ -596,11 +627,11 @@ __device__ __forceinline__ void zline_body(const AxisArgs<T> &a, const int cta, 
             if (a.ticket && c == 0) ax_q_sum<C::NT>(qs, a.qpart, a.ticket, a.Qd, (double)a.M, cta, nctas);
             return;
         }
-        V::A(v, sm, tw, lane);
+        V::A(v, sm, lane);
         __syncwarp();
-        V::B(sm, g, lane);
+        V::B(sm, tab, lane);
         __syncwarp();
-        V::Ainv(v, sm, tw, lane);
+        V::Ainv(v, sm, lane);
     }
     pdl_launch_dependents();
 #pragma unroll
@@ -637,8 +668,10 @@ struct PlaneAxCfg {
     static constexpr int PITCH = (SPAN + 3) / 8 * 8 + 4;
     static __device__ __forceinline__ int zpos(int z) { return z + z / RZ2; }
     static __device__ __forceinline__ int ypos(int y) { return y * PITCH + 4 * (y / RY2); }
-    static constexpr size_t TILE = sizeof(cpx<T>) * (size_t)(NY * PITCH + 4 * (NY / RY2));
-    static constexpr size_t SMEM = TILE + AxTables<T, NY>::BYTES + AxTables<T, NZ>::BYTES;
+    static constexpr size_t TILE = (sizeof(cpx<T>) * (size_t)(NY * PITCH + 4 * (NY / RY2)) + 15) / 16 * 16;
+    using TabY = AxTables<T, RY1, RY2>;
+    using TabZ = AxTables<T, RZ1, RZ2>;
+    static constexpr size_t SMEM = TILE + TabY::BYTES + TabZ::BYTES;
     static_assert(PITCH >= SPAN, "pitch covers the padded row");
 };
 
@@ -652,13 +685,12 @@ __device__ __forceinline__ void planeax_body(const AxisArgs<T> &a, const int x, 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cpx<T> *P = reinterpret_cast<cpx<T> *>(smem_raw);
     T *Pr = reinterpret_cast<T *>(smem_raw);
-    unsigned char *taby = smem_raw + C::TILE, *tabz = taby + AxTables<T, NY>::BYTES;
+    typename C::TabY taby{smem_raw + C::TILE};
+    typename C::TabZ tabz{smem_raw + C::TILE + C::TabY::BYTES};
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    AxTables<T, NY>::load(taby, a.twy, a.gy, threadIdx.x, C::NT);
-    AxTables<T, NZ>::load(tabz, a.twz, a.gz, threadIdx.x, C::NT);
+    taby.load(a.twy, a.gy, threadIdx.x, C::NT);
+    tabz.load(a.twz, a.gz, threadIdx.x, C::NT);
     pdl_wait();
-    const cpx<T> *twy = AxTables<T, NY>::tw(taby), *twz = AxTables<T, NZ>::tw(tabz);
-    const T *gy = AxTables<T, NY>::g(taby), *gz = AxTables<T, NZ>::g(tabz);
     cpx<T> *S = ax_field(a, c) + x * NY * C::NCOL;
 
     // y lines: a lane's tasks are (column, j2) and (column, k1), column fastest
@@ -670,28 +702,21 @@ __device__ __forceinline__ void planeax_body(const AxisArgs<T> &a, const int x, 
         if (okA) {
             Dft<C::RY1, -1, T>::run(v);
 #pragma unroll
-            for (int k = 0; k < C::RY1; k++)
-                P[C::ypos(yj + C::RY2 * k) + col] = k ? ctw<-1>(v[k], twy[yj * (C::RY1 + 1) + k]) : v[k];
+            for (int k = 0; k < C::RY1; k++) P[C::ypos(yj + C::RY2 * k) + col] = v[k];
         }
         __syncwarp();
         if (okB) {
             cpx<T> u[C::RY2];
 #pragma unroll
             for (int i = 0; i < C::RY2; i++) u[i] = P[C::ypos(C::RY2 * yj + i) + col];
-            Dft<C::RY2, -1, T>::run(u);
-#pragma unroll
-            for (int k = 0; k < C::RY2; k++) u[k] = cscale(u[k], gy[yj + C::RY1 * k]);
-            Dft<C::RY2, 1, T>::run(u);
+            taby.convolve(u, yj);
 #pragma unroll
             for (int i = 0; i < C::RY2; i++) P[C::ypos(C::RY2 * yj + i) + col] = u[i];
         }
         __syncwarp();
         if (okA) {
 #pragma unroll
-            for (int k = 0; k < C::RY1; k++) {
-                const cpx<T> t = P[C::ypos(yj + C::RY2 * k) + col];
-                v[k] = k ? ctw<1>(t, twy[yj * (C::RY1 + 1) + k]) : t;
-            }
+            for (int k = 0; k < C::RY1; k++) v[k] = P[C::ypos(yj + C::RY2 * k) + col];
             Dft<C::RY1, 1, T>::run(v);
         }
     };
@@ -707,28 +732,21 @@ __device__ __forceinline__ void planeax_body(const AxisArgs<T> &a, const int x, 
         if (okA) {
             Dft<C::RZ1, -1, T>::run(v);
 #pragma unroll
-            for (int k = 0; k < C::RZ1; k++)
-                P[zat(l0 + zlA, zjA + C::RZ2 * k)] = k ? ctw<-1>(v[k], twz[zjA * (C::RZ1 + 1) + k]) : v[k];
+            for (int k = 0; k < C::RZ1; k++) P[zat(l0 + zlA, zjA + C::RZ2 * k)] = v[k];
         }
         __syncwarp();
         if (okB) {
             cpx<T> u[C::RZ2];
 #pragma unroll
             for (int i = 0; i < C::RZ2; i++) u[i] = P[zat(l0 + zlB, C::RZ2 * zjB + i)];
-            Dft<C::RZ2, -1, T>::run(u);
-#pragma unroll
-            for (int k = 0; k < C::RZ2; k++) u[k] = cscale(u[k], gz[zjB + C::RZ1 * k]);
-            Dft<C::RZ2, 1, T>::run(u);
+            tabz.convolve(u, zjB);
 #pragma unroll
             for (int i = 0; i < C::RZ2; i++) P[zat(l0 + zlB, C::RZ2 * zjB + i)] = u[i];
         }
         __syncwarp();
         if (okA) {
 #pragma unroll
-            for (int k = 0; k < C::RZ1; k++) {
-                const cpx<T> t = P[zat(l0 + zlA, zjA + C::RZ2 * k)];
-                v[k] = k ? ctw<1>(t, twz[zjA * (C::RZ1 + 1) + k]) : t;
-            }
+            for (int k = 0; k < C::RZ1; k++) v[k] = P[zat(l0 + zlA, zjA + C::RZ2 * k)];
             Dft<C::RZ1, 1, T>::run(v);
         }
     };
