@@ -344,11 +344,19 @@ __device__ __forceinline__ double ax_q_part(cpx<T> v)
 // q^_{i+1} = v.x p.y and q_{N-i} q^_{N-i} = p.x v.y; the middle slot of an odd
 // chain has no partner and gives the one product v.x v.y.
 template <typename T>
-__device__ __forceinline__ void ax_acc(const AxisArgs<T> &a, int o, cpx<T> v)
+__device__ __forceinline__ float2 ax_partner(const AxisArgs<T> &a, int o)
+{
+    return a.partner ? __ldcs(reinterpret_cast<const float2 *>(a.partner) + o) : make_float2(0.f, 0.f);
+}
+template <typename T>
+__device__ __forceinline__ float2 ax_sums(const AxisArgs<T> &a, int o)
+{
+    return a.acc_init ? make_float2(0.f, 0.f) : reinterpret_cast<const float2 *>(a.acc)[o];
+}
+template <typename T>
+__device__ __forceinline__ void ax_acc(const AxisArgs<T> &a, int o, cpx<T> v, float2 p, float2 s)
 {
     static_assert(kPairs<T>, "FP32 pairs only");
-    const float2 p = a.partner ? __ldcs(reinterpret_cast<const float2 *>(a.partner) + o) : make_float2(0.f, 0.f);
-    float2 s = a.acc_init ? make_float2(0.f, 0.f) : reinterpret_cast<const float2 *>(a.acc)[o];
     float pa, pb = 0.f;
     if (a.partner) {
         pa = v.x * p.y;
@@ -460,8 +468,11 @@ __device__ __forceinline__ void strided_body(const AxisArgs<T> &a, const cpx<T> 
     __syncthreads();
     V::A(v, sm, tid);
     // h comes in while stage B works from shared memory: the registers that
-    // held the line's points are free until Ainv
+    // held the line's points are free until Ainv.  With the sums, so do the
+    // partner slot and the sums: loaded at their use they made the 128^3 chain
+    // 1565 us, loaded here 1204 (the fewer CTAs per SM cost less than the waits).
     cpx<T> h[kH ? V::RA : 1][C::R1];
+    float2 pv[kAcc ? V::RA : 1][C::R1], sv[kAcc ? V::RA : 1][C::R1];
     if constexpr (kH) {
 #pragma unroll
         for (int s = 0; s < V::RA; s++) {
@@ -469,6 +480,18 @@ __device__ __forceinline__ void strided_body(const AxisArgs<T> &a, const cpx<T> 
             if (!live(t)) continue;
 #pragma unroll
             for (int j = 0; j < C::R1; j++) h[s][j] = ax_h<MODE != AX_OUT>(a, c, at(t, j));
+        }
+    }
+    if constexpr (kAcc) {
+#pragma unroll
+        for (int s = 0; s < V::RA; s++) {
+            const int t = tid + s * C::NT;
+            if (!live(t)) continue;
+#pragma unroll
+            for (int j = 0; j < C::R1; j++) {
+                pv[s][j] = ax_partner(a, at(t, j));
+                sv[s][j] = ax_sums(a, at(t, j));
+            }
         }
     }
     __syncthreads();
@@ -485,7 +508,7 @@ __device__ __forceinline__ void strided_body(const AxisArgs<T> &a, const cpx<T> 
             for (int j = 0; j < C::R1; j++) {
                 v[s][j] = {v[s][j].x * h[s][j].x, v[s][j].y * h[s][j].y};
                 if (MODE != AX_HA) ax_store<MODE != AX_OUT>(a, c, at(t, j), v[s][j]);
-                if constexpr (kAcc) ax_acc(a, at(t, j), v[s][j]);
+                if constexpr (kAcc) ax_acc(a, at(t, j), v[s][j], pv[s][j], sv[s][j]);
                 if (kLast) qs += ax_q_part(v[s][j]);
             }
         }
@@ -596,6 +619,7 @@ __device__ __forceinline__ void zline_body(const AxisArgs<T> &a, const int cta, 
     __syncthreads();
     V::A(v, sm, lane);
     cpx<T> h[kInit ? 1 : V::RA][C::R1];  // as in strided_body
+    float2 pv[kAcc ? V::RA : 1][C::R1], sv[kAcc ? V::RA : 1][C::R1];
     if constexpr (!kInit) {
 #pragma unroll
         for (int s = 0; s < V::RA; s++) {
@@ -603,6 +627,18 @@ __device__ __forceinline__ void zline_body(const AxisArgs<T> &a, const int cta, 
             if (!live(t)) continue;
 #pragma unroll
             for (int j = 0; j < C::R1; j++) h[s][j] = axz_h(a, c, at(t, j));
+        }
+    }
+    if constexpr (kAcc) {
+#pragma unroll
+        for (int s = 0; s < V::RA; s++) {
+            const int t = lane + s * 32;
+            if (!live(t)) continue;
+#pragma unroll
+            for (int j = 0; j < C::R1; j++) {
+                pv[s][j] = ax_partner(a, at(t, j));
+                sv[s][j] = ax_sums(a, at(t, j));
+            }
         }
     }
     __syncwarp();
@@ -619,7 +655,7 @@ __device__ __forceinline__ void zline_body(const AxisArgs<T> &a, const int cta, 
             for (int j = 0; j < C::R1; j++) {
                 v[s][j] = {v[s][j].x * h[s][j].x, v[s][j].y * h[s][j].y};
                 if (MODE != AX_HA) axz_store(a, c, at(t, j), v[s][j]);
-                if constexpr (kAcc) ax_acc(a, at(t, j), v[s][j]);
+                if constexpr (kAcc) ax_acc(a, at(t, j), v[s][j], pv[s][j], sv[s][j]);
                 if (kLast) qs += ax_q_part(v[s][j]);
             }
         }
