@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(kRedThreads, 4)
     HistPtrs hist{};
     for (int m = 1; m <= nh; m++) hist.p[m - 1] = S->Dh[S->phys[m]];
     const long long M = S->M;
-    concentrations_body<T>(q, M, N, NA, S->w, S->w + 2 * M, S->w + 3 * M, Qd, static_cast<T *>(S->Dh[S->cur]), nh,
+    concentrations_body<T, sizeof(T) == 8>(q, M, N, NA, S->w, S->w + 2 * M, S->w + 3 * M, Qd, static_cast<T *>(S->Dh[S->cur]), nh,
                            hist, S->partials, blockIdx.x, gridDim.x);
 }
 

@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(kRedThreads, 4) ens_conc_kernel(EnsRep *__rest
         concentrations_acc_body(R.acc, R.q, R.M, R.N, R.w + 2 * R.M, R.w + 3 * R.M, R.Qd, R.Dh[R.cur], nh, hist,
                                 R.partials, blockIdx.x, R.red_blocks);
     else
-        concentrations_body<float>(R.q, R.M, R.N, R.NA, R.w, R.w + 2 * R.M, R.w + 3 * R.M, R.Qd, R.Dh[R.cur], nh,
+        concentrations_body<float, false>(R.q, R.M, R.N, R.NA, R.w, R.w + 2 * R.M, R.w + 3 * R.M, R.Qd, R.Dh[R.cur], nh,
                                    hist, R.partials, blockIdx.x, R.red_blocks);
 }
 

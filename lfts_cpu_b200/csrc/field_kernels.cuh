@@ -90,6 +90,95 @@ __device__ __forceinline__ void vload(const T *p, T (&out)[V])
     for (int j = 0; j < V; j++) out[j] = e[j];
 }
 
+// Block sums of acc[0..nh], one barrier for all of them; each in block_sum's order
+__device__ __forceinline__ void dot_partials(const double (&acc)[kRedWidth], int nh,
+                                             double (&sh)[kRedWidth][kRedThreads / 32], double *out)
+{
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+    for (int m = 0; m < kRedWidth; m++) {
+        if (m > nh) break;
+        double v = acc[m];
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0) sh[m][wid] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x <= nh) {
+        double s = 0.0;
+        for (int i = 0; i < kRedThreads / 32; i++) s += sh[threadIdx.x][i];
+        out[threadIdx.x] = s;
+    }
+}
+
+// Threads that share the sum over the monomers of one vector of mesh points (FP64).
+// A mesh too small to fill the grid with one thread a vector leaves each thread a
+// serial chain of loads; split over up to 32 threads, the pass and its reduction
+// went from 18.7 to 12.4 us at 16^3, 39.5 to 31 at 48^3 (N = 64, ten history
+// vectors).  Where the mesh fills the grid one thread sums, in its own
+// instantiation: the split's shared memory cost 80^3 and larger meshes 1-2 %.
+// FP32-mixed sums stay with one thread: another order of the FP64 sum moved the
+// fields of a short ensemble run by 2.6e-5 through its replicas' Anderson loops.
+template <typename T>
+__host__ __device__ __forceinline__ int conc_slices(long long M, int N, int nblk)
+{
+    if (sizeof(T) == 4) return 1;
+    const long long nvec = M / 2, threads = (long long)nblk * kRedThreads;
+    int s = 1;
+    while (s < 32 && 2 * s * nvec <= threads && 4 * s <= N) s *= 2;
+    return s;
+}
+
+// sums over monomers i0 <= i < i1 (FP32: and N + 1 - i) of q_i q^_i at mesh points
+// r0 ... r0 + V - 1: those of A monomers (i <= NA) and of B monomers
+template <typename T, int V>
+__device__ __forceinline__ void conc_sums(const T *__restrict__ q, long long M, int N, int NA, long long r0, int i0,
+                                          int i1, double (&sA)[V], double (&sB)[V])
+{
+    // slot i holds [q_i | q^_{N+1-i}] (src/diblock.cc:19-24); slot i at q + (i-1)*2M
+    if constexpr (sizeof(T) == 4) {
+        // FP32 layout: slot i holds pairs (q_i, q^_{N+1-i}) (axis_conv.cuh),
+        // so slots i and j = N+1-i together give q_i q^_i and q_j q^_j
+#pragma unroll 4
+        for (int i = i0; i < i1; i++) {
+            const int j = N + 1 - i;
+            T a[2 * V], b[2 * V];
+            vload<T, V>(q + (long long)(i - 1) * 2 * M + 2 * r0, *reinterpret_cast<T(*)[V]>(a));
+            vload<T, V>(q + (long long)(i - 1) * 2 * M + 2 * r0 + V, *reinterpret_cast<T(*)[V]>(a + V));
+            vload<T, V>(q + (long long)(j - 1) * 2 * M + 2 * r0, *reinterpret_cast<T(*)[V]>(b));
+            vload<T, V>(q + (long long)(j - 1) * 2 * M + 2 * r0 + V, *reinterpret_cast<T(*)[V]>(b + V));
+#pragma unroll
+            for (int p = 0; p < V; p++) {
+                const double pi = __dmul_rn((double)a[2 * p], (double)b[2 * p + 1]);  // q_i q^_i
+                if (i <= NA)
+                    sA[p] = __dadd_rn(sA[p], pi);
+                else
+                    sB[p] = __dadd_rn(sB[p], pi);
+                if (j != i) {
+                    const double pj = __dmul_rn((double)b[2 * p], (double)a[2 * p + 1]);  // q_j q^_j
+                    if (j <= NA)
+                        sA[p] = __dadd_rn(sA[p], pj);
+                    else
+                        sB[p] = __dadd_rn(sB[p], pj);
+                }
+            }
+        }
+    } else {
+#pragma unroll 8
+        for (int i = i0; i < i1; i++) {
+            T a[V], b[V];
+            vload<T, V>(q + (long long)(i - 1) * 2 * M + r0, a);
+            vload<T, V>(q + (long long)(N - i) * 2 * M + M + r0, b);
+            if (i <= NA) {
+#pragma unroll
+                for (int j = 0; j < V; j++) sA[j] = __dadd_rn(sA[j], __dmul_rn((double)a[j], (double)b[j]));
+            } else {
+#pragma unroll
+                for (int j = 0; j < V; j++) sB[j] = __dadd_rn(sB[j], __dmul_rn((double)a[j], (double)b[j]));
+            }
+        }
+    }
+}
+
 // phi-/phi+ (src/diblock.cc:50-57, 85-95) and, when Dh0 != nullptr, the
 // Anderson residual Dh0 = phi+ - 1 with partial sums of Dh0*Dh0 and
 // Dh0*Dh_m, m = 1..nh (src/anderson.cc:35-55).  Each thread handles V
@@ -97,7 +186,8 @@ __device__ __forceinline__ void vload(const T *p, T (&out)[V])
 // body of block `blk` of `nblk` (the grid-stride partition fixes the order of
 // the dot-product partial sums, so a replica's result does not depend on how
 // its blocks are launched)
-template <typename T>
+// SPLIT: compiled for meshes of several slices too
+template <typename T, bool SPLIT>
 __device__ __forceinline__ void concentrations_body(
     const T *__restrict__ q, long long M, int N, int NA, const double *__restrict__ w,
     double *__restrict__ phim, double *__restrict__ phip, const double *__restrict__ Qd,
@@ -106,48 +196,18 @@ __device__ __forceinline__ void concentrations_body(
 {
     constexpr int V = sizeof(T) == 4 ? 4 : 2;
     using VT = typename VecOf<T, V>::type;
-    __shared__ double sh[kRedThreads / 32];
+    __shared__ double sh[kRedWidth][kRedThreads / 32];
     const double Q = Qd[0];
     const double NQ = __dmul_rn((double)N, Q);
     double acc[kRedWidth];
 #pragma unroll
     for (int m = 0; m < kRedWidth; m++) acc[m] = 0.0;
     const long long nvec = M / V;
-    const long long stride = (long long)nblk * blockDim.x;
-    for (long long g = (long long)blk * blockDim.x + threadIdx.x; g < nvec; g += stride) {
-        const long long r0 = g * V;
-        // slot i holds [q_i | q^_{N+1-i}] (src/diblock.cc:19-24); slot i at q + (i-1)*2M
-        double sA[V], sB[V];
-#pragma unroll
-        for (int j = 0; j < V; j++) sA[j] = sB[j] = 0.0;
+    const int terms = sizeof(T) == 4 ? (N + 1) / 2 : N;
+    const int slices = SPLIT ? conc_slices<T>(M, N, nblk) : 1;
+    auto finish = [&](const long long r0, const double(&sA)[V], const double(&sB)[V]) {
         T hA[V], hB[V];
         if constexpr (sizeof(T) == 4) {
-            // FP32 packed layout: slot i holds pairs (q_i, q^_{N+1-i}) (fft_packed.cuh),
-            // so slots i and j = N+1-i together give q_i q^_i and q_j q^_j
-#pragma unroll 4
-            for (int i = 1; 2 * i <= N + 1; i++) {
-                const int j = N + 1 - i;
-                T a[2 * V], b[2 * V];
-                vload<T, V>(q + (long long)(i - 1) * 2 * M + 2 * r0, *reinterpret_cast<T(*)[V]>(a));
-                vload<T, V>(q + (long long)(i - 1) * 2 * M + 2 * r0 + V, *reinterpret_cast<T(*)[V]>(a + V));
-                vload<T, V>(q + (long long)(j - 1) * 2 * M + 2 * r0, *reinterpret_cast<T(*)[V]>(b));
-                vload<T, V>(q + (long long)(j - 1) * 2 * M + 2 * r0 + V, *reinterpret_cast<T(*)[V]>(b + V));
-#pragma unroll
-                for (int p = 0; p < V; p++) {
-                    const double pi = __dmul_rn((double)a[2 * p], (double)b[2 * p + 1]);  // q_i q^_i
-                    if (i <= NA)
-                        sA[p] = __dadd_rn(sA[p], pi);
-                    else
-                        sB[p] = __dadd_rn(sB[p], pi);
-                    if (j != i) {
-                        const double pj = __dmul_rn((double)b[2 * p], (double)a[2 * p + 1]);  // q_j q^_j
-                        if (j <= NA)
-                            sA[p] = __dadd_rn(sA[p], pj);
-                        else
-                            sB[p] = __dadd_rn(sB[p], pj);
-                    }
-                }
-            }
             T h[2 * V];
             vload<T, V>(q + 2 * r0, *reinterpret_cast<T(*)[V]>(h));
             vload<T, V>(q + 2 * r0 + V, *reinterpret_cast<T(*)[V]>(h + V));
@@ -157,19 +217,6 @@ __device__ __forceinline__ void concentrations_body(
                 hB[p] = h[2 * p + 1];
             }
         } else {
-#pragma unroll 8
-            for (int i = 1; i <= N; i++) {
-                T a[V], b[V];
-                vload<T, V>(q + (long long)(i - 1) * 2 * M + r0, a);
-                vload<T, V>(q + (long long)(N - i) * 2 * M + M + r0, b);
-                if (i <= NA) {
-#pragma unroll
-                    for (int j = 0; j < V; j++) sA[j] = __dadd_rn(sA[j], __dmul_rn((double)a[j], (double)b[j]));
-                } else {
-#pragma unroll
-                    for (int j = 0; j < V; j++) sB[j] = __dadd_rn(sB[j], __dmul_rn((double)a[j], (double)b[j]));
-                }
-            }
             vload<T, V>(q + r0, hA);
             vload<T, V>(q + M + r0, hB);
         }
@@ -210,15 +257,46 @@ __device__ __forceinline__ void concentrations_body(
                 }
             }
         }
+    };
+    if (!SPLIT || slices == 1) {
+        const long long stride = (long long)nblk * blockDim.x;
+        for (long long g = (long long)blk * blockDim.x + threadIdx.x; g < nvec; g += stride) {
+            double sA[V], sB[V];
+#pragma unroll
+            for (int j = 0; j < V; j++) sA[j] = sB[j] = 0.0;
+            conc_sums<T, V>(q, M, N, NA, g * V, 1, 1 + terms, sA, sB);
+            finish(g * V, sA, sB);
+        }
+    } else {
+        // `width` vectors a block, each of its `slices` threads a range of monomers;
+        // nvec <= nblk * width, so a block has one round
+        __shared__ double part[2 * V][SPLIT ? kRedThreads : 1];
+        const int width = kRedThreads / slices, lane = threadIdx.x % width, slice = threadIdx.x / width;
+        const long long g = (long long)blk * width + lane;
+        double sA[V], sB[V];
+#pragma unroll
+        for (int j = 0; j < V; j++) sA[j] = sB[j] = 0.0;
+        if (g < nvec)
+            conc_sums<T, V>(q, M, N, NA, g * V, 1 + slice * terms / slices, 1 + (slice + 1) * terms / slices, sA, sB);
+#pragma unroll
+        for (int j = 0; j < V; j++) {
+            part[2 * j][threadIdx.x] = sA[j];
+            part[2 * j + 1][threadIdx.x] = sB[j];
+        }
+        __syncthreads();
+        if (slice == 0 && g < nvec) {
+            for (int k = 1; k < slices; k++) {
+#pragma unroll
+                for (int j = 0; j < V; j++) {
+                    sA[j] = __dadd_rn(sA[j], part[2 * j][k * width + lane]);
+                    sB[j] = __dadd_rn(sB[j], part[2 * j + 1][k * width + lane]);
+                }
+            }
+            finish(g * V, sA, sB);
+        }
     }
     (void)w;
-    if (!Dh0) return;
-#pragma unroll
-    for (int m = 0; m < kRedWidth; m++) {
-        if (m > nh) break;
-        const double s = block_sum(acc[m], sh);
-        if (threadIdx.x == 0) partials[(long long)blk * kRedWidth + m] = s;
-    }
+    if (Dh0) dot_partials(acc, nh, sh, partials + (long long)blk * kRedWidth);
 }
 
 // The same with the sums over the monomers already formed by the contour chain
@@ -231,7 +309,7 @@ __device__ __forceinline__ void concentrations_acc_body(
     double *__restrict__ phip, const double *__restrict__ Qd, float *__restrict__ Dh0, int nh, const HistPtrs &hist,
     double *__restrict__ partials, const int blk, const int nblk)
 {
-    __shared__ double sh[kRedThreads / 32];
+    __shared__ double sh[kRedWidth][kRedThreads / 32];
     const double NQ = __dmul_rn((double)N, Qd[0]);
     double dots[kRedWidth];
 #pragma unroll
@@ -272,13 +350,7 @@ __device__ __forceinline__ void concentrations_acc_body(
             }
         }
     }
-    if (!Dh0) return;
-#pragma unroll
-    for (int m = 0; m < kRedWidth; m++) {
-        if (m > nh) break;
-        const double s = block_sum(dots[m], sh);
-        if (threadIdx.x == 0) partials[(long long)blk * kRedWidth + m] = s;
-    }
+    if (Dh0) dot_partials(dots, nh, sh, partials + (long long)blk * kRedWidth);
 }
 
 static __global__ void __launch_bounds__(kRedThreads, 4) concentrations_acc_kernel(
@@ -289,13 +361,13 @@ static __global__ void __launch_bounds__(kRedThreads, 4) concentrations_acc_kern
     concentrations_acc_body(acc, h, M, N, phim, phip, Qd, Dh0, nh, hist, partials, blockIdx.x, gridDim.x);
 }
 
-template <typename T>
+template <typename T, bool SPLIT>
 static __global__ void __launch_bounds__(kRedThreads, 4) concentrations_kernel(
     const T *__restrict__ q, long long M, int N, int NA, const double *__restrict__ w,
     double *__restrict__ phim, double *__restrict__ phip, const double *__restrict__ Qd,
     T *__restrict__ Dh0, int nh, HistPtrs hist, double *__restrict__ partials)
 {
-    concentrations_body<T>(q, M, N, NA, w, phim, phip, Qd, Dh0, nh, hist, partials, blockIdx.x, gridDim.x);
+    concentrations_body<T, SPLIT>(q, M, N, NA, w, phim, phip, Qd, Dh0, nh, hist, partials, blockIdx.x, gridDim.x);
 }
 
 // out[m] = sum over blocks of partials[b][m], fixed order; block m < width

@@ -519,6 +519,16 @@ void enqueue_chain_launches(lfts_ctx *c)
     }
 }
 
+// phi from the stored slots, and with Dh0 the residual and its dot products
+template <typename T>
+void launch_concs(lfts_ctx *c, void *Dh0, int nh, const HistPtrs &hist)
+{
+    auto *fn = conc_slices<T>(c->M, c->N, c->red_blocks) > 1 ? concentrations_kernel<T, true>
+                                                             : concentrations_kernel<T, false>;
+    fn<<<stream_grid(c), kRedThreads, 0, c->st>>>(static_cast<const T *>(c->q), c->M, c->N, c->NA, c->w, c->w + 2 * c->M,
+                                                  c->w + 3 * c->M, c->Qd, static_cast<T *>(Dh0), nh, hist, c->partials);
+}
+
 template <typename T>
 void enqueue_concs(lfts_ctx *c, void *Dh0, int nh, const HistPtrs &hist)
 {
@@ -528,9 +538,7 @@ void enqueue_concs(lfts_ctx *c, void *Dh0, int nh, const HistPtrs &hist)
             static_cast<const float *>(c->acc), static_cast<const float *>(c->q), c->M, c->N, c->w + 2 * c->M,
             c->w + 3 * c->M, c->Qd, static_cast<float *>(Dh0), nh, hist, c->partials);
     else
-        concentrations_kernel<T><<<stream_grid(c), kRedThreads, 0, c->st>>>(
-            static_cast<const T *>(c->q), c->M, c->N, c->NA, c->w, c->w + 2 * c->M, c->w + 3 * c->M, c->Qd,
-            static_cast<T *>(Dh0), nh, hist, c->partials);
+        launch_concs<T>(c, Dh0, nh, hist);
     c->launches++;
     if (Dh0) {
         reduce_partials_kernel<<<nh + 1, 256, 0, c->st>>>(c->partials, c->red_blocks, nh + 1, c->red);
@@ -742,9 +750,7 @@ void enqueue_calc(lfts_ctx *c)
             static_cast<const float *>(c->acc), static_cast<const float *>(c->q), c->M, c->N, c->w + 2 * c->M,
             c->w + 3 * c->M, c->Qd, nullptr, 0, HistPtrs{}, c->partials);
     else
-        concentrations_kernel<T><<<stream_grid(c), kRedThreads, 0, c->st>>>(
-            static_cast<const T *>(c->q), c->M, c->N, c->NA, c->w, c->w + 2 * c->M, c->w + 3 * c->M, c->Qd, nullptr,
-            0, HistPtrs{}, c->partials);
+        launch_concs<T>(c, nullptr, 0, HistPtrs{});
 }
 
 // a tile choice is timed on whole calc_concs (chain + concentrations): the
@@ -1919,17 +1925,13 @@ int lfts_profile_iteration(lfts_ctx *c, int reps, double *ms_chain, double *ms_c
     CK(cudaEventRecord(ev[1], c->st));
     for (int r = 0; r < reps; r++) {
         if (c->prec == LFTS_FP64)
-            concentrations_kernel<double><<<stream_grid(c), kRedThreads, 0, c->st>>>(
-                static_cast<const double *>(c->q), M, c->N, c->NA, c->w, c->w + 2 * M, c->w + 3 * M, c->Qd,
-                static_cast<double *>(c->Dh[c->cur]), kMaxHist, Dhp, c->partials);
+            launch_concs<double>(c, c->Dh[c->cur], kMaxHist, Dhp);
         else if (c->phi_in_chain)
             concentrations_acc_kernel<<<stream_grid(c), kRedThreads, 0, c->st>>>(
                 static_cast<const float *>(c->acc), static_cast<const float *>(c->q), M, c->N, c->w + 2 * M,
                 c->w + 3 * M, c->Qd, static_cast<float *>(c->Dh[c->cur]), kMaxHist, Dhp, c->partials);
         else
-            concentrations_kernel<float><<<stream_grid(c), kRedThreads, 0, c->st>>>(
-                static_cast<const float *>(c->q), M, c->N, c->NA, c->w, c->w + 2 * M, c->w + 3 * M, c->Qd,
-                static_cast<float *>(c->Dh[c->cur]), kMaxHist, Dhp, c->partials);
+            launch_concs<float>(c, c->Dh[c->cur], kMaxHist, Dhp);
         reduce_partials_kernel<<<kRedWidth, 256, 0, c->st>>>(c->partials, c->red_blocks, kRedWidth, c->red);
     }
     CK(cudaEventRecord(ev[2], c->st));
