@@ -90,6 +90,21 @@ __device__ __forceinline__ void vload(const T *p, T (&out)[V])
     for (int j = 0; j < V; j++) out[j] = e[j];
 }
 
+// The same with the line marked for early eviction from L2: slots are read once a
+// chain, and lines kept in their place made the next chain's stores go to memory
+// at once (64^3 FP32, N = 64: chain after a concentration pass 335 us, 287 so;
+// FP64 463 and 427; 96^3 FP32 640 and 595).  The Anderson history likewise: an
+// iteration at 80^3 FP32 562 us, 533 so.
+template <typename T, int V>
+__device__ __forceinline__ void vload_once(const T *p, T (&out)[V])
+{
+    using VT = typename VecOf<T, V>::type;
+    const VT v = __ldcs(reinterpret_cast<const VT *>(p));
+    const T *e = reinterpret_cast<const T *>(&v);
+#pragma unroll
+    for (int j = 0; j < V; j++) out[j] = e[j];
+}
+
 // Block sums of acc[0..nh], one barrier for all of them; each in block_sum's order
 __device__ __forceinline__ void dot_partials(const double (&acc)[kRedWidth], int nh,
                                              double (&sh)[kRedWidth][kRedThreads / 32], double *out)
@@ -142,10 +157,10 @@ __device__ __forceinline__ void conc_sums(const T *__restrict__ q, long long M, 
         for (int i = i0; i < i1; i++) {
             const int j = N + 1 - i;
             T a[2 * V], b[2 * V];
-            vload<T, V>(q + (long long)(i - 1) * 2 * M + 2 * r0, *reinterpret_cast<T(*)[V]>(a));
-            vload<T, V>(q + (long long)(i - 1) * 2 * M + 2 * r0 + V, *reinterpret_cast<T(*)[V]>(a + V));
-            vload<T, V>(q + (long long)(j - 1) * 2 * M + 2 * r0, *reinterpret_cast<T(*)[V]>(b));
-            vload<T, V>(q + (long long)(j - 1) * 2 * M + 2 * r0 + V, *reinterpret_cast<T(*)[V]>(b + V));
+            vload_once<T, V>(q + (long long)(i - 1) * 2 * M + 2 * r0, *reinterpret_cast<T(*)[V]>(a));
+            vload_once<T, V>(q + (long long)(i - 1) * 2 * M + 2 * r0 + V, *reinterpret_cast<T(*)[V]>(a + V));
+            vload_once<T, V>(q + (long long)(j - 1) * 2 * M + 2 * r0, *reinterpret_cast<T(*)[V]>(b));
+            vload_once<T, V>(q + (long long)(j - 1) * 2 * M + 2 * r0 + V, *reinterpret_cast<T(*)[V]>(b + V));
 #pragma unroll
             for (int p = 0; p < V; p++) {
                 const double pi = __dmul_rn((double)a[2 * p], (double)b[2 * p + 1]);  // q_i q^_i
@@ -166,8 +181,8 @@ __device__ __forceinline__ void conc_sums(const T *__restrict__ q, long long M, 
 #pragma unroll 8
         for (int i = i0; i < i1; i++) {
             T a[V], b[V];
-            vload<T, V>(q + (long long)(i - 1) * 2 * M + r0, a);
-            vload<T, V>(q + (long long)(N - i) * 2 * M + M + r0, b);
+            vload_once<T, V>(q + (long long)(i - 1) * 2 * M + r0, a);
+            vload_once<T, V>(q + (long long)(N - i) * 2 * M + M + r0, b);
             if (i <= NA) {
 #pragma unroll
                 for (int j = 0; j < V; j++) sA[j] = __dadd_rn(sA[j], __dmul_rn((double)a[j], (double)b[j]));
@@ -251,7 +266,7 @@ __device__ __forceinline__ void concentrations_body(
             for (int m = 1; m < kRedWidth; m++) {
                 if (m <= nh) {
                     T hv[V];
-                    vload<T, V>(static_cast<const T *>(hist.p[m - 1]) + r0, hv);
+                    vload_once<T, V>(static_cast<const T *>(hist.p[m - 1]) + r0, hv);
 #pragma unroll
                     for (int j = 0; j < V; j++) acc[m] = __dadd_rn(acc[m], __dmul_rn(d[j], (double)hv[j]));
                 }
@@ -343,7 +358,7 @@ __device__ __forceinline__ void concentrations_acc_body(
 #pragma unroll
             for (int m = 1; m < kRedWidth; m++) {
                 if (m <= nh) {
-                    const float2 hv = *reinterpret_cast<const float2 *>(static_cast<const float *>(hist.p[m - 1]) + r0);
+                    const float2 hv = __ldcs(reinterpret_cast<const float2 *>(static_cast<const float *>(hist.p[m - 1]) + r0));
                     dots[m] = __dadd_rn(dots[m], __dmul_rn(d[0], (double)hv.x));
                     dots[m] = __dadd_rn(dots[m], __dmul_rn(d[1], (double)hv.y));
                 }
@@ -403,8 +418,8 @@ __device__ __forceinline__ void anderson_update_body(double *__restrict__ wp, H 
 #pragma unroll
             for (int n = 0; n < kMaxHist; n++) {
                 if (n < nh) {
-                    const double whn = (double)static_cast<const H *>(wh.p[n])[r];
-                    const double dhn = (double)static_cast<const H *>(Dh.p[n])[r];
+                    const double whn = (double)__ldcs(static_cast<const H *>(wh.p[n]) + r);
+                    const double dhn = (double)__ldcs(static_cast<const H *>(Dh.p[n]) + r);
                     const double hn = __dadd_rn(whn, __dmul_rn(lambda, dhn));
                     acc = __dadd_rn(acc, __dmul_rn(c[n], __dsub_rn(hn, base)));
                 }
