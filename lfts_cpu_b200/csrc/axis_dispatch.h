@@ -29,7 +29,16 @@ bool axis_kernels(int mx, int my, int mz, int cw, AxisSet<float> *o);
 // choice: its CTAs' partial sums for Q then do not depend on the tiles.
 constexpr int kLastCw = 16;
 
-// Whether y and z lines share a kernel, one CTA per x-plane.
-constexpr bool axis_planes(int my, int mz) { return my * mz <= 48 * 48; }
+// Whether y and z lines share a kernel, one CTA per x-plane (and FP64 chain): one
+// launch less a step while a CTA has little of a plane to work through.  Chain with
+// one kernel / two, N = 64, us: 32^3 FP64 194 / 285, 40^3 267 / 315, FP32 221 / 244;
+// 48^3 FP64 385 / 322, 64^3 FP32 363 / 273.  FP64 planes of 64 x 64, whose stages
+// are all of 8 points and fill their warps: calc_concs 467 / 476, with 128 of them
+// 710 / 765.
+template <typename T>
+constexpr bool axis_planes(int my, int mz)
+{
+    return my * mz <= 2048 || (!kPairs<T> && my == 64 && mz == 64);
+}
 
 }  // namespace lfts

@@ -44,7 +44,7 @@ static void fill_z(AxisSet<T> *o)
 template <typename T, int NY, int NZ>
 static void fill_plane(AxisSet<T> *o)
 {
-    if constexpr (axis_planes(NY, NZ)) {
+    if constexpr (axis_planes<T>(NY, NZ)) {
         using C = PlaneAxCfg<T, NY, NZ>;
         o->plane[AX_INIT_W] = {planeax_kernel<T, NY, NZ, AX_INIT_W>, C::NT, C::SMEM, 1};
         o->plane[AX_INIT_Q] = {planeax_kernel<T, NY, NZ, AX_INIT_Q>, C::NT, C::SMEM, 1};
@@ -73,7 +73,7 @@ static bool fill_axis(int mx, int my, int mz, int cw, AxisSet<T> *o)
 #define LFTS_P(a, b)                                   \
     if (my == a && mz == b) {                          \
         p = true;                                      \
-        if constexpr (axis_planes(a, b)) {             \
+        if constexpr (axis_planes<T>(a, b)) {             \
             fill_plane<T, a, b>(o);                    \
         } else {                                       \
             if (cw == 8) fill_y<T, a, 8>(o);           \
