@@ -11,20 +11,22 @@
 // (3 N L_alpha^3); this kernel accumulates, per alpha,
 //     S_alpha = sum_i sum_k w(kz) g(k) k_alpha^2 Re[qhat_i conj(qhat^_{i+1})]
 // and the host applies the constant.  The yz-plane forward transforms of the
-// pair (q_i, q^_{i+1}) come from plane_kernel (PLANE_INIT_Q, chains 0 and 1);
-// this x-pencil variant transforms both chains' columns of a tile and forms the
-// products in registers.
+// pairs (q_i, q^_{i+1}) come from fwd_plane_kernel_t; this x-pencil variant
+// transforms both chains' columns of a tile and forms the products in registers.
+// A launch takes several terms i at once (grid y): one term's 2 mx planes and
+// few hundred pencils leave most of the GPU idle, and the 63 terms of a 64^3 chain
+// took 890 us in launches of one, 360 us in launches of five.
 #pragma once
 #include "fft_kernels.cuh"
 
 namespace lfts {
 
 struct AdjArgs {
-    const cpx<double> *spec;  // chain 0 at spec, chain 1 at spec + mx*ncol
+    const cpx<double> *spec;  // per term: chain 0 at spec, chain 1 at spec + mx*ncol
     const cpx<double> *twx;
     const double *gx, *gy, *gz;  // factorised g (1/M in gz)
     int ncol, KZ, mx, my, mz;
-    double *partial;  // [gridDim.x][3], accumulated over launches
+    double *partial;  // [term][gridDim.x][3], accumulated over launches
 };
 
 template <int NX, int CW>
@@ -59,7 +61,7 @@ __global__ void __launch_bounds__(AdjCfg<NX, CW>::NT) pencil_adj_kernel(AdjArgs 
         if (t < CW * R2 && col < ncol) {
 #pragma unroll
             for (int ch = 0; ch < 2; ch++) {
-                const cpx<double> *Sg = a.spec + (long long)ch * a.mx * ncol;
+                const cpx<double> *Sg = a.spec + (2LL * blockIdx.y + ch) * a.mx * ncol;
                 cpx<double> *Tl = ch ? T1 : T0;
                 cpx<double> v[R1];
 #pragma unroll
@@ -111,7 +113,7 @@ __global__ void __launch_bounds__(AdjCfg<NX, CW>::NT) pencil_adj_kernel(AdjArgs 
     if (threadIdx.x < 3) {
         double v = 0.0;
         for (int w = 0; w < C::NT / 32; w++) v += red[threadIdx.x][w];
-        a.partial[blockIdx.x * 3 + threadIdx.x] += v;
+        a.partial[(blockIdx.y * gridDim.x + blockIdx.x) * 3 + threadIdx.x] += v;
     }
 }
 

@@ -63,8 +63,10 @@ struct lfts_ctx {
     std::vector<double> sk_K;  // K value reported for each bin
 
     void *sf_buf = nullptr;    // step_fwd scratch: q_in, q_out, h (2M each, FP64)
-    double *adj_partial = nullptr;  // adjoint block partials [blocks][3]
-    double *adj_buf = nullptr;      // checkpointed adjoint: recomputed q segment + discard row
+    double *adj_partial = nullptr;  // adjoint block partials [term][blocks][3]
+    void *adj_spec = nullptr;       // half spectra of the terms of one launch
+    int adj_batch = 0;              // those terms
+    double *adj_buf = nullptr;      // checkpointed adjoint: two recomputed q segments
     int adj_buf_slots = 0;
     AdjKernel adj{};
 

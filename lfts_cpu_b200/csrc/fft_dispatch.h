@@ -25,7 +25,7 @@ struct PencilKernels {
 };
 
 struct PlaneKernel {
-    void (*fn)(PlaneArgs<double>);
+    void (*fn)(FwdArgs);
     int nt;
     size_t smem;
 };

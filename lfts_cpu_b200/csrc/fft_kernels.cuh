@@ -301,8 +301,17 @@ struct TwStage {
 };
 
 // ------------------------------------------------------------ plane kernel --
+// rows of up to kFwdBatch pairs of fields (field f of pair b: src[f][b]); one CTA
+// per x-plane, field and pair, half spectra to spec + (2 b + f) mx NY KZ
+constexpr int kFwdBatch = 16;
+struct FwdArgs {
+    const double *src[2][kFwdBatch];
+    cpx<double> *spec;
+    const cpx<double> *twy, *twz;  // exp(-2 pi i t/n) tables
+};
+
 template <int NY, int NZ>
-__global__ void __launch_bounds__(PlaneCfg<double, NY, NZ>::NT) fwd_plane_kernel_t(PlaneArgs<double> a)
+__global__ void __launch_bounds__(PlaneCfg<double, NY, NZ>::NT) fwd_plane_kernel_t(FwdArgs a)
 {
     using T = double;
     using C = PlaneCfg<T, NY, NZ>;
@@ -313,10 +322,10 @@ __global__ void __launch_bounds__(PlaneCfg<double, NY, NZ>::NT) fwd_plane_kernel
     cpx<T> *twa = twy + NY;            // TA: stage-A z twiddles
     cpx<T> *colbuf = twa + C::NTA + C::NTB;
 
-    const int x = blockIdx.x, c = blockIdx.y;
-    const int mx = gridDim.x;
+    const int x = blockIdx.x, mx = gridDim.x;
+    const double *src = a.src[blockIdx.y][blockIdx.z];
     const long long plane_off = (long long)x * NY * NZ;
-    cpx<T> *Sg = a.spec + ((long long)c * mx + x) * NY * KZ;
+    cpx<T> *Sg = a.spec + (((long long)2 * blockIdx.z + blockIdx.y) * mx + x) * NY * KZ;
 
     TwStage<C, T> tws;
     tws.load(a.twy, a.twz);
@@ -329,7 +338,7 @@ __global__ void __launch_bounds__(PlaneCfg<double, NY, NZ>::NT) fwd_plane_kernel
     for (int t = lane; t < ntask; t += 32) {
         const int q = q0 + t / NZ, z = t % NZ;
         const long long ia = plane_off + (2 * q) * NZ + z, ib = ia + NZ;
-        P[2 * q * KZP + C::zpos(z)] = {a.src[c * a.src_stride + ia], a.src[c * a.src_stride + ib]};
+        P[2 * q * KZP + C::zpos(z)] = {src[ia], src[ib]};
     }
     __syncwarp();
     z_fwdA_tw<C>(P, twa);

@@ -1207,8 +1207,8 @@ int anderson_mix(lfts_ctx *c, int maxIter, double errTol, int *k_out)
 // ---- structure function -------------------------------------------------------
 int sk_sample(lfts_ctx *c)
 {
-    PlaneArgs<double> a{};
-    a.src = c->w;  // W-
+    FwdArgs a{};
+    a.src[0][0] = c->w;  // W-
     a.spec = static_cast<cpx<double> *>(c->skspec);
     const bool fp64 = c->prec == LFTS_FP64;
     a.twy = static_cast<const cpx<double> *>(fp64 ? c->tw[1] : c->sktw[1]);
@@ -1345,6 +1345,7 @@ void ctx_free(lfts_ctx *c)
     cudaFree(c->sf_buf);
     cudaFree(c->adj_partial);
     cudaFree(c->adj_buf);
+    cudaFree(c->adj_spec);
     drop_chain_graph(c);
     cudaFree(c->acc);
     cudaFree(c->d_mix);
@@ -1417,20 +1418,13 @@ int step_fwd_impl(lfts_ctx *c, const double *q_in, double *q_out, const double *
 
 namespace {
 
-// One adjoint term: forward transforms of q_i (chain 0) and q^_{i+1}
-// (chain 1), then the k^2-weighted products summed into c->adj_partial.
-int adjoint_term(lfts_ctx *c, const double *q_i, const double *qh_ip1)
+// Adjoint terms: forward transforms of q_i (field 0) and q^_{i+1} (field 1) of n
+// monomers i, then the k^2-weighted products summed into c->adj_partial.
+void adjoint_terms(lfts_ctx *c, const FwdArgs &f, int n)
 {
-    PlaneArgs<double> a{};
-    a.src = q_i;
-    a.src_stride = (long long)(qh_ip1 - q_i);
-    a.spec = static_cast<cpx<double> *>(c->field);
-    a.twy = static_cast<const cpx<double> *>(c->tw[1]);
-    a.twz = static_cast<const cpx<double> *>(c->tw[2]);
-    c->fwd_yz.fn<<<dim3(c->mx, 2), c->fwd_yz.nt, c->fwd_yz.smem, c->st>>>(a);
-    c->launches++;
+    c->fwd_yz.fn<<<dim3(c->mx, 2, n), c->fwd_yz.nt, c->fwd_yz.smem, c->st>>>(f);
     AdjArgs aa{};
-    aa.spec = static_cast<const cpx<double> *>(c->field);
+    aa.spec = f.spec;
     aa.twx = static_cast<const cpx<double> *>(c->tw[0]);
     aa.gx = static_cast<const double *>(c->gtab[0]);
     aa.gy = static_cast<const double *>(c->gtab[1]);
@@ -1441,10 +1435,33 @@ int adjoint_term(lfts_ctx *c, const double *q_i, const double *qh_ip1)
     aa.my = c->my;
     aa.mz = c->mz;
     aa.partial = c->adj_partial;
-    c->adj.fn<<<(aa.ncol + c->adj.cw - 1) / c->adj.cw, c->adj.nt, c->adj.smem, c->st>>>(aa);
-    c->launches++;
-    return LFTS_OK;
+    c->adj.fn<<<dim3((aa.ncol + c->adj.cw - 1) / c->adj.cw, n), c->adj.nt, c->adj.smem, c->st>>>(aa);
+    c->launches += 2;
 }
+
+// Terms given one by one, launched c->adj_batch at a time
+struct AdjointBatch {
+    lfts_ctx *c;
+    FwdArgs f{};
+    int n = 0;
+    explicit AdjointBatch(lfts_ctx *ctx) : c(ctx)
+    {
+        f.spec = static_cast<cpx<double> *>(c->adj_spec);
+        f.twy = static_cast<const cpx<double> *>(c->tw[1]);
+        f.twz = static_cast<const cpx<double> *>(c->tw[2]);
+    }
+    void add(const double *q_i, const double *qh_ip1)
+    {
+        f.src[0][n] = q_i;
+        f.src[1][n] = qh_ip1;
+        if (++n == c->adj_batch) flush();
+    }
+    void flush()
+    {
+        if (n) adjoint_terms(c, f, n);
+        n = 0;
+    }
+};
 
 // Propagators of both chains with q stored only at monomers 1, 1+K, 1+2K, ...
 // (q^ in full); returns after Q is reduced.
@@ -1461,18 +1478,23 @@ int chain_checkpointed(lfts_ctx *c, int K)
     return LFTS_OK;
 }
 
-// q_{c0+1} .. q_{c0+n} recomputed from the checkpoint q_{c0} into adj_buf rows 1..n
-void recompute_segment(lfts_ctx *c, const double *q_c0, int c0, int n)
+// Two segments recomputed side by side, as the two FP64 fields of the axis
+// kernels: segment s's q_{c0+1} .. q_{c0+n[s]} from its checkpoint q_{c0} (row 0)
+// into rows 1 .. n[s], n[0] >= n[1]
+void recompute_segments(lfts_ctx *c, const double *const row0[2], double *const rows[2], const int c0[2],
+                        const int n[2])
 {
     AxisArgs<double> a = axis_args<double>(c);
-    a.src[0] = q_c0;
+    const int nseg = n[1] > 0 ? 2 : 1;
+    for (int s = 0; s < nseg; s++) a.src[s] = row0[s];
     a.ticket = nullptr;
-    launch_yz<double>(c, AX_INIT_Q, a, 1, c->st);
-    for (int j = 1; j <= n; j++) {
-        const int i = c0 + j - 1;  // monomer step i makes q_{i+1}
-        a.hsel[0] = hsel_chain0(c, i);
-        a.q[0] = c->adj_buf + (long long)j * c->M;
-        launch_step<double>(c, j, j < n ? AX_H : AX_H_LAST, a, 1, c->st);
+    launch_yz<double>(c, AX_INIT_Q, a, nseg, c->st);
+    for (int j = 1; j <= n[0]; j++) {
+        for (int s = 0; s < nseg; s++) {
+            a.hsel[s] = hsel_chain0(c, c0[s] + j - 1);  // monomer step i = c0 + j - 1 makes q_{i+1}
+            a.q[s] = j <= n[s] ? rows[s] + (long long)j * c->M : nullptr;
+        }
+        launch_step<double>(c, j, j < n[0] ? AX_H : AX_H_LAST, a, nseg, c->st);
     }
 }
 
@@ -1836,42 +1858,62 @@ int lfts_backward(lfts_ctx *c, int ckpt_every, double *dH_dL, double *dH_dXbN, d
     CK(cudaFuncSetAttribute(c->adj.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->adj.smem));
     const long long M = c->M;
     const int nblk = (c->my * c->KZ + c->adj.cw - 1) / c->adj.cw;
-    if (!c->adj_partial) CK(cudaMalloc(&c->adj_partial, sizeof(double) * 3 * nblk));
-    CK(cudaMemsetAsync(c->adj_partial, 0, sizeof(double) * 3 * nblk, c->st));
+    if (!c->adj_spec) {
+        // terms per launch: about four CTAs per SM of 2 mx planes a term
+        c->adj_batch = std::max(1, std::min(kFwdBatch, (4 * c->sms + 2 * c->mx - 1) / (2 * c->mx)));
+        CK(cudaMalloc(&c->adj_spec, sizeof(cpx<double>) * 2 * (size_t)c->Mk * c->adj_batch));
+    }
+    const int nrows = nblk * c->adj_batch;
+    if (!c->adj_partial) CK(cudaMalloc(&c->adj_partial, sizeof(double) * 3 * nrows));
+    CK(cudaMemsetAsync(c->adj_partial, 0, sizeof(double) * 3 * nrows, c->st));
     double *q = static_cast<double *>(c->q);
     const int N = c->N;
     // q_i is the first half of slot i, q^_{i+1} the second half of slot N-i
     auto qh = [&](int i1) { return q + (long long)(N - i1) * 2 * M + M; };  // q^_{i1}
+    AdjointBatch terms(c);
     if (ckpt_every == 0) {
         int rc = calc_concs_sync(c, nullptr);
         if (rc) return rc;
-        for (int i = 1; i < N; i++) adjoint_term(c, q + (long long)(i - 1) * 2 * M, qh(i + 1));
+        for (int i = 1; i < N; i++) terms.add(q + (long long)(i - 1) * 2 * M, qh(i + 1));
     } else {
-        const int K = ckpt_every;
-        if (c->adj_buf_slots < K) {
+        const int K = std::min(ckpt_every, N);
+        const int slots = 1 + K < N ? 2 * K : K;  // one segment: no second one beside it
+        if (c->adj_buf_slots < slots) {
             cudaFree(c->adj_buf);
             c->adj_buf = nullptr;
-            CK(cudaMalloc(&c->adj_buf, sizeof(double) * (size_t)K * M));
-            c->adj_buf_slots = K;
+            c->adj_buf_slots = 0;
+            CK(cudaMalloc(&c->adj_buf, sizeof(double) * (size_t)slots * M));
+            c->adj_buf_slots = slots;
         }
         chain_checkpointed(c, K);
-        for (int c0 = 1; c0 < N; c0 += K) {
-            const int last = std::min(c0 + K - 1, N - 1);  // terms i = c0 .. last
-            const double *qc = q + (long long)(c0 - 1) * 2 * M;
-            if (last > c0) recompute_segment(c, qc, c0, last - c0);
-            for (int i = c0; i <= last; i++)
-                adjoint_term(c, i == c0 ? qc : c->adj_buf + (long long)(i - c0) * M, qh(i + 1));
+        // two segments (terms i = c0 .. c0 + n) at a time
+        for (int c1 = 1; c1 < N; c1 += 2 * K) {
+            int c0[2], n[2];
+            const double *row0[2];
+            double *rows[2];
+            for (int s = 0; s < 2; s++) {
+                c0[s] = c1 + s * K;
+                n[s] = std::min(c0[s] + K - 1, N - 1) - c0[s];
+                row0[s] = q + (long long)(c0[s] - 1) * 2 * M;
+                rows[s] = c->adj_buf + (long long)s * K * M;
+            }
+            if (n[0] > 0) recompute_segments(c, row0, rows, c0, n);
+            for (int s = 0; s < 2; s++)
+                for (int j = 0; j <= n[s]; j++)
+                    terms.add(j ? rows[s] + (long long)j * M : row0[s], qh(c0[s] + j + 1));
+            if (K > 1) terms.flush();  // before the rows are written again
         }
         c->have_concs = false;  // phi was not recomputed
     }
+    terms.flush();
     CK(cudaGetLastError());
-    std::vector<double> part(3 * (size_t)nblk);
+    std::vector<double> part(3 * (size_t)nrows);
     CK(cudaMemcpyAsync(part.data(), c->adj_partial, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, c->st));
     CK(cudaMemcpyAsync(c->red_host, c->Qd, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     const double Q = c->red_host[0], lnQ = c->red_host[1];
     double S[3] = {0.0, 0.0, 0.0};
-    for (int b = 0; b < nblk; b++)
+    for (int b = 0; b < nrows; b++)
         for (int d = 0; d < 3; d++) S[d] += part[3 * (size_t)b + d];
     // dH/dL = -(1/Q) dQ/dL, dQ/dL_a = (1/M) 4 pi^2 S_a / (3 N L_a^3)
     for (int d = 0; d < 3; d++) {
