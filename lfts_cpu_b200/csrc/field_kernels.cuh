@@ -468,23 +468,36 @@ static __global__ void __launch_bounds__(kRedThreads) h_sums_kernel(const double
     if (threadIdx.x == 0) partials[(long long)blockIdx.x * kRedWidth + 1] = s2;
 }
 
-// Spherical average of S(k) (src/strFunc.cc:50-76): one thread per |K| bin,
-// summing its wavevectors in the reference's stable-sorted order.
-static __global__ void sk_bin_kernel(const double *__restrict__ S, const int *__restrict__ order,
-                              const int *__restrict__ wt, const int *__restrict__ bin_start, int nbins,
-                              double coeff_over_ns, double half_over_chi, double *__restrict__ out)
+// Spherical average of S(k) (src/strFunc.cc:50-76): one warp per |K| bin, which
+// loads 32 of its wavevectors at a time and adds them in the reference's
+// stable-sorted order.  Bound by the largest bin's chain of loads and adds (one
+// thread per bin: lfts_sk_bin at 64^3 72 us, at 128^3 129; so 37 and 66).
+static __global__ void __launch_bounds__(256) sk_bin_kernel(const double *__restrict__ S, const int *__restrict__ order,
+                                                            const int *__restrict__ wt,
+                                                            const int *__restrict__ bin_start, int nbins,
+                                                            double coeff_over_ns, double half_over_chi,
+                                                            double *__restrict__ out)
 {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    const int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (b >= nbins) return;
+    const int k0 = bin_start[b], k1 = bin_start[b + 1];
     double s = 0.0;
     int n = 0;
-    for (int k = bin_start[b]; k < bin_start[b + 1]; k++) {
-        const int p = order[k];
-        const double term = __dsub_rn(__dmul_rn(coeff_over_ns, S[p]), half_over_chi);
-        s = __dadd_rn(s, __dmul_rn((double)wt[p], term));
-        n += wt[p];
+    for (int k = k0; k < k1; k += 32) {
+        double x = 0.0;
+        int w = 0;
+        if (k + lane < k1) {
+            const int p = order[k + lane];
+            w = wt[p];
+            x = __dmul_rn((double)w, __dsub_rn(__dmul_rn(coeff_over_ns, S[p]), half_over_chi));
+        }
+        const int m = min(32, k1 - k);
+        for (int j = 0; j < m; j++) {  // in order, as one thread would
+            s = __dadd_rn(s, __shfl_sync(0xffffffffu, x, j));
+            n += __shfl_sync(0xffffffffu, w, j);
+        }
     }
-    out[b] = s / (double)n;
+    if (lane == 0) out[b] = s / (double)n;
 }
 
 // [a | b] halves (M each) <-> M pairs (a, b): the FP32 packed path stores h

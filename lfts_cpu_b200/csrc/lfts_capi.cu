@@ -1781,7 +1781,7 @@ int lfts_sk_bin(lfts_ctx *c, double dK, double *K_out, double *S_out, int *nbins
     const double CV = c->p.C * V;
     const double M = (double)c->M;
     const double coeff = CV / (c->p.XbN * c->p.XbN * M * M);
-    sk_bin_kernel<<<(c->sk_nbins + 127) / 128, 128, 0, c->st>>>(c->S, c->sk_order, c->sk_wt, c->sk_bins,
+    sk_bin_kernel<<<(c->sk_nbins + 7) / 8, 256, 0, c->st>>>(c->S, c->sk_order, c->sk_wt, c->sk_bins,
                                                                c->sk_nbins, coeff / (double)c->nsamples,
                                                                0.5 / c->p.XbN, c->sk_out);
     c->launches++;
@@ -1798,16 +1798,16 @@ int lfts_get_H(lfts_ctx *c, double *H)
     if (!c || !H) return LFTS_ERR_ARG;
     if (!c->fields_set) return LFTS_ERR_STATE;
     DeviceGuard g(c->dev);
-    double lnQ = 0.0;
-    int rc = calc_concs_sync(c, &lnQ);
+    int rc = calc_concs_sync(c, nullptr);
     if (rc) return rc;
     h_sums_kernel<<<stream_grid(c), kRedThreads, 0, c->st>>>(c->w, c->M, c->partials);
     reduce_partials_kernel<<<2, 256, 0, c->st>>>(c->partials, c->red_blocks, 2, c->red);
     c->launches += 2;
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(c->red_host, c->red, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(c->red_host + 2, c->Qd, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
-    const double wp_sum = c->red_host[0], wm2_sum = c->red_host[1];
+    const double wp_sum = c->red_host[0], wm2_sum = c->red_host[1], lnQ = c->red_host[3];
     *H = -lnQ + (wm2_sum / c->p.XbN - wp_sum) / (double)c->M;
     return LFTS_OK;
 }
@@ -1906,12 +1906,16 @@ int lfts_backward(lfts_ctx *c, int ckpt_every, double *dH_dL, double *dH_dXbN, d
         c->have_concs = false;  // phi was not recomputed
     }
     terms.flush();
+    h_sums_kernel<<<stream_grid(c), kRedThreads, 0, c->st>>>(c->w, M, c->partials);
+    reduce_partials_kernel<<<2, 256, 0, c->st>>>(c->partials, c->red_blocks, 2, c->red);
+    c->launches += 2;
     CK(cudaGetLastError());
     std::vector<double> part(3 * (size_t)nrows);
     CK(cudaMemcpyAsync(part.data(), c->adj_partial, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaMemcpyAsync(c->red_host, c->Qd, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(c->red_host, c->red, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(c->red_host + 2, c->Qd, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
-    const double Q = c->red_host[0], lnQ = c->red_host[1];
+    const double wp_sum = c->red_host[0], wm2_sum = c->red_host[1], Q = c->red_host[2], lnQ = c->red_host[3];
     double S[3] = {0.0, 0.0, 0.0};
     for (int b = 0; b < nrows; b++)
         for (int d = 0; d < 3; d++) S[d] += part[3 * (size_t)b + d];
@@ -1920,12 +1924,6 @@ int lfts_backward(lfts_ctx *c, int ckpt_every, double *dH_dL, double *dH_dXbN, d
         const double L = c->p.L[d];
         dH_dL[d] = -(kTwoPi * kTwoPi * S[d] / (3.0 * N * L * L * L)) / ((double)M * Q);
     }
-    h_sums_kernel<<<stream_grid(c), kRedThreads, 0, c->st>>>(c->w, M, c->partials);
-    reduce_partials_kernel<<<2, 256, 0, c->st>>>(c->partials, c->red_blocks, 2, c->red);
-    c->launches += 2;
-    CK(cudaMemcpyAsync(c->red_host, c->red, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    const double wp_sum = c->red_host[0], wm2_sum = c->red_host[1];
     const double X = c->p.XbN;
     if (dH_dXbN) *dH_dXbN = -wm2_sum / (X * X * (double)M);
     if (H) *H = -lnQ + (wm2_sum / X - wp_sum) / (double)M;
