@@ -58,6 +58,7 @@ struct AxisArgs {
     long long M;
     const double *w;           // INIT_W: W- (M) and w+ (M)
     double Nd;                 // N as a double (h = exp(-w/N))
+    double L[3];               // SELF kernels: box, for the tables that they make themselves
     const T *h;                // FP32: (hA, hB) pairs; FP64: [hA | hB]
     const T *src[2];           // INIT_Q: the chains' real rows
     T *q[2];                   // FP32: q[0] = the slot's pairs; FP64: each chain's half (null: not stored)
@@ -131,6 +132,20 @@ struct AxTables {
             const int k1 = i % R1, r = i / R1;
             tw(k1)[r] = twg[k1 * r];
             g(k1)[r] = gg[i];
+        }
+    }
+    // the same from the axis's length and box side, for callers without tables in
+    // memory: chain length nc, g divided by div
+    __device__ __forceinline__ void make(double L, int nc, double div, int tid, int nt)
+    {
+        const double two_pi = 6.283185307179586476925286766559005768;
+        for (int i = tid; i < N; i += nt) {
+            const int k1 = i % R1, r = i / R1, k = i <= N / 2 ? i : i - N;
+            double sn, cs;
+            sincospi(-2.0 * (k1 * r) / N, &sn, &cs);
+            tw(k1)[r] = {(T)cs, (T)sn};
+            const double ksq = (double)k * k / (L * L);
+            g(k1)[r] = (T)(exp(-two_pi * two_pi * ksq / (6.0 * nc)) / div);
         }
     }
     // stage B of one task: v[u], the inputs of outputs k1 + R1 k2, there and back
@@ -438,9 +453,9 @@ struct StridedCfg {
     using Conv = LineConv<T, R1, R2, CW, NT, true, Idx>;
 };
 
-template <typename T, int N, int CW, int MODE>
-__device__ __forceinline__ void strided_body(const AxisArgs<T> &a, const cpx<T> *twg, const T *gg, const int c,
-                                             const int stride, const int ncol, const int tile, const int base,
+// (SELF: the CTA makes its tables, AxTables::make)
+template <typename T, int N, int CW, int MODE, bool SELF, int AXIS>
+__device__ __forceinline__ void strided_body(const AxisArgs<T> &a, const int c, const int stride, const int ncol, const int tile, const int base,
                                              const int nctas)
 {
     using C = StridedCfg<T, N, CW>;
@@ -451,7 +466,10 @@ __device__ __forceinline__ void strided_body(const AxisArgs<T> &a, const cpx<T> 
     cpx<T> *sm = reinterpret_cast<cpx<T> *>(smem_raw);
     const int tid = threadIdx.x, col0 = tile * CW;
     typename C::Tables tab{smem_raw + C::TILE};
-    tab.load(twg, gg, tid, C::NT);
+    if constexpr (SELF)
+        tab.make(a.L[AXIS], (int)a.Nd, 1.0, tid, C::NT);
+    else
+        tab.load(AXIS == 0 ? a.twx : a.twy, AXIS == 0 ? a.gx : a.gy, tid, C::NT);
     pdl_wait();
 
     // complex value of stage-A task t's point j
@@ -534,29 +552,29 @@ __device__ __forceinline__ void strided_body(const AxisArgs<T> &a, const cpx<T> 
 }
 
 // x lines: tile of CW columns of chain c's field (FP64: pairs of real columns)
-template <typename T, int N, int CW, int MODE>
+template <typename T, int N, int CW, int MODE, bool SELF = false>
 __device__ __forceinline__ void xline_body(const AxisArgs<T> &a, int tile, int c, int nctas)
 {
     const int ncol = a.my * a.mz / kChains<T>;
-    strided_body<T, N, CW, MODE>(a, a.twx, a.gx, c, ncol, ncol, tile, 0, nctas);
+    strided_body<T, N, CW, MODE, SELF, 0>(a, c, ncol, ncol, tile, 0, nctas);
 }
 // y lines of x-plane x
-template <typename T, int N, int CW>
+template <typename T, int N, int CW, bool SELF = false>
 __device__ __forceinline__ void yline_body(const AxisArgs<T> &a, int tile, int x, int c)
 {
     const int ncol = a.mz / kChains<T>;
-    strided_body<T, N, CW, AX_CONV>(a, a.twy, a.gy, c, ncol, ncol, tile, x * N * ncol, 0);
+    strided_body<T, N, CW, AX_CONV, SELF, 1>(a, c, ncol, ncol, tile, x * N * ncol, 0);
 }
 
-template <typename T, int N, int CW, int MODE>
+template <typename T, int N, int CW, int MODE, bool SELF = false>
 __global__ void __launch_bounds__(StridedCfg<T, N, CW>::NT) xline_kernel(AxisArgs<T> a)
 {
-    xline_body<T, N, CW, MODE>(a, blockIdx.x, blockIdx.z + a.cbase, gridDim.x);
+    xline_body<T, N, CW, MODE, SELF>(a, blockIdx.x, blockIdx.z + a.cbase, gridDim.x);
 }
-template <typename T, int N, int CW>
+template <typename T, int N, int CW, bool SELF = false>
 __global__ void __launch_bounds__(StridedCfg<T, N, CW>::NT) yline_kernel(AxisArgs<T> a)
 {
-    yline_body<T, N, CW>(a, blockIdx.x, blockIdx.y, blockIdx.z + a.cbase);
+    yline_body<T, N, CW, SELF>(a, blockIdx.x, blockIdx.y, blockIdx.z + a.cbase);
 }
 
 // ------------------------------------------------------------- contiguous lines --
@@ -579,7 +597,7 @@ struct ZCfg {
     static_assert(PITCH >= SPAN, "pitch covers the padded line");
 };
 
-template <typename T, int N, int MODE>
+template <typename T, int N, int MODE, bool SELF = false>
 __device__ __forceinline__ void zline_body(const AxisArgs<T> &a, const int cta, const int c, const int nctas)
 {
     using C = ZCfg<T, N>;
@@ -593,7 +611,10 @@ __device__ __forceinline__ void zline_body(const AxisArgs<T> &a, const int cta, 
     const int nlines = a.mx * a.my / kChains<T>;
     const int line0 = (cta * C::NW + wid) * C::LPW;
     typename C::Tables tab{smem_raw + C::TILE};
-    tab.load(a.twz, a.gz, threadIdx.x, C::NT);
+    if constexpr (SELF)
+        tab.make(a.L[2], (int)a.Nd, (double)a.M, threadIdx.x, C::NT);
+    else
+        tab.load(a.twz, a.gz, threadIdx.x, C::NT);
     pdl_wait();
 
     auto live = [&](int t) { return V::okA(t) && line0 + V::lineA(t) < nlines; };
@@ -679,10 +700,10 @@ __device__ __forceinline__ void zline_body(const AxisArgs<T> &a, const int cta, 
     }
 }
 
-template <typename T, int N, int MODE>
+template <typename T, int N, int MODE, bool SELF = false>
 __global__ void __launch_bounds__(ZCfg<T, N>::NT) zline_kernel(AxisArgs<T> a)
 {
-    zline_body<T, N, MODE>(a, blockIdx.x, blockIdx.z + a.cbase, gridDim.x);
+    zline_body<T, N, MODE, SELF>(a, blockIdx.x, blockIdx.z + a.cbase, gridDim.x);
 }
 
 // -------------------------------------------------------------------- yz planes --
@@ -711,7 +732,7 @@ struct PlaneAxCfg {
     static_assert(PITCH >= SPAN, "pitch covers the padded row");
 };
 
-template <typename T, int NY, int NZ, int MODE>
+template <typename T, int NY, int NZ, int MODE, bool SELF = false>
 __device__ __forceinline__ void planeax_body(const AxisArgs<T> &a, const int x, const int c, const int nctas)
 {
     using C = PlaneAxCfg<T, NY, NZ>;
@@ -724,8 +745,13 @@ __device__ __forceinline__ void planeax_body(const AxisArgs<T> &a, const int x, 
     typename C::TabY taby{smem_raw + C::TILE};
     typename C::TabZ tabz{smem_raw + C::TILE + C::TabY::BYTES};
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    taby.load(a.twy, a.gy, threadIdx.x, C::NT);
-    tabz.load(a.twz, a.gz, threadIdx.x, C::NT);
+    if constexpr (SELF) {
+        taby.make(a.L[1], (int)a.Nd, 1.0, threadIdx.x, C::NT);
+        tabz.make(a.L[2], (int)a.Nd, (double)a.M, threadIdx.x, C::NT);
+    } else {
+        taby.load(a.twy, a.gy, threadIdx.x, C::NT);
+        tabz.load(a.twz, a.gz, threadIdx.x, C::NT);
+    }
     pdl_wait();
     cpx<T> *S = ax_field(a, c) + x * NY * C::NCOL;
 
@@ -886,10 +912,10 @@ __device__ __forceinline__ void planeax_body(const AxisArgs<T> &a, const int x, 
     }
 }
 
-template <typename T, int NY, int NZ, int MODE>
+template <typename T, int NY, int NZ, int MODE, bool SELF = false>
 __global__ void __launch_bounds__(PlaneAxCfg<T, NY, NZ>::NT) planeax_kernel(AxisArgs<T> a)
 {
-    planeax_body<T, NY, NZ, MODE>(a, blockIdx.x, blockIdx.z + a.cbase, gridDim.x);
+    planeax_body<T, NY, NZ, MODE, SELF>(a, blockIdx.x, blockIdx.z + a.cbase, gridDim.x);
 }
 
 }  // namespace lfts

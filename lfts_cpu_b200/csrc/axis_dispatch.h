@@ -25,6 +25,14 @@ struct AxisSet {
 bool axis_kernels(int mx, int my, int mz, int cw, AxisSet<double> *o);
 bool axis_kernels(int mx, int my, int mz, int cw, AxisSet<float> *o);
 
+// The kernels of one contour step on the caller's arrays that make their own
+// tables (FP64): z lines or planes from the caller's rows, y lines, x lines out
+struct AxisStepSet {
+    AxisFn<double> first, y, out;
+    bool planes;
+};
+bool axis_step_kernels(int mx, int my, int mz, AxisStepSet *o);
+
 // Columns per CTA of the x-line kernel that ends a chain, whatever the tile
 // choice: its CTAs' partial sums for Q then do not depend on the tiles.
 constexpr int kLastCw = 16;

@@ -3,9 +3,11 @@
 // (a host framework that owns every device allocation through its own pool,
 // a real-time loop that may not call into the allocator, or a library layered
 // under an allocator-free API).  The caller passes device inputs and outputs;
-// the step's scratch (the two chains' fields and the twiddle / Boltzmann-weight
-// tables) lives in one file-scope
-// device array of fixed size, so this path makes no allocation at all.
+// the step's scratch, the two chains' fields, lives in one file-scope device array
+// of fixed size, so this path makes no allocation at all.  The kernels make their
+// own twiddle and Boltzmann-weight tables in shared memory: a kernel of one CTA
+// that wrote them to memory first, with a plain launch for each of the others,
+// took 14.3 us a call at 24^3 against 9.9.
 //
 // Limits and sharing rules, stated once here and in include/lfts_b200.h:
 //  * FP64 only; 2 * mx * my * (mz/2 + 1) <= LFTS_NOALLOC_MAX_SPECTRUM complex
@@ -14,8 +16,8 @@
 //  * The array is one per device and shared by every call: two calls whose
 //    kernels overlap on a GPU (different streams, or different host threads)
 //    race on it.  Serialise them (one stream, or events).
-//  * Nothing in the array has to start at zero: every call rewrites the tables
-//    and the fields before reading them.  The array keeps the last call's contents.
+//  * Nothing in the array has to start at zero: every call rewrites the fields
+//    before reading them.  The array keeps the last call's contents.
 //  * The first call on a device looks up the array's device address (with
 //    that device current); make that first call before any stream capture.
 #include <cmath>
@@ -38,15 +40,8 @@ namespace {
 constexpr long long kMaxSpec = LFTS_NOALLOC_MAX_SPECTRUM;  // complex values, both chains
 constexpr int kMaxLen = 128;                               // largest compiled FFT length
 
-struct NoallocLayout {
-    static constexpr size_t spec = 0;
-    static constexpr size_t tw = spec + sizeof(cpx<double>) * kMaxSpec;      // 3 x kMaxLen complex
-    static constexpr size_t g = tw + sizeof(cpx<double>) * 3 * kMaxLen;      // 3 x kMaxLen doubles
-    static constexpr size_t bytes = g + sizeof(double) * 3 * kMaxLen;
-};
-
 // the scratch: one per device, shared by all calls (see the rules above)
-static __device__ __align__(256) unsigned char g_step_scratch[NoallocLayout::bytes];
+static __device__ __align__(256) unsigned char g_step_scratch[sizeof(cpx<double>) * kMaxSpec];
 
 constexpr int kMaxDevices = 64;
 // device address of g_step_scratch per device, looked up once per device
@@ -57,30 +52,6 @@ constexpr int kMaxDevices = 64;
 unsigned char *g_scratch_addr[kMaxDevices] = {};
 std::once_flag g_scratch_once[kMaxDevices];
 cudaError_t g_scratch_err[kMaxDevices] = {};
-
-// twiddles exp(-2 pi i t/n) and the factorised Boltzmann weight of
-// src/step.cc:69-89 (1/M folded into the z factor), computed on the device
-__global__ void noalloc_tables_kernel(cpx<double> *tw, double *g, int mx, int my, int mz, double Lx, double Ly,
-                                      double Lz, int N, double M)
-{
-    const int n[3] = {mx, my, mz};
-    const double L[3] = {Lx, Ly, Lz};
-    const double two_pi = 6.283185307179586476925286766559005768;
-    for (int d = 0; d < 3; d++) {
-        for (int t = threadIdx.x; t < n[d]; t += blockDim.x) {
-            double s, c;
-            sincospi(-2.0 * t / n[d], &s, &c);
-            tw[d * kMaxLen + t] = {c, s};
-        }
-        for (int K = threadIdx.x; K < n[d]; K += blockDim.x) {
-            const int k = K <= n[d] / 2 ? K : K - n[d];
-            const double ksq = (double)k * k / (L[d] * L[d]);
-            double v = exp(-two_pi * two_pi * ksq / (6.0 * N));
-            if (d == 2) v /= M;
-            g[d * kMaxLen + K] = v;
-        }
-    }
-}
 
 int fail(int code, const char *msg)
 {
@@ -102,13 +73,24 @@ int device_setup(int dev)
     return LFTS_OK;
 }
 
-// one launch of the step, with the kernel's dynamic shared-memory limit
-bool launch(const AxisFn<double> &f, dim3 grid, cudaStream_t st, const AxisArgs<double> &a)
+// one launch of the step, with the kernel's dynamic shared-memory limit; one after
+// the first may be scheduled while its predecessor drains (pdl_wait): its tables
+// are made by then
+bool launch(const AxisFn<double> &f, dim3 grid, cudaStream_t st, bool after, const AxisArgs<double> &a)
 {
     if (cudaFuncSetAttribute(f.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem) != cudaSuccess)
         return false;
-    f.fn<<<grid, f.nt, f.smem, st>>>(a);
-    return true;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(f.nt);
+    cfg.dynamicSmemBytes = f.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = after ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, f.fn, a) == cudaSuccess;
 }
 
 }  // namespace
@@ -131,8 +113,8 @@ int lfts_step_fwd_noalloc(const lfts_params *p, const double *q_in, double *q_ou
     if (2LL * mx * my * KZ > kMaxSpec)
         return fail(LFTS_ERR_ARG, "mesh above the no-alloc scratch limit: 2*mx*my*(mz/2+1) must be <= "
                                   "LFTS_NOALLOC_MAX_SPECTRUM (64^3 meshes fit)");
-    AxisSet<double> ax;
-    if (!axis_kernels(mx, my, mz, kLastCw, &ax))
+    AxisStepSet ax;
+    if (!axis_step_kernels(mx, my, mz, &ax))
         return fail(LFTS_ERR_UNSUPPORTED, "mesh size without an FFT kernel");
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices)
@@ -141,22 +123,13 @@ int lfts_step_fwd_noalloc(const lfts_params *p, const double *q_in, double *q_ou
     if (rc) return rc;
 
     unsigned char *base = g_scratch_addr[dev];
-    cpx<double> *tw = reinterpret_cast<cpx<double> *>(base + NoallocLayout::tw);
-    double *g = reinterpret_cast<double *>(base + NoallocLayout::g);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const long long M = (long long)mx * my * mz;
     const int NB = p->N - p->NA;
 
-    noalloc_tables_kernel<<<1, 128, 0, st>>>(tw, g, mx, my, mz, p->L[0], p->L[1], p->L[2], p->N, (double)M);
-
     AxisArgs<double> a{};
-    a.S = reinterpret_cast<double *>(base + NoallocLayout::spec);
-    a.twx = tw;
-    a.twy = tw + kMaxLen;
-    a.twz = tw + 2 * kMaxLen;
-    a.gx = g;
-    a.gy = g + kMaxLen;
-    a.gz = g + 2 * kMaxLen;
+    a.S = reinterpret_cast<double *>(base);
+    for (int d = 0; d < 3; d++) a.L[d] = p->L[d];
     a.mx = mx;
     a.my = my;
     a.mz = mz;
@@ -170,17 +143,11 @@ int lfts_step_fwd_noalloc(const lfts_params *p, const double *q_in, double *q_ou
     a.hsel[0] = i < p->NA ? 0 : 1;  // src/step.cc:53-57
     a.hsel[1] = i < NB ? 1 : 0;     // src/step.cc:60-64
     // z and y lines, then x lines and the product with h (axis_conv.cuh)
-    bool ok;
-    if (ax.planes) {
-        ok = launch(ax.plane[AX_INIT_Q], dim3(mx, 1, 2), st, a);
-    } else {
-        const AxisFn<double> &z = ax.z[AX_INIT_Q];
-        ok = launch(z, dim3((mx * my / 2 + z.per - 1) / z.per, 1, 2), st, a) &&
-             launch(ax.y, dim3((mz / 2 + ax.y.per - 1) / ax.y.per, mx, 2), st, a);
-    }
-    const AxisFn<double> &x = ax.x[AX_OUT];
-    ok = ok && launch(x, dim3((my * mz / 2 + x.per - 1) / x.per, 1, 2), st, a);
-    if (!ok) return fail(LFTS_ERR_CUDA, "cudaFuncSetAttribute failed");
+    const AxisFn<double> &f = ax.first, &x = ax.out;
+    bool ok = launch(f, dim3(ax.planes ? mx : (mx * my / 2 + f.per - 1) / f.per, 1, 2), st, false, a);
+    if (!ax.planes) ok = ok && launch(ax.y, dim3((mz / 2 + ax.y.per - 1) / ax.y.per, mx, 2), st, true, a);
+    ok = ok && launch(x, dim3((my * mz / 2 + x.per - 1) / x.per, 1, 2), st, true, a);
+    if (!ok) return fail(LFTS_ERR_CUDA, cudaGetErrorString(cudaGetLastError()));
 
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail(LFTS_ERR_CUDA, cudaGetErrorString(e));

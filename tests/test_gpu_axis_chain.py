@@ -114,3 +114,43 @@ def test_noalloc_step_on_8_byte_aligned_arrays(native_lib, m):
                     continue
                 ref = conv(q[c * M:(c + 1) * M].reshape(m), g).ravel() * h[hs[c] * M:(hs[c] + 1) * M]
                 assert rel_err(got[c * M:(c + 1) * M], ref) < FP64_TOL
+
+
+def test_noalloc_step_in_a_captured_graph(native_lib):
+    """After a first call, the step can be captured into a graph and replayed on
+    new contents of the same arrays."""
+    import torch
+
+    from lfts_cpu_b200.capi import Params
+    m, N, NA = (16, 32, 64), 7, 3
+    M, L = int(np.prod(m)), box((16, 32, 64))
+    p = Params()
+    p.N, p.NA, p.XbN, p.C, p.dt = N, NA, 15.0, 50.0, 0.5
+    for d in range(3):
+        p.m[d], p.L[d] = m[d], L[d]
+    q, h, out = (torch.ones(2 * M, dtype=torch.float64, device="cuda") for _ in range(3))
+
+    def call():
+        st = torch.cuda.current_stream().cuda_stream
+        assert native_lib.lfts_step_fwd_noalloc(C.byref(p), C.c_void_p(q.data_ptr()), C.c_void_p(out.data_ptr()),
+                                                C.c_void_p(h.data_ptr()), 2, C.c_void_p(st)) == 0
+
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call()
+    for seed in (1, 2):
+        rng = np.random.default_rng(seed)
+        qh, hh = rng.uniform(0.2, 1.5, 2 * M), rng.uniform(0.5, 1.2, 2 * M)
+        q.copy_(torch.from_numpy(qh))
+        h.copy_(torch.from_numpy(hh))
+        graph.replay()
+        torch.cuda.synchronize()
+        got = out.cpu().numpy()
+        g = weights(m, L, N)
+        for c, half in ((0, 0), (1, 1)):  # step 2 of NA = 3, NB = 4
+            ref = conv(qh[c * M:(c + 1) * M].reshape(m), g).ravel() * hh[half * M:(half + 1) * M]
+            assert rel_err(got[c * M:(c + 1) * M], ref) < FP64_TOL
