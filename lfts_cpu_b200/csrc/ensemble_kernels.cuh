@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(PlaneCCfg<float, NY, NZ>::NT, 1)
 
 // the three-stage plane body (64, 96, 128 planes), as the single context uses
 template <typename C3, int MODE>
-__global__ void __launch_bounds__(C3::NT, 1)
+__global__ void __launch_bounds__(C3::NT, C3::MINB)
     ens_plane3_kernel(EnsRep *__restrict__ reps, const int *__restrict__ members, int i)
 {
     const EnsRep &R = reps[members[blockIdx.y]];

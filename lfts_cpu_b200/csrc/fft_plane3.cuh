@@ -30,10 +30,10 @@
 
 namespace lfts {
 
-template <int NY_, int NZ_, int Y1_, int Z1_, int NT_, int KP_>
+template <int NY_, int NZ_, int Y1_, int Z1_, int NT_, int KP_, int MINB_ = 1>
 struct Plane3Cfg {
     static constexpr int NY = NY_, NZ = NZ_, Y1 = Y1_, Y2 = NY_ / Y1_, Z1 = Z1_, Z2 = NZ_ / Z1_;
-    static constexpr int NT = NT_, KP = KP_;
+    static constexpr int NT = NT_, KP = KP_, MINB = MINB_;  // threads, row pitch, CTAs per SM the registers allow
     static constexpr int NS1 = NZ * Y2, NS2 = Y1 * Z2, NS3 = NY * Z1;  // tasks per stage
     // TY[j2 * Y1 + k1] = w^(j2 k1) (NY entries), TZ[c1 * Z2 + jz] = w^(jz c1) (NZ entries)
     static constexpr size_t TOFF = sizeof(cpx<float>) * (size_t)(NY * KP);
@@ -41,7 +41,7 @@ struct Plane3Cfg {
     static constexpr size_t SMEM = TOFF + sizeof(cpx<float>) * (NY + NZ) + sizeof(float) * NZ;
     static __host__ __device__ constexpr int pos(int p) { return p + 2 * (p / Z2); }
     static_assert(Z2 == 16, "S3 runs of 16 values");
-    static_assert(NS1 <= NT && NS2 <= NT && NY + 2 * NZ <= NT, "at most one S1 / S2 task (table entry) per thread");
+    static_assert(NS1 <= NT && NY + 2 * NZ <= NT, "at most one S1 task (table entry) per thread");
     static_assert(pos(NZ - 1) < KP && KP % 2 == 0, "row pitch");
 };
 
@@ -49,6 +49,13 @@ struct Plane3Cfg {
 using Plane3_128 = Plane3Cfg<128, 128, 32, 8, 512, 142>;
 using Plane3_96 = Plane3Cfg<96, 96, 32, 6, 512, 108>;
 using Plane3_64 = Plane3Cfg<64, 64, 16, 4, 256, 72>;
+// 96 planes beyond one per SM (the ensemble's groups of several replicas): S1 has
+// 288 tasks, S2 512, S3 576.  With 288 threads and two rounds of S2 and S3, 91
+// registers let two CTAs share an SM; 512 threads, at one CTA per SM, leave 224
+// idle in S1 and need a second round of S3 for 64 tasks.  A capped step of the
+// 32-replica configuration, whose 8 replicas of 96^3 launch 768 planes, 68.3 ->
+// 59.0 ms.  PLANE_LAST keeps 512: its sum for Q is formed thread by thread.
+using Plane3_96s = Plane3Cfg<96, 96, 32, 6, 288, 108, 2>;
 
 // the 16 values of an S3 task: a run of 16 slots, 16-byte aligned
 __device__ __forceinline__ void p3_ld16(const cpx<float> *run, cpx<float> (&g)[16])
@@ -100,10 +107,9 @@ __device__ __forceinline__ void p3_s1_fwd(const cpx<float> *P, cpx<float> *__res
 }
 
 template <typename C>
-__device__ __forceinline__ void p3_s2_inv(cpx<float> *P, const cpx<float> *TY, const cpx<float> *TZ)
+__device__ __forceinline__ void p3_s2_inv_task(cpx<float> *P, const cpx<float> *TY, const cpx<float> *TZ,
+                                               const int t)
 {
-    const int t = threadIdx.x;
-    if (t >= C::NS2) return;
     const int jz = t % C::Z2, k1 = t / C::Z2;  // half-warps share k1, lanes run over jz
     cpx<float> d[C::Y2][C::Z1];
 #pragma unroll
@@ -138,12 +144,22 @@ __device__ __forceinline__ void p3_s2_inv(cpx<float> *P, const cpx<float> *TY, c
 #pragma unroll
         for (int c1 = 0; c1 < C::Z1; c1++) P[(k1 + C::Y1 * k2) * C::KP + C::pos(jz + C::Z2 * c1)] = d[k2][c1];
 }
-
 template <typename C>
-__device__ __forceinline__ void p3_s2_fwd(cpx<float> *P, const cpx<float> *TY, const cpx<float> *TZ)
+__device__ __forceinline__ void p3_s2_inv(cpx<float> *P, const cpx<float> *TY, const cpx<float> *TZ)
 {
     const int t = threadIdx.x;
-    if (t >= C::NS2) return;
+    if constexpr (C::NS2 <= C::NT) {
+        if (t < C::NS2) p3_s2_inv_task<C>(P, TY, TZ, t);
+    } else {
+#pragma unroll 1
+        for (int u = t; u < C::NS2; u += C::NT) p3_s2_inv_task<C>(P, TY, TZ, u);
+    }
+}
+
+template <typename C>
+__device__ __forceinline__ void p3_s2_fwd_task(cpx<float> *P, const cpx<float> *TY, const cpx<float> *TZ,
+                                               const int t)
+{
     const int jz = t % C::Z2, k1 = t / C::Z2;
     cpx<float> d[C::Y2][C::Z1];
 #pragma unroll
@@ -177,6 +193,17 @@ __device__ __forceinline__ void p3_s2_fwd(cpx<float> *P, const cpx<float> *TY, c
     for (int j2 = 0; j2 < C::Y2; j2++)
 #pragma unroll
         for (int b = 0; b < C::Z1; b++) P[(k1 + C::Y1 * j2) * C::KP + C::pos(jz + C::Z2 * b)] = d[j2][b];
+}
+template <typename C>
+__device__ __forceinline__ void p3_s2_fwd(cpx<float> *P, const cpx<float> *TY, const cpx<float> *TZ)
+{
+    const int t = threadIdx.x;
+    if constexpr (C::NS2 <= C::NT) {
+        if (t < C::NS2) p3_s2_fwd_task<C>(P, TY, TZ, t);
+    } else {
+#pragma unroll 1
+        for (int u = t; u < C::NS2; u += C::NT) p3_s2_fwd_task<C>(P, TY, TZ, u);
+    }
 }
 
 // S3 tasks: (y, c1) = (u / Z1, u % Z1) for u = threadIdx.x + NT s, s < ROUNDS
@@ -353,7 +380,7 @@ __device__ __forceinline__ void p3_prefetch_tail(const PlaneArgs<float> &a, cons
 }
 
 template <typename C, int MODE>
-__global__ void __launch_bounds__(C::NT, 1) plane3_kernel(PlaneArgs<float> a)
+__global__ void __launch_bounds__(C::NT, C::MINB) plane3_kernel(PlaneArgs<float> a)
 {
     if (MODE == PLANE_G && a.pf_ctas > 0) {
         const int mx = (int)gridDim.x - a.pf_ctas;

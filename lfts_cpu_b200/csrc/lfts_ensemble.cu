@@ -49,7 +49,7 @@ using PencilFn = void (*)(EnsRep *, const int *);
 
 struct PlaneSet {
     PlaneFn fn[4];
-    int nt;
+    int nt[4];
     size_t smem;
 };
 struct PencilSet {
@@ -66,10 +66,10 @@ void fill_plane(PlaneSet *o)
 {
     using C = PlaneCCfg<float, N, N>;
     o->fn[PLANE_INIT_W] = ens_plane_kernel<N, N, PLANE_INIT_W>;
-    o->fn[PLANE_INIT_Q] = ens_plane_kernel<N, N, PLANE_INIT_Q>;
+    o->fn[PLANE_INIT_Q] = nullptr;
     o->fn[PLANE_STEP] = ens_plane_kernel<N, N, PLANE_STEP>;
     o->fn[PLANE_LAST] = ens_plane_kernel<N, N, PLANE_LAST>;
-    o->nt = C::NT;
+    for (int m = 0; m < 4; m++) o->nt[m] = C::NT;
     o->smem = C::SMEM;
 }
 
@@ -82,26 +82,31 @@ void fill_pencil(PencilSet *o)
     o->smem = C::SMEM;
 }
 
-template <typename C3>
+// CL: the configuration of PLANE_LAST
+template <typename C3, typename CL = C3>
 void fill_plane3(PlaneSet *o)
 {
     o->fn[PLANE_INIT_W] = ens_plane3_kernel<C3, PLANE_INIT_W>;
-    o->fn[PLANE_INIT_Q] = ens_plane3_kernel<C3, PLANE_INIT_Q>;
+    o->fn[PLANE_INIT_Q] = nullptr;
     o->fn[PLANE_STEP] = ens_plane3_kernel<C3, PLANE_STEP>;
-    o->fn[PLANE_LAST] = ens_plane3_kernel<C3, PLANE_LAST>;
-    o->nt = C3::NT;
+    o->fn[PLANE_LAST] = ens_plane3_kernel<CL, PLANE_LAST>;
+    for (int m = 0; m < 4; m++) o->nt[m] = m == PLANE_LAST ? CL::NT : C3::NT;
     o->smem = C3::SMEM;
 }
 
 // yz-plane kernels of an ensemble mesh: three transform stages per axis
 // (fft_plane3.cuh: 64 and 96 planes) or two (fft_packed.cuh), the same bodies
 // a single FP32-mixed context runs with those tiles
-bool ens_plane(int ny, int nz, int stages, PlaneSet *o)
+// `several`: a launch has more planes than the GPU has SMs
+bool ens_plane(int ny, int nz, int stages, bool several, PlaneSet *o)
 {
     if (ny != nz) return false;
     if (stages == 3) {
         if (ny == 96) {
-            fill_plane3<Plane3_96>(o);
+            if (several)
+                fill_plane3<Plane3_96s, Plane3_96>(o);
+            else
+                fill_plane3<Plane3_96>(o);
             return true;
         }
         if (ny == 64) {
@@ -126,12 +131,13 @@ using PencilXFn = void (*)(EnsRep *, const int *, int);
 struct PencilXSet {
     PencilXFn fn[kPencilModes];
     PlaneFn plane_g;  // the chain's yz-plane kernel (PLANE_G, three stages)
+    int plane_g_nt;
     int nt;
     size_t smem;
 };
 
 template <int N, int CW>
-void fill_pencil_x(PencilXSet *o)
+void fill_pencil_x(PencilXSet *o, bool several)
 {
     using C = PencilCfg<float, N, CW>;
     for (int m = 0; m < kPencilModes; m++) o->fn[m] = nullptr;
@@ -140,18 +146,19 @@ void fill_pencil_x(PencilXSet *o)
     o->fn[PENCIL_H_LAST] = ens_pencil_x_kernel<N, CW, PENCIL_H_LAST>;
     o->fn[PENCIL_HA] = ens_pencil_x_kernel<N, CW, PENCIL_HA>;
     o->fn[PENCIL_HA_LAST] = ens_pencil_x_kernel<N, CW, PENCIL_HA_LAST>;
-    o->plane_g = ens_plane3_kernel<Plane3_96, PLANE_G>;
+    o->plane_g = several ? ens_plane3_kernel<Plane3_96s, PLANE_G> : ens_plane3_kernel<Plane3_96, PLANE_G>;
+    o->plane_g_nt = several ? Plane3_96s::NT : Plane3_96::NT;
     o->nt = C::NT;
     o->smem = C::SMEM;
 }
 
 // cubic 96^3 replicas only (the plane kernel is the three-stage 96 x 96 one)
-bool ens_pencil_x(int nx, int ny, int nz, int cw, PencilXSet *o)
+bool ens_pencil_x(int nx, int ny, int nz, int cw, bool several, PencilXSet *o)
 {
     if (nx != 96 || ny != 96 || nz != 96) return false;
-    if (cw == 8) { fill_pencil_x<96, 8>(o); return true; }
-    if (cw == 16) { fill_pencil_x<96, 16>(o); return true; }
-    if (cw == 32) { fill_pencil_x<96, 32>(o); return true; }
+    if (cw == 8) { fill_pencil_x<96, 8>(o, several); return true; }
+    if (cw == 16) { fill_pencil_x<96, 16>(o, several); return true; }
+    if (cw == 32) { fill_pencil_x<96, 32>(o, several); return true; }
     return false;
 }
 
@@ -172,6 +179,7 @@ bool ens_pencil(int nx, int cw, PencilSet *o)
 struct Group {
     int mx = 0, my = 0, mz = 0, cw = 0, stages = 2;
     int xh = 0, phi = 0;  // h-in-pencil chain; concentration sums in it
+    bool several = false;  // more planes than SMs
     std::vector<int> members;
     int *d_members = nullptr;
     PlaneSet pl{};
@@ -263,7 +271,7 @@ long long enqueue_group_chain(lfts_ensemble *e, Group &g, bool overlap)
         g.px.fn[PENCIL_INIT_W]<<<egrid, g.px.nt, g.px.smem, g.st>>>(e->d_reps, g.d_members, 0);
         n++;
         for (int i = 1; i < e->N; i++) {
-            launch_after(overlap, g.px.plane_g, pgrid, g.pl.nt, g.pl.smem, g.st, e->d_reps, (const int *)g.d_members, i);
+            launch_after(overlap, g.px.plane_g, pgrid, g.px.plane_g_nt, g.pl.smem, g.st, e->d_reps, (const int *)g.d_members, i);
             const int p = e->N - i;  // partner slot
             const bool last = i + 1 == e->N;
             const int mode = (!g.phi || p > i + 1) ? (last ? PENCIL_H_LAST : PENCIL_H)
@@ -274,11 +282,12 @@ long long enqueue_group_chain(lfts_ensemble *e, Group &g, bool overlap)
         ens_plane_q_sums_kernel<<<pgrid, 256, 0, g.st>>>(e->d_reps, g.d_members);
         return n + 1;
     }
-    g.pl.fn[PLANE_INIT_W]<<<pgrid, g.pl.nt, g.pl.smem, g.st>>>(e->d_reps, g.d_members, 0);
+    g.pl.fn[PLANE_INIT_W]<<<pgrid, g.pl.nt[PLANE_INIT_W], g.pl.smem, g.st>>>(e->d_reps, g.d_members, 0);
     n++;
     for (int i = 1; i < e->N; i++) {
         launch_after(overlap, g.pe.fn, egrid, g.pe.nt, g.pe.smem, g.st, e->d_reps, (const int *)g.d_members);
-        launch_after(overlap, g.pl.fn[i + 1 < e->N ? PLANE_STEP : PLANE_LAST], pgrid, g.pl.nt, g.pl.smem, g.st, e->d_reps,
+        const int mode = i + 1 < e->N ? PLANE_STEP : PLANE_LAST;
+        launch_after(overlap, g.pl.fn[mode], pgrid, g.pl.nt[mode], g.pl.smem, g.st, e->d_reps,
                      (const int *)g.d_members, i);
         n += 2;
     }
@@ -493,11 +502,11 @@ int set_group_tiles(Group &g, const GroupTiles &t)
     PlaneSet pl{};
     PencilSet pe{};
     PencilXSet px{};
-    if (!ens_plane(g.my, g.mz, t.stages, &pl) || !ens_pencil(g.mx, t.cw, &pe)) return LFTS_ERR_UNSUPPORTED;
+    if (!ens_plane(g.my, g.mz, t.stages, g.several, &pl) || !ens_pencil(g.mx, t.cw, &pe)) return LFTS_ERR_UNSUPPORTED;
     if (t.phi && !t.xh) return LFTS_ERR_UNSUPPORTED;
-    if (t.xh && (t.stages != 3 || !ens_pencil_x(g.mx, g.my, g.mz, t.cw, &px))) return LFTS_ERR_UNSUPPORTED;
+    if (t.xh && (t.stages != 3 || !ens_pencil_x(g.mx, g.my, g.mz, t.cw, g.several, &px))) return LFTS_ERR_UNSUPPORTED;
     for (int m = 0; m < 4; m++)
-        EK(cudaFuncSetAttribute(pl.fn[m], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
+        if (pl.fn[m]) EK(cudaFuncSetAttribute(pl.fn[m], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
     EK(cudaFuncSetAttribute(pe.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pe.smem));
     if (t.xh) {
         EK(cudaFuncSetAttribute(px.plane_g, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
@@ -545,7 +554,7 @@ std::vector<GroupTiles> group_candidates(const Group &g)
         for (int cw : {8, 16, 32}) {
             if (cw_forced > 0 && cw != cw_forced) continue;
             for (int xh : {0, 1}) {
-                if (xh && (stages != 3 || !ens_pencil_x(g.mx, g.my, g.mz, cw, &px))) continue;
+                if (xh && (stages != 3 || !ens_pencil_x(g.mx, g.my, g.mz, cw, g.several, &px))) continue;
                 if (fxh && ((fxh[0] != '0') != (xh == 1))) continue;
                 for (int phi : {0, 1}) {
                     if (phi && !xh) continue;
@@ -682,7 +691,7 @@ int lfts_ensemble_create(const lfts_params *params, const unsigned long long *se
         }
         PlaneSet ps;
         PencilSet qs;
-        if (!ens_plane(p.m[1], p.m[2], 2, &ps) || !ens_pencil(p.m[0], 16, &qs)) {
+        if (!ens_plane(p.m[1], p.m[2], 2, false, &ps) || !ens_pencil(p.m[0], 16, &qs)) {
             lfts_internal_set_error("ensemble meshes: 16, 24, 32, 48, 64 or 96 points per side, cubic planes");
             return LFTS_ERR_UNSUPPORTED;
         }
@@ -751,7 +760,7 @@ int lfts_ensemble_create(const lfts_params *params, const unsigned long long *se
             g.mz = c->mz;
             g.cw = 16;
             g.stages = 2;
-            ens_plane(g.my, g.mz, g.stages, &g.pl);
+            ens_plane(g.my, g.mz, g.stages, false, &g.pl);
             if (!ens_pencil(g.mx, g.cw, &g.pe)) return fail(LFTS_ERR_UNSUPPORTED);
             e->groups.push_back(g);
             gi = (int)e->groups.size() - 1;
@@ -762,6 +771,7 @@ int lfts_ensemble_create(const lfts_params *params, const unsigned long long *se
         cudaEventCreateWithFlags(&e->fork, cudaEventDisableTiming) != cudaSuccess)
         return fail(LFTS_ERR_CUDA);
     for (Group &g : e->groups) {
+        g.several = g.mx * (int)g.members.size() > e->rep[0]->sms;
         if (cudaStreamCreateWithFlags(&g.st, cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreateWithFlags(&g.join, cudaEventDisableTiming) != cudaSuccess ||
             cudaMalloc(&g.d_members, sizeof(int) * g.members.size()) != cudaSuccess ||
@@ -769,7 +779,7 @@ int lfts_ensemble_create(const lfts_params *params, const unsigned long long *se
                 cudaSuccess)
             return fail(LFTS_ERR_CUDA);
         for (int m = 0; m < 4; m++)
-            if (cudaFuncSetAttribute(g.pl.fn[m], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.pl.smem) !=
+            if (g.pl.fn[m] && cudaFuncSetAttribute(g.pl.fn[m], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.pl.smem) !=
                 cudaSuccess)
                 return fail(LFTS_ERR_CUDA);
         if (cudaFuncSetAttribute(g.pe.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.pe.smem) !=
