@@ -38,8 +38,8 @@ struct lfts_ctx {
     unsigned *ticket = nullptr;  // CTAs of the chain's last kernel that are done
     double *Qd = nullptr;      // Q, ln Q
     double *partials = nullptr;
-    double *red = nullptr;     // kRedWidth reduced values (device)
-    double *red_host = nullptr;  // pinned copy
+    double *red_host = nullptr;  // kRedWidth reduced values (pinned host memory that kernels write)
+    double *Q_host = nullptr;    // Q, ln Q of the last concentrations (beside it)
     int red_blocks = 0;
 
     double *eta[2] = {};       // Langevin noise: prev, new

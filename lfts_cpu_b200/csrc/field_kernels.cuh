@@ -368,11 +368,19 @@ __device__ __forceinline__ void concentrations_acc_body(
     if (Dh0) dot_partials(dots, nh, sh, partials + (long long)blk * kRedWidth);
 }
 
+// Q and ln Q into pinned host memory: the host reads them after its next
+// synchronisation, without a copy in between (each took about 4 us of a call)
+__device__ __forceinline__ void q_to_host(const double *Qd, double *Q_host)
+{
+    if (Q_host && blockIdx.x == 0 && threadIdx.x < 2) Q_host[threadIdx.x] = Qd[threadIdx.x];
+}
+
 static __global__ void __launch_bounds__(kRedThreads, 4) concentrations_acc_kernel(
     const float *__restrict__ acc, const float *__restrict__ h, long long M, int N, double *__restrict__ phim,
     double *__restrict__ phip, const double *__restrict__ Qd, float *__restrict__ Dh0, int nh, HistPtrs hist,
-    double *__restrict__ partials)
+    double *__restrict__ partials, double *Q_host)
 {
+    q_to_host(Qd, Q_host);
     concentrations_acc_body(acc, h, M, N, phim, phip, Qd, Dh0, nh, hist, partials, blockIdx.x, gridDim.x);
 }
 
@@ -380,14 +388,16 @@ template <typename T, bool SPLIT>
 static __global__ void __launch_bounds__(kRedThreads, 4) concentrations_kernel(
     const T *__restrict__ q, long long M, int N, int NA, const double *__restrict__ w,
     double *__restrict__ phim, double *__restrict__ phip, const double *__restrict__ Qd,
-    T *__restrict__ Dh0, int nh, HistPtrs hist, double *__restrict__ partials)
+    T *__restrict__ Dh0, int nh, HistPtrs hist, double *__restrict__ partials, double *Q_host)
 {
+    q_to_host(Qd, Q_host);
     concentrations_body<T, SPLIT>(q, M, N, NA, w, phim, phip, Qd, Dh0, nh, hist, partials, blockIdx.x, gridDim.x);
 }
 
 // out[m] = sum over blocks of partials[b][m], fixed order; block m < width
 // reduces column m (launch width blocks of 256 threads: every column's sum
-// is formed in the same order as by one block looping over the columns)
+// is formed in the same order as by one block looping over the columns); out
+// may be pinned host memory, as Q_host above
 static __global__ void reduce_partials_kernel(const double *partials, int nblocks, int width, double *out)
 {
     __shared__ double sh[32];

@@ -526,7 +526,8 @@ void launch_concs(lfts_ctx *c, void *Dh0, int nh, const HistPtrs &hist)
     auto *fn = conc_slices<T>(c->M, c->N, c->red_blocks) > 1 ? concentrations_kernel<T, true>
                                                              : concentrations_kernel<T, false>;
     fn<<<stream_grid(c), kRedThreads, 0, c->st>>>(static_cast<const T *>(c->q), c->M, c->N, c->NA, c->w, c->w + 2 * c->M,
-                                                  c->w + 3 * c->M, c->Qd, static_cast<T *>(Dh0), nh, hist, c->partials);
+                                                  c->w + 3 * c->M, c->Qd, static_cast<T *>(Dh0), nh, hist, c->partials,
+                                                  c->Q_host);
 }
 
 template <typename T>
@@ -536,12 +537,12 @@ void enqueue_concs(lfts_ctx *c, void *Dh0, int nh, const HistPtrs &hist)
     if (c->phi_in_chain)
         concentrations_acc_kernel<<<stream_grid(c), kRedThreads, 0, c->st>>>(
             static_cast<const float *>(c->acc), static_cast<const float *>(c->q), c->M, c->N, c->w + 2 * c->M,
-            c->w + 3 * c->M, c->Qd, static_cast<float *>(Dh0), nh, hist, c->partials);
+            c->w + 3 * c->M, c->Qd, static_cast<float *>(Dh0), nh, hist, c->partials, c->Q_host);
     else
         launch_concs<T>(c, Dh0, nh, hist);
     c->launches++;
     if (Dh0) {
-        reduce_partials_kernel<<<nh + 1, 256, 0, c->st>>>(c->partials, c->red_blocks, nh + 1, c->red);
+        reduce_partials_kernel<<<nh + 1, 256, 0, c->st>>>(c->partials, c->red_blocks, nh + 1, c->red_host);
         c->launches++;
     }
 }
@@ -748,7 +749,7 @@ void enqueue_calc(lfts_ctx *c)
     if (c->phi_in_chain)
         concentrations_acc_kernel<<<stream_grid(c), kRedThreads, 0, c->st>>>(
             static_cast<const float *>(c->acc), static_cast<const float *>(c->q), c->M, c->N, c->w + 2 * c->M,
-            c->w + 3 * c->M, c->Qd, nullptr, 0, HistPtrs{}, c->partials);
+            c->w + 3 * c->M, c->Qd, nullptr, 0, HistPtrs{}, c->partials, c->Q_host);
     else
         launch_concs<T>(c, nullptr, 0, HistPtrs{});
 }
@@ -955,9 +956,8 @@ int calc_concs_sync(lfts_ctx *c, double *lnQ)
     enqueue_concs_any(c, nullptr, 0, none);
     CK(cudaGetLastError());
     if (lnQ) {
-        CK(cudaMemcpyAsync(c->red_host, c->Qd, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
         CK(cudaStreamSynchronize(c->st));
-        *lnQ = c->red_host[1];
+        *lnQ = c->Q_host[1];
     }
     c->have_concs = true;
     return LFTS_OK;
@@ -982,7 +982,6 @@ int anderson_mix_host(lfts_ctx *c, int maxIter, double errTol, int *k_out)
         }
         void *Dh0 = c->Dh[c->cur];
         enqueue_concs_any(c, Dh0, nh, Dhp);
-        CK(cudaMemcpyAsync(c->red_host, c->red, (nh + 1) * sizeof(double), cudaMemcpyDeviceToHost, c->st));
         CK(cudaStreamSynchronize(c->st));
         const double S1 = c->red_host[0];
         err = std::pow(S1 / (double)M, 0.5);
@@ -1288,8 +1287,8 @@ int ctx_alloc(lfts_ctx *c)
     CK(cudaMemset(c->ticket, 0, sizeof(unsigned)));
     CK(cudaMalloc(&c->Qd, sizeof(double) * 2));
     CK(cudaMalloc(&c->partials, sizeof(double) * kRedWidth * c->red_blocks));
-    CK(cudaMalloc(&c->red, sizeof(double) * kRedWidth));
-    CK(cudaMallocHost(&c->red_host, sizeof(double) * kRedWidth));
+    CK(cudaMallocHost(&c->red_host, sizeof(double) * (kRedWidth + 2)));
+    c->Q_host = c->red_host + kRedWidth;
     for (int i = 0; i < 2; i++) {
         CK(cudaMalloc(&c->eta[i], sizeof(double) * M));
         CK(cudaMemset(c->eta[i], 0, sizeof(double) * M));
@@ -1329,7 +1328,6 @@ void ctx_free(lfts_ctx *c)
     cudaFree(c->ticket);
     cudaFree(c->Qd);
     cudaFree(c->partials);
-    cudaFree(c->red);
     if (c->red_host) cudaFreeHost(c->red_host);
     for (int i = 0; i < 2; i++) cudaFree(c->eta[i]);
     for (int i = 0; i < kRedWidth; i++) {
@@ -1801,13 +1799,11 @@ int lfts_get_H(lfts_ctx *c, double *H)
     int rc = calc_concs_sync(c, nullptr);
     if (rc) return rc;
     h_sums_kernel<<<stream_grid(c), kRedThreads, 0, c->st>>>(c->w, c->M, c->partials);
-    reduce_partials_kernel<<<2, 256, 0, c->st>>>(c->partials, c->red_blocks, 2, c->red);
+    reduce_partials_kernel<<<2, 256, 0, c->st>>>(c->partials, c->red_blocks, 2, c->red_host);
     c->launches += 2;
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(c->red_host, c->red, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaMemcpyAsync(c->red_host + 2, c->Qd, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
-    const double wp_sum = c->red_host[0], wm2_sum = c->red_host[1], lnQ = c->red_host[3];
+    const double wp_sum = c->red_host[0], wm2_sum = c->red_host[1], lnQ = c->Q_host[1];
     *H = -lnQ + (wm2_sum / c->p.XbN - wp_sum) / (double)c->M;
     return LFTS_OK;
 }
@@ -1907,15 +1903,14 @@ int lfts_backward(lfts_ctx *c, int ckpt_every, double *dH_dL, double *dH_dXbN, d
     }
     terms.flush();
     h_sums_kernel<<<stream_grid(c), kRedThreads, 0, c->st>>>(c->w, M, c->partials);
-    reduce_partials_kernel<<<2, 256, 0, c->st>>>(c->partials, c->red_blocks, 2, c->red);
+    reduce_partials_kernel<<<2, 256, 0, c->st>>>(c->partials, c->red_blocks, 2, c->red_host);
     c->launches += 2;
     CK(cudaGetLastError());
     std::vector<double> part(3 * (size_t)nrows);
     CK(cudaMemcpyAsync(part.data(), c->adj_partial, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaMemcpyAsync(c->red_host, c->red, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaMemcpyAsync(c->red_host + 2, c->Qd, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(c->Q_host, c->Qd, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
-    const double wp_sum = c->red_host[0], wm2_sum = c->red_host[1], Q = c->red_host[2], lnQ = c->red_host[3];
+    const double wp_sum = c->red_host[0], wm2_sum = c->red_host[1], Q = c->Q_host[0], lnQ = c->Q_host[1];
     double S[3] = {0.0, 0.0, 0.0};
     for (int b = 0; b < nrows; b++)
         for (int d = 0; d < 3; d++) S[d] += part[3 * (size_t)b + d];
@@ -1969,10 +1964,10 @@ int lfts_profile_iteration(lfts_ctx *c, int reps, double *ms_chain, double *ms_c
         else if (c->phi_in_chain)
             concentrations_acc_kernel<<<stream_grid(c), kRedThreads, 0, c->st>>>(
                 static_cast<const float *>(c->acc), static_cast<const float *>(c->q), M, c->N, c->w + 2 * M,
-                c->w + 3 * M, c->Qd, static_cast<float *>(c->Dh[c->cur]), kMaxHist, Dhp, c->partials);
+                c->w + 3 * M, c->Qd, static_cast<float *>(c->Dh[c->cur]), kMaxHist, Dhp, c->partials, c->Q_host);
         else
             launch_concs<float>(c, c->Dh[c->cur], kMaxHist, Dhp);
-        reduce_partials_kernel<<<kRedWidth, 256, 0, c->st>>>(c->partials, c->red_blocks, kRedWidth, c->red);
+        reduce_partials_kernel<<<kRedWidth, 256, 0, c->st>>>(c->partials, c->red_blocks, kRedWidth, c->red_host);
     }
     CK(cudaEventRecord(ev[2], c->st));
     for (int r = 0; r < reps; r++) {
