@@ -42,7 +42,7 @@ int cuda_fail(cudaError_t e, const char *what)
 
 constexpr double kTwoPi = 6.283185307179586476925286766559005768;
 // x-pencil tile widths used when autotuning is off (the usual winners at 128^3)
-constexpr int kDefaultCwFp32 = 16, kDefaultCwFp64 = 32;
+constexpr int kDefaultCwFp32 = 16, kDefaultCwFp64 = 16;
 
 // Gaussian elimination with partial pivoting (first maximal |pivot|,
 // reciprocal scaling of the sub-column, right-looking rank-1 updates), then
@@ -702,6 +702,9 @@ int apply_default_tiles(lfts_ctx *c, const lfts_tiles &t)
 // (LFTS_PENCIL_CW, LFTS_ONE_STREAM, LFTS_PHI_IN_CHAIN fix one choice each;
 // LFTS_XH_CHAIN=0 leaves the sums out).  plane_stages and h_in_pencil name the
 // transform chain that such a choice belongs to.
+// The width that was the fastest on none of the cubic meshes is not tried: FP64 32
+// (64^3 460 us a call against 423, 128^3 2562 against 2223), FP32 8 (354 against 326,
+// 1405 against 1273); it costs a context's first creation as much as the others.
 std::vector<lfts_tiles> tile_candidates(const lfts_ctx *c)
 {
     std::vector<lfts_tiles> out;
@@ -711,7 +714,7 @@ std::vector<lfts_tiles> tile_candidates(const lfts_ctx *c)
     const char *fphi = std::getenv("LFTS_PHI_IN_CHAIN");
     const int cw_forced = fcw ? std::atoi(fcw) : 0;
     for (int cw : {8, 16, 32}) {
-        if (cw_forced > 0 && cw != cw_forced) continue;
+        if (cw_forced > 0 ? cw != cw_forced : cw == (c->prec == LFTS_FP64 ? 32 : 8)) continue;
         if (c->prec == LFTS_FP64) {
             for (int two : {1, 0}) {
                 if (fone && ((fone[0] == '1') == (two == 1))) continue;
@@ -740,28 +743,15 @@ lfts_tiles default_tiles(const lfts_ctx *c)
     return cand.empty() ? lfts_tiles{cw, 2, 0, c->prec == LFTS_FP64 ? 1 : 0, 0, 1} : cand.front();
 }
 
-// one calc_concs without the Anderson dot products: the chain, then the
-// concentrations from the stored slots or from the sums the chain formed
-template <typename T>
-void enqueue_calc(lfts_ctx *c)
-{
-    enqueue_chain_launches<T>(c);
-    if (c->phi_in_chain)
-        concentrations_acc_kernel<<<stream_grid(c), kRedThreads, 0, c->st>>>(
-            static_cast<const float *>(c->acc), static_cast<const float *>(c->q), c->M, c->N, c->w + 2 * c->M,
-            c->w + 3 * c->M, c->Qd, nullptr, 0, HistPtrs{}, c->partials, c->Q_host);
-    else
-        launch_concs<T>(c, nullptr, 0, HistPtrs{});
-}
-
-// a tile choice is timed on whole calc_concs (chain + concentrations): the
-// choices differ in how the concentration work is split between them
-template <typename T>
+// a tile choice is timed on whole calc_concs, replayed from the chain's graph as
+// calls run it (launched one by one, a chain of 3 us kernels takes the host's time:
+// 64^3 FP64 then got 460 us a call where the best choice takes 423)
 int time_chain(lfts_ctx *c, cudaEvent_t e0, cudaEvent_t e1, float *ms)
 {
-    enqueue_calc<T>(c);  // warm-up
+    HistPtrs none{};
+    enqueue_concs_any(c, nullptr, 0, none);  // warm-up
     CK(cudaEventRecord(e0, c->st));
-    for (int r = 0; r < 3; r++) enqueue_calc<T>(c);
+    for (int r = 0; r < 3; r++) enqueue_concs_any(c, nullptr, 0, none);
     CK(cudaEventRecord(e1, c->st));
     CK(cudaEventSynchronize(e1));
     CK(cudaGetLastError());
@@ -781,8 +771,7 @@ int tune_tiles(lfts_ctx *c, lfts_tiles *best)
     for (const lfts_tiles &t : tile_candidates(c)) {
         if (apply_default_tiles(c, t) != LFTS_OK) continue;
         float ms = 0.f;
-        rc = c->prec == LFTS_FP64 ? time_chain<double>(c, e0, e1, &ms) : time_chain<float>(c, e0, e1, &ms);
-        if (rc) break;
+        if ((rc = time_chain(c, e0, e1, &ms))) break;
         if (!found || ms < best_ms) {
             best_ms = ms;
             *best = t;
