@@ -427,6 +427,17 @@ __device__ __forceinline__ void pencil_body(const PencilArgs<T> &a, const int ti
         twx[t] = a.twx[t];
         if (MODE == PENCIL_CONV) gxs[t] = a.gx[t];  // POWER mode has no g table
     }
+    // g along y and z of this thread's column (its tasks are whole columns apart), fetched
+    // while the predecessor drains: loaded where it is used, behind the transform, its
+    // latency lay in the chain of every step (48^3 FP32 415 us a calc_concs against 407,
+    // a body iteration of the ensemble's 32 replicas 7.38 ms against 7.25, both with the
+    // h pairs below ahead of the transform too)
+    static_assert(C::NT % CW == 0, "tasks of one thread are a multiple of CW apart");
+    T gyz = 0;
+    if (MODE == PENCIL_CONV) {
+        const int col = col0 + threadIdx.x % CW;
+        if (col < ncol) gyz = a.gy[col / a.KZ] * a.gz[col % a.KZ];
+    }
     pdl_wait();
 
     // X1: forward stage A from global (strided rows), twiddles, to smem.  At
@@ -474,6 +485,14 @@ __device__ __forceinline__ void pencil_body(const PencilArgs<T> &a, const int ti
                 av[k2] = a.acc_init ? make_float2(0.f, 0.f) : ap[o];
             }
         }
+        // the (hA, hB) pairs (L2), for the same reason
+        constexpr bool kH = kAcc || MODE == PENCIL_H || MODE == PENCIL_H_LAST;
+        float2 hv[kH ? R2 : 1];
+        if constexpr (kH) {
+#pragma unroll
+            for (int k2 = 0; k2 < R2; k2++)
+                hv[k2] = __ldg(reinterpret_cast<const float2 *>(a.h) + (long long)(k1 + R1 * k2) * ncol + col);
+        }
         if constexpr (MODE == PENCIL_INIT_W) {
             // hA = exp(-(W- + w+)/N), hB = exp(-(-W- + w+)/N)  (src/diblock.cc:64-72),
             // single-precision exponential as the FP32 plane kernels' INIT_W
@@ -498,7 +517,7 @@ __device__ __forceinline__ void pencil_body(const PencilArgs<T> &a, const int ti
 #pragma unroll
             for (int k2 = 0; k2 < R2; k2++) {
                 const long long o = (long long)(k1 + R1 * k2) * ncol + col;
-                const float2 h = __ldg(reinterpret_cast<const float2 *>(a.h) + o);
+                const float2 h = hv[k2];
                 const float va = v[k2].x * (hs0 ? h.y : h.x);
                 const float vb = v[k2].y * (hs1 ? h.y : h.x);
                 __stcs(reinterpret_cast<float2 *>(a.qout) + o, make_float2(va, vb));
@@ -513,7 +532,7 @@ __device__ __forceinline__ void pencil_body(const PencilArgs<T> &a, const int ti
 #pragma unroll
             for (int k2 = 0; k2 < R2; k2++) {
                 const long long o = (long long)(k1 + R1 * k2) * ncol + col;
-                const float2 h = __ldg(reinterpret_cast<const float2 *>(a.h) + o);
+                const float2 h = hv[k2];
                 const float va = v[k2].x * (hs0 ? h.y : h.x);
                 const float vb = v[k2].y * (hs1 ? h.y : h.x);
                 if (MODE == PENCIL_HA_LAST) __stcs(reinterpret_cast<float2 *>(a.qout) + o, make_float2(va, vb));
@@ -546,7 +565,6 @@ __device__ __forceinline__ void pencil_body(const PencilArgs<T> &a, const int ti
             for (int u = 0; u < R2; u++) Tl[C::row(R2 * k1 + u) * CW + cl] = ctw<1>(v[u], twx[(u * k1) % NX]);
         }
         if (MODE == PENCIL_CONV) {
-            const T gyz = a.gy[col / a.KZ] * a.gz[col % a.KZ];
 #pragma unroll
             for (int k2 = 0; k2 < R2; k2++) v[k2] = cscale(v[k2], gxs[k1 + R1 * k2] * gyz);
             Dft<R2, 1, T>::run(v);

@@ -186,8 +186,11 @@ __device__ __forceinline__ void pc_z_fwdB(cpx<T> *P)
     }
 }
 
-// h values of this warp's stage-B tasks (rows in transposed y order); loaded
-// before the first z phase so the DRAM latency overlaps its shared-memory work.
+// h values of this warp's stage-B tasks (rows in transposed y order); those of the
+// first round are loaded with the spectrum (before the first z phase, whose
+// shared-memory work is shorter than the load, a calc_concs of 24^3 took 335 us
+// against 320, of 48^3 418 against 413), the rest before the first z phase
+// (register budget).
 // 8-byte pair load / streaming store of the stored propagators
 __device__ __forceinline__ cpx<float> ld_pair(const cpx<float> *p)
 {
@@ -377,9 +380,12 @@ __device__ __forceinline__ void plane_c_body(const PlaneArgs<T> &a, const int x,
         return;
     }
 
+    PcH<C, T> hv;
+    const cpx<T> *hp = reinterpret_cast<const cpx<T> *>(a.h) + plane_off;
     {
         cpx<T> v[C::RY1];
         pc_y_invA_load<C>(Sg, v);
+        hv.load(hp, a.hsel0, a.hsel1, 0, 1);
         tws.store(twy);
         __syncthreads();
         pc_y_A<C>(P, v, twy, true);
@@ -388,11 +394,6 @@ __device__ __forceinline__ void plane_c_body(const PlaneArgs<T> &a, const int x,
     pc_y_B<C, 1, false>(P, twy);
     __syncthreads();
     // z section, warp-local (rows in transposed y order)
-    // h of the first stage-B round goes out before the first z phase, the
-    // rest after it (register budget)
-    PcH<C, T> hv;
-    const cpx<T> *hp = reinterpret_cast<const cpx<T> *>(a.h) + plane_off;
-    hv.load(hp, a.hsel0, a.hsel1, 0, 1);
     pc_z_A<C, 1, true>(P, twa);
     hv.load(hp, a.hsel0, a.hsel1, 1, PcH<C, T>::RND);
     __syncwarp();
