@@ -61,7 +61,6 @@ __global__ void __launch_bounds__(PlaneCCfg<float, NY, NZ>::NT, 1)
     a.twy = R.tw[1];
     a.twz = R.tw[2];
     a.qpart = R.qpart;
-    a.nchains = 2;
     a.Nd = (double)R.N;
     if (MODE == PLANE_INIT_W) {
         a.qout = R.q;  // slot 1 = [hA | hB]
@@ -87,12 +86,11 @@ __global__ void __launch_bounds__(C3::NT, C3::MINB)
     a.twy = R.tw[1];
     a.twz = R.tw[2];
     a.qpart = R.qpart;
-    a.nchains = 2;
     a.Nd = (double)R.N;
     if (MODE == PLANE_INIT_W) {
         a.qout = R.q;
     } else if (MODE == PLANE_G) {
-        // the h-in-pencil chain's plane (enqueue_chain_launches): g from the
+        // the h-in-pencil chain's plane (enqueue_transform_chain): g from the
         // separable tables; ahead of a summing pencil, its partner slot to L2
         a.gx = R.g[0];
         a.gy = R.g[1];
@@ -108,7 +106,7 @@ __global__ void __launch_bounds__(C3::NT, C3::MINB)
 }
 
 // The h-in-pencil chain's x-pencils (the single context's
-// enqueue_chain_launches, same arguments): INIT_W (h from the fields, stored
+// enqueue_transform_chain, same arguments): INIT_W (h from the fields, stored
 // as slot 1), H (store slot i+1), and, from the middle of the chain on when
 // the replica forms its concentration sums in the chain (R.acc), HA / HA_LAST
 // (add the slot's products with its stored partner slot N-i).

@@ -12,7 +12,6 @@ static void fill_plane_c(PlaneKernels<T> *o)
 {
     using C = PlaneCCfg<T, NY, NZ>;
     o->fn[PLANE_INIT_W] = plane_c_kernel<T, NY, NZ, PLANE_INIT_W>;
-    o->fn[PLANE_INIT_Q] = nullptr;  // steps of given rows run axis by axis
     o->fn[PLANE_STEP] = plane_c_kernel<T, NY, NZ, PLANE_STEP>;
     o->fn[PLANE_LAST] = plane_c_kernel<T, NY, NZ, PLANE_LAST>;
     o->fn[PLANE_G] = nullptr;
@@ -71,7 +70,6 @@ template <typename C>
 static void fill_plane3(PlaneKernels<float> *o)
 {
     o->fn[PLANE_INIT_W] = plane3_kernel<C, PLANE_INIT_W>;
-    o->fn[PLANE_INIT_Q] = nullptr;  // steps of given rows run axis by axis
     o->fn[PLANE_STEP] = plane3_kernel<C, PLANE_STEP>;
     o->fn[PLANE_LAST] = plane3_kernel<C, PLANE_LAST>;
     // the h-in-pencil chain runs on 96 x 96 and 128 x 128 planes

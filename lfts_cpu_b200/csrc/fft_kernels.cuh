@@ -39,27 +39,21 @@ __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefe
 
 enum PlaneMode : int {
     PLANE_INIT_W = 0,  // h = exp(-w/N) from the fields, store h, forward transform
-    PLANE_INIT_Q = 1,  // forward transform of given real rows (q_in or W-)
-    PLANE_STEP = 2,    // inverse, x h, store q, forward
-    PLANE_LAST = 3,    // inverse, x h, store q, partial sum of chain 0 (for Q)
-    PLANE_G = 4,       // inverse, x g (separable tables), forward; stores nothing
+    PLANE_STEP = 1,    // inverse, x h, store q, forward
+    PLANE_LAST = 2,    // inverse, x h, store q, partial sum of chain 0 (for Q)
+    PLANE_G = 3,       // inverse, x g (separable tables), forward; stores nothing
 };
-constexpr int kPlaneModes = 5;
+constexpr int kPlaneModes = 4;
 
 template <typename T>
 struct PlaneArgs {
     const double *w;      // INIT_W: W- (M) and w+ (M), FP64
-    const T *src;         // INIT_Q: source rows, chain c at src + c*src_stride
-    long long src_stride;
-    const double *src64;  // INIT_Q from FP64 rows (used when src == nullptr)
     T *qout;              // stored propagators, chain c at qout + c*M
     const T *h;           // [hA | hB]
     cpx<T> *spec;         // half spectra, chain c at spec + c*mx*my*KZ
     const cpx<T> *twy, *twz;  // exp(-2 pi i t/n) tables
     double *qpart;        // LAST: per-plane sums of chain 0
     int hsel0, hsel1;     // h half used by chain 0 / chain 1 (0 = hA, 1 = hB)
-    int cbase;            // chain index of blockIdx.y == 0 (one-chain launches)
-    int nchains;
     double Nd;            // N as a double (h = exp(-w/N))
     const T *gx, *gy, *gz;  // PLANE_G: separable Boltzmann weight, 1/M folded into gz
     const T *pf;          // PLANE_G: (chain 1, chain 2) slot that the next x-pencil reads, pulled into L2
@@ -358,7 +352,7 @@ __global__ void __launch_bounds__(PlaneCfg<double, NY, NZ>::NT) fwd_plane_kernel
 enum PencilMode : int {
     PENCIL_CONV = 0,    // forward x, times g, inverse x (in place in the spectrum)
     PENCIL_POWER = 1,   // forward x, S += |X|^2 (structure function sample)
-    // the h-in-pencil chain (FP32 packed field): see enqueue_chain_launches
+    // the h-in-pencil chain (FP32 packed field): see enqueue_transform_chain
     PENCIL_H = 2,       // forward x, times h, store q, inverse x
     PENCIL_H_LAST = 3,  // forward x, times h, store q
     PENCIL_INIT_W = 4,  // h = exp(-w/N) from the fields, store it, inverse x
@@ -465,7 +459,7 @@ __device__ __forceinline__ void pencil_body(const PencilArgs<T> &a, const int ti
     // X2: forward stage B -> X[k1 + R1 k2]; then g and inverse stage B, or |X|^2.
     // The h modes see the forward transform of their input at real-space x =
     // k1 + R1 k2 (the chain that uses them is written out at
-    // enqueue_chain_launches); INIT_W starts from h at those points.
+    // enqueue_transform_chain); INIT_W starts from h at those points.
     for (int t = threadIdx.x; t < CW * R1; t += C::NT) {
         const int cl = t % CW, k1 = t / CW, col = col0 + cl;
         if (col >= ncol) continue;

@@ -6,7 +6,7 @@
 // through a full complex 3-D transform: FFT(Z) = FFT(q) + i FFT(q^), the
 // product with g keeps that split, and after the inverse transform Re Z is
 // chain 1 and Im Z is chain 2 (each then multiplied by its own h).  Compared
-// with two half-spectrum real transforms (plane_kernel) this removes the
+// with two half-spectrum real transforms this removes the
 // row-pair packing/unpacking and the packed Nyquist column, at the same FFT
 // count.  A 128x128 complex FP32 plane (139 KB with padding) fits one CTA.
 //
@@ -279,7 +279,7 @@ __device__ __forceinline__ void pc_z_invB_h(cpx<T> *P, const cpx<T> *twb, const 
     }
 }
 
-// twiddle tables: twy[NY], TA, TB (as in plane_kernel)
+// twiddle tables: twy[NY], TA, TB
 template <typename C, typename T>
 struct PcTw {
     static constexpr int NY = C::RY1 * C::RY2, NZ = C::RZ1 * C::RZ2;
@@ -340,7 +340,7 @@ __device__ __forceinline__ void plane_c_body(const PlaneArgs<T> &a, const int x,
     tws.load(a.twy, a.twz);
     pdl_wait();
 
-    if (MODE == PLANE_INIT_W || MODE == PLANE_INIT_Q) {
+    if (MODE == PLANE_INIT_W) {
         tws.store(twy);
         int r0, nr;
         warp_rows<C>(threadIdx.x >> 5, r0, nr);
@@ -349,20 +349,11 @@ __device__ __forceinline__ void plane_c_body(const PlaneArgs<T> &a, const int x,
         for (int t = lane; t < nr * NZ; t += 32) {
             const int y = r0 + t / NZ, z = t % NZ;
             const long long i = plane_off + (long long)y * NZ + z;
-            T v1, v2;
-            if (MODE == PLANE_INIT_W) {
-                // hA = exp(-(W- + w+)/N), hB = exp(-(-W- + w+)/N)  (src/diblock.cc:64-72)
-                const double wm = a.w[i], wp = a.w[M + i];
-                v1 = (T)exp(-(wm + wp) / a.Nd);
-                v2 = (T)exp(-(-wm + wp) / a.Nd);
-                reinterpret_cast<cpx<T> *>(a.qout)[i] = {v1, v2};
-            } else if (a.src) {
-                v1 = a.src[i];
-                v2 = a.src[a.src_stride + i];
-            } else {
-                v1 = (T)a.src64[i];
-                v2 = (T)a.src64[a.src_stride + i];
-            }
+            // hA = exp(-(W- + w+)/N), hB = exp(-(-W- + w+)/N)  (src/diblock.cc:64-72)
+            const double wm = a.w[i], wp = a.w[M + i];
+            const T v1 = (T)exp(-(wm + wp) / a.Nd);
+            const T v2 = (T)exp(-(-wm + wp) / a.Nd);
+            reinterpret_cast<cpx<T> *>(a.qout)[i] = {v1, v2};
             P[y * KP + C::zpos(z)] = {v1, v2};
         }
         __syncthreads();  // twiddle tables (and rows)

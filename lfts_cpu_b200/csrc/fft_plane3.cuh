@@ -257,8 +257,8 @@ __device__ __forceinline__ void p3_s3(cpx<float> *P, const PlaneArgs<float> &a, 
     }
 }
 
-// INIT: real rows from global (h from the fields, or given rows), forward S3
-template <typename C, int MODE>
+// INIT_W: real rows h from the fields, forward S3
+template <typename C>
 __device__ __forceinline__ void p3_s3_init(cpx<float> *P, const PlaneArgs<float> &a, long long plane_off, long long M)
 {
     constexpr int NZ = C::NZ, Z1 = C::Z1, Z2 = C::Z2;
@@ -272,21 +272,12 @@ __device__ __forceinline__ void p3_s3_init(cpx<float> *P, const PlaneArgs<float>
 #pragma unroll
         for (int c2 = 0; c2 < Z2; c2++) {
             const long long i = plane_off + y * NZ + c1 + Z1 * c2;
-            float v1, v2;
-            if (MODE == PLANE_INIT_W) {
-                // hA = exp(-(W- + w+)/N), hB = exp(-(-W- + w+)/N)  (src/diblock.cc:64-72)
-                // (single-precision exponential: h is stored in FP32)
-                const double wm = a.w[i], wp = a.w[M + i];
-                v1 = expf((float)(-(wm + wp) / a.Nd));
-                v2 = expf((float)(-(-wm + wp) / a.Nd));
-                reinterpret_cast<cpx<float> *>(a.qout)[i] = {v1, v2};
-            } else if (a.src) {
-                v1 = a.src[i];
-                v2 = a.src[a.src_stride + i];
-            } else {
-                v1 = (float)a.src64[i];
-                v2 = (float)a.src64[a.src_stride + i];
-            }
+            // hA = exp(-(W- + w+)/N), hB = exp(-(-W- + w+)/N)  (src/diblock.cc:64-72)
+            // (single-precision exponential: h is stored in FP32)
+            const double wm = a.w[i], wp = a.w[M + i];
+            const float v1 = expf((float)(-(wm + wp) / a.Nd));
+            const float v2 = expf((float)(-(-wm + wp) / a.Nd));
+            reinterpret_cast<cpx<float> *>(a.qout)[i] = {v1, v2};
             g[c2] = {v1, v2};
         }
         Dft<Z2, -1, float>::run(g);
@@ -329,8 +320,8 @@ __device__ __forceinline__ void plane3_body(const PlaneArgs<float> &a, const int
     }
     pdl_wait();
 
-    if (MODE == PLANE_INIT_W || MODE == PLANE_INIT_Q) {
-        p3_s3_init<C, MODE>(P, a, plane_off, M);
+    if (MODE == PLANE_INIT_W) {
+        p3_s3_init<C>(P, a, plane_off, M);
         __syncthreads();
         p3_s2_fwd<C>(P, TY, TZ);
         __syncthreads();

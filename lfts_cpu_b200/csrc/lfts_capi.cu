@@ -317,7 +317,6 @@ PlaneArgs<float> plane_args(lfts_ctx *c)
     a.twy = static_cast<const cpx<float> *>(c->tw[1]);
     a.twz = static_cast<const cpx<float> *>(c->tw[2]);
     a.qpart = c->qpart;
-    a.nchains = 2;
     a.Nd = (double)c->N;
     a.gx = static_cast<const float *>(c->gtab[0]);
     a.gy = static_cast<const float *>(c->gtab[1]);
@@ -1845,8 +1844,15 @@ int lfts_backward(lfts_ctx *c, int ckpt_every, double *dH_dL, double *dH_dXbN, d
     const int nblk = (c->my * c->KZ + c->adj.cw - 1) / c->adj.cw;
     if (!c->adj_spec) {
         // terms per launch: about four CTAs per SM of 2 mx planes a term
+        // (one, if the device has no room for more)
         c->adj_batch = std::max(1, std::min(kFwdBatch, (4 * c->sms + 2 * c->mx - 1) / (2 * c->mx)));
-        CK(cudaMalloc(&c->adj_spec, sizeof(cpx<double>) * 2 * (size_t)c->Mk * c->adj_batch));
+        const size_t term = sizeof(cpx<double>) * 2 * (size_t)c->Mk;
+        if (cudaMalloc(&c->adj_spec, term * c->adj_batch) != cudaSuccess) {
+            cudaGetLastError();
+            c->adj_spec = nullptr;
+            c->adj_batch = 1;
+            CK(cudaMalloc(&c->adj_spec, term));
+        }
     }
     const int nrows = nblk * c->adj_batch;
     if (!c->adj_partial) CK(cudaMalloc(&c->adj_partial, sizeof(double) * 3 * nrows));
@@ -1862,23 +1868,28 @@ int lfts_backward(lfts_ctx *c, int ckpt_every, double *dH_dL, double *dH_dXbN, d
         for (int i = 1; i < N; i++) terms.add(q + (long long)(i - 1) * 2 * M, qh(i + 1));
     } else {
         const int K = std::min(ckpt_every, N);
-        const int slots = 1 + K < N ? 2 * K : K;  // one segment: no second one beside it
-        if (c->adj_buf_slots < slots) {
+        int segs = 1 + K < N ? 2 : 1;  // segments side by side; one alone if there is no second or no room
+        if (c->adj_buf_slots < segs * K) {
             cudaFree(c->adj_buf);
             c->adj_buf = nullptr;
             c->adj_buf_slots = 0;
-            CK(cudaMalloc(&c->adj_buf, sizeof(double) * (size_t)slots * M));
-            c->adj_buf_slots = slots;
+            if (segs == 2 && cudaMalloc(&c->adj_buf, sizeof(double) * 2 * (size_t)K * M) != cudaSuccess) {
+                cudaGetLastError();
+                c->adj_buf = nullptr;
+                segs = 1;
+            }
+            if (!c->adj_buf) CK(cudaMalloc(&c->adj_buf, sizeof(double) * (size_t)K * M));
+            c->adj_buf_slots = segs * K;
         }
         chain_checkpointed(c, K);
-        // two segments (terms i = c0 .. c0 + n) at a time
-        for (int c1 = 1; c1 < N; c1 += 2 * K) {
+        // `segs` segments (terms i = c0 .. c0 + n) at a time
+        for (int c1 = 1; c1 < N; c1 += segs * K) {
             int c0[2], n[2];
             const double *row0[2];
             double *rows[2];
             for (int s = 0; s < 2; s++) {
                 c0[s] = c1 + s * K;
-                n[s] = std::min(c0[s] + K - 1, N - 1) - c0[s];
+                n[s] = s < segs ? std::min(c0[s] + K - 1, N - 1) - c0[s] : -1;
                 row0[s] = q + (long long)(c0[s] - 1) * 2 * M;
                 rows[s] = c->adj_buf + (long long)s * K * M;
             }

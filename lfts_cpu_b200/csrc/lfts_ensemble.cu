@@ -48,8 +48,8 @@ using PlaneFn = void (*)(EnsRep *, const int *, int);
 using PencilFn = void (*)(EnsRep *, const int *);
 
 struct PlaneSet {
-    PlaneFn fn[4];
-    int nt[4];
+    PlaneFn fn[3];  // PLANE_INIT_W, PLANE_STEP, PLANE_LAST
+    int nt[3];
     size_t smem;
 };
 struct PencilSet {
@@ -66,10 +66,9 @@ void fill_plane(PlaneSet *o)
 {
     using C = PlaneCCfg<float, N, N>;
     o->fn[PLANE_INIT_W] = ens_plane_kernel<N, N, PLANE_INIT_W>;
-    o->fn[PLANE_INIT_Q] = nullptr;
     o->fn[PLANE_STEP] = ens_plane_kernel<N, N, PLANE_STEP>;
     o->fn[PLANE_LAST] = ens_plane_kernel<N, N, PLANE_LAST>;
-    for (int m = 0; m < 4; m++) o->nt[m] = C::NT;
+    for (int m = 0; m < 3; m++) o->nt[m] = C::NT;
     o->smem = C::SMEM;
 }
 
@@ -87,10 +86,9 @@ template <typename C3, typename CL = C3>
 void fill_plane3(PlaneSet *o)
 {
     o->fn[PLANE_INIT_W] = ens_plane3_kernel<C3, PLANE_INIT_W>;
-    o->fn[PLANE_INIT_Q] = nullptr;
     o->fn[PLANE_STEP] = ens_plane3_kernel<C3, PLANE_STEP>;
     o->fn[PLANE_LAST] = ens_plane3_kernel<CL, PLANE_LAST>;
-    for (int m = 0; m < 4; m++) o->nt[m] = m == PLANE_LAST ? CL::NT : C3::NT;
+    for (int m = 0; m < 3; m++) o->nt[m] = m == PLANE_LAST ? CL::NT : C3::NT;
     o->smem = C3::SMEM;
 }
 
@@ -256,7 +254,7 @@ void launch_after(bool overlap, void (*fn)(Args...), dim3 grid, int nt, size_t s
 }
 
 // one contour chain of every member of group g, on g.st; returns the launches.
-// Two chain orders, as a single context's (enqueue_chain_launches):
+// Two chain orders, as a single context's (enqueue_transform_chain):
 //   h in the plane: INIT_W plane, N-1 x (x-pencil with g, plane with h storing slot i+1)
 //   h in the pencil (96^3): INIT_W pencil, N-1 x (plane with g, pencil with h
 //     storing slot i+1 -- or, with the sums in the chain, adding the products
@@ -482,7 +480,7 @@ int ensure_graphs(lfts_ensemble *e, int maxIter, double tol)
 }
 
 // ---- batched tile choice ---------------------------------------------------------
-// Each mesh group's tiles (x-pencil width 8/16/32; yz-plane stages 3 or 2 where
+// Each mesh group's tiles (x-pencil width 16 or 32; yz-plane stages 3 or 2 where
 // both exist; at 96^3 also the h-in-pencil chain, with or without the
 // concentration sums in it) are picked by timing the group's batched contour
 // chain and concentration pass, all its replicas active, on its own stream --
@@ -505,7 +503,7 @@ int set_group_tiles(Group &g, const GroupTiles &t)
     if (!ens_plane(g.my, g.mz, t.stages, g.several, &pl) || !ens_pencil(g.mx, t.cw, &pe)) return LFTS_ERR_UNSUPPORTED;
     if (t.phi && !t.xh) return LFTS_ERR_UNSUPPORTED;
     if (t.xh && (t.stages != 3 || !ens_pencil_x(g.mx, g.my, g.mz, t.cw, g.several, &px))) return LFTS_ERR_UNSUPPORTED;
-    for (int m = 0; m < 4; m++)
+    for (int m = 0; m < 3; m++)
         if (pl.fn[m]) EK(cudaFuncSetAttribute(pl.fn[m], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
     EK(cudaFuncSetAttribute(pe.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pe.smem));
     if (t.xh) {
@@ -781,7 +779,7 @@ int lfts_ensemble_create(const lfts_params *params, const unsigned long long *se
             cudaMemcpy(g.d_members, g.members.data(), sizeof(int) * g.members.size(), cudaMemcpyHostToDevice) !=
                 cudaSuccess)
             return fail(LFTS_ERR_CUDA);
-        for (int m = 0; m < 4; m++)
+        for (int m = 0; m < 3; m++)
             if (g.pl.fn[m] && cudaFuncSetAttribute(g.pl.fn[m], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.pl.smem) !=
                 cudaSuccess)
                 return fail(LFTS_ERR_CUDA);
