@@ -334,6 +334,26 @@ def run_precision(lfts, precision, steps, warmup, rank, device, torch, clocks=No
     return res
 
 
+def storing_chain_ms(lfts, tiles, device):
+    """ms of the default contour chain with the same tile width when it stores every slot."""
+    fixed = {"LFTS_AUTOTUNE": "0", "LFTS_PHI_IN_CHAIN": "0", "LFTS_PENCIL_CW": str(tiles["pencil_cw"])}
+    before = {k: os.environ.get(k) for k in fixed}
+    os.environ.update(fixed)
+    try:
+        s = lfts.System(CFG["N"], CFG["NA"], CFG["XN"], CFG["C"], CFG["dt"], CFG["m"], CFG["L"],
+                        precision=lfts.LFTS_FP32_MIXED, device=device)
+    finally:
+        for k, v in before.items():
+            if v is None:
+                del os.environ[k]
+            else:
+                os.environ[k] = v
+    s.set_fields(make_initial_fields(int(np.prod(CFG["m"])), CFG["field_seed"]))
+    ms = min(s.profile_chain()[2] for _ in range(3))
+    s.close()
+    return ms
+
+
 def time_calc_concs(s, torch, device, reps=5):
     """Mean ms of one calc_concs (contour chain, Q, concentrations) on the
     context's current fields: CUDA events on the context's stream around the
@@ -595,8 +615,9 @@ def main(argv=None):
     part_chain, part_conc, part_upd = fp32_sys.profile_iteration(5)
     tiles32 = fp32_sys.tiles()
     ms_calc = time_calc_concs(fp32_sys, torch, device)
-    # the yz-plane kernel split over a thread-block cluster (tile plane_split)
-    # against the tuned choice: chain of one calc_concs, CUDA events
+    # the 3-D transform chain, which set_tiles installs on an FP32-mixed context, with
+    # its yz-plane kernel split over a thread-block cluster (tile plane_split) and
+    # without: chain of one calc_concs, CUDA events
     split_alt = None
     alt = dict(tiles32, plane_split=8 if tiles32.get("plane_split", 1) == 1 else 1)
     try:
@@ -606,18 +627,16 @@ def main(argv=None):
         ms_tuned = min(fp32_sys.profile_iteration(3)[0] for _ in range(2))
         split_alt = {"tuned_plane_split": tiles32["plane_split"],
                      "chain_ms": {str(tiles32["plane_split"]): ms_tuned, str(alt["plane_split"]): ms_alt},
-                     "note": "contour chain of one calc_concs with one CTA per 128x128 x-plane (1) or the plane "
-                             "spread over an 8-CTA cluster (8); results bitwise equal"}
+                     "note": "contour chain of one calc_concs by 3-D transforms (set_tiles) with one CTA per 128x128 "
+                             "x-plane (1) or the plane spread over an 8-CTA cluster (8); results bitwise equal"}
     except lfts.LftsError:
-        fp32_sys.set_tiles(**tiles32)
+        pass
+    fp32_sys.close()
     # the contour step of a chain that stores every slot (the tuned chain may
     # form the concentration sums in its second half instead)
     ch_storing = None
     if tiles32.get("phi_in_chain"):
-        fp32_sys.set_tiles(**dict(tiles32, phi_in_chain=0))
-        ch_storing = min(fp32_sys.profile_chain()[2] for _ in range(3))
-        fp32_sys.set_tiles(**tiles32)
-    fp32_sys.close()
+        ch_storing = storing_chain_ms(lfts, tiles32, device)
     fp64 = run_precision(lfts, lfts.LFTS_FP64, args.steps, args.warmup, rank, device, torch, None)
     fp64_sys = fp64.pop("system")
     tiles64 = fp64_sys.tiles()
@@ -696,13 +715,13 @@ def main(argv=None):
                     "d2h_bytes_per_step": fp32["d2h_bytes_per_step"],
                     "steps": "the timed steps replayed from the same state and noise, noise read from pinned host memory",
                     "same_anderson_K": fp32["e2e_same_K"]},
-            "roofline": {"bound": "hbm", "kernel": "calc_concs: contour chain (yz-plane + x-pencil kernels, both "
+            "roofline": {"bound": "hbm", "kernel": "calc_concs: contour chain (x- and y-, z-line kernels, both "
                                                    "chains, FP32) + Q + concentrations, one graph replay",
                          "achieved": achieved_cc, "peak": peak, "unit": "GB/s", "frac": achieved_cc / peak,
                          "peak_kind": peak_kind, "traffic": traffic_cc,
                          "algorithmic_bytes_per_launch": W_cc_bytes, "ms_per_launch": ms_calc,
                          "unit_of_work": "one calc_concs, W_cc = 7 N M propagator words (4 B) + 6 M field words (8 B)"},
-            "roofline_contour_step": {"bound": "hbm", "kernel": "one contour step (yz-plane + x-pencil kernels)",
+            "roofline_contour_step": {"bound": "hbm", "kernel": "one contour step (x- and y-, z-line kernels)",
                                       "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                                       "peak_kind": peak_kind, "traffic": traffic,
                                       "algorithmic_bytes_per_launch": step_bytes, "ms_per_step": step_ms,
