@@ -154,3 +154,32 @@ def test_noalloc_step_in_a_captured_graph(native_lib):
         for c, half in ((0, 0), (1, 1)):  # step 2 of NA = 3, NB = 4
             ref = conv(qh[c * M:(c + 1) * M].reshape(m), g).ravel() * hh[half * M:(half + 1) * M]
             assert rel_err(got[c * M:(c + 1) * M], ref) < FP64_TOL
+
+
+@pytest.mark.parametrize("m", [(128, 12, 12), (96, 12, 20), (64, 20, 20), (48, 24, 16), (80, 16, 32), (40, 40, 40),
+                               (12, 32, 64), (20, 48, 48), (64, 64, 64), (32, 80, 80), (24, 96, 96), (8, 128, 128)])
+def test_fp32_chain_of_a_default_context(lfts, m, monkeypatch):
+    """FP32-mixed contexts above 16384 points run this chain until set_tiles is called."""
+    N, NA = 5, 2
+    L, M = box(m), int(np.prod(m))
+    w = np.random.default_rng(M).normal(0.0, 1.0, 2 * M)
+    g = weights(m, L, N)
+    hA, hB = (np.exp(-x / N).reshape(m) for x in (w[:M] + w[M:], w[M:] - w[:M]))
+    q = [hA]
+    for i in range(1, N):
+        q.append((hA if i < NA else hB) * conv(q[-1], g))
+    monkeypatch.setenv("LFTS_AUTOTUNE", "0")
+    monkeypatch.setenv("LFTS_PHI_IN_CHAIN", "0")
+    first = None
+    for cw in (8, 16, 32):
+        monkeypatch.setenv("LFTS_PENCIL_CW", str(cw))
+        s = lfts.System(N, NA, 15.0, 50.0, 0.5, m, L, precision=1)
+        assert s.tiles()["pencil_cw"] == cw
+        s.set_fields(w)
+        lnq, p = s.calc_concs(), s.propagators()
+        s.close()
+        assert abs(lnq - np.log(q[-1].mean())) < FP32_TOL * max(1.0, abs(lnq))
+        for i in range(1, N + 1):
+            assert rel_err(p[i, 0], q[i - 1].ravel()) < FP32_TOL, (cw, i)
+        first = first or (lnq, p)
+        assert lnq == first[0] and np.array_equal(p, first[1]), cw
