@@ -64,7 +64,7 @@ struct lfts_ctx {
 
     void *sf_buf = nullptr;    // step_fwd scratch: q_in, q_out, h (2M each, FP64)
     double *adj_partial = nullptr;  // adjoint block partials [term][blocks][3]
-    void *adj_spec = nullptr;       // half spectra of the terms of one launch
+    void *adj_spec = nullptr;       // half spectra of the terms of one launch (null: one, in `field`)
     int adj_batch = 0;              // those terms
     double *adj_buf = nullptr;      // checkpointed adjoint: two recomputed q segments
     int adj_buf_slots = 0;

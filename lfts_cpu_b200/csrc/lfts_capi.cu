@@ -1431,6 +1431,41 @@ void adjoint_terms(lfts_ctx *c, const FwdArgs &f, int n)
     c->launches += 2;
 }
 
+// Device scratch of lfts_backward: K rows a segment for the recomputed propagators
+// (K = 0: all are stored), the spectra of the terms of one launch, their partial
+// sums.  The rows come first, since nothing else can stand in for them, and the
+// spectra give way to them; without room for spectra of their own one term at a
+// time goes through the chain's field, which is free between the chain and the
+// next recomputed segments.
+int adjoint_scratch(lfts_ctx *c, int nblk, int K, int *segs)
+{
+    auto try_alloc = [](auto **p, size_t bytes) {
+        if (cudaMalloc(reinterpret_cast<void **>(p), bytes) == cudaSuccess) return true;
+        cudaGetLastError();
+        *p = nullptr;
+        return false;
+    };
+    if (c->adj_buf_slots < *segs * K) {
+        const size_t row = sizeof(double) * (size_t)c->M;
+        cudaFree(c->adj_buf);
+        c->adj_buf = nullptr;
+        c->adj_buf_slots = 0;
+        if (*segs == 2 && !try_alloc(&c->adj_buf, 2 * K * row)) *segs = 1;
+        if (!c->adj_buf && !try_alloc(&c->adj_buf, K * row)) {
+            cudaFree(c->adj_spec);
+            c->adj_spec = nullptr;
+            CK(cudaMalloc(&c->adj_buf, K * row));
+        }
+        c->adj_buf_slots = *segs * K;
+    }
+    // terms per launch: about four CTAs per SM of 2 mx planes a term
+    const int batch = std::max(1, std::min(kFwdBatch, (4 * c->sms + 2 * c->mx - 1) / (2 * c->mx)));
+    if (!c->adj_partial) CK(cudaMalloc(&c->adj_partial, sizeof(double) * 3 * nblk * batch));
+    if (!c->adj_spec) try_alloc(&c->adj_spec, sizeof(cpx<double>) * 2 * (size_t)c->Mk * batch);
+    c->adj_batch = c->adj_spec ? batch : 1;
+    return LFTS_OK;
+}
+
 // Terms given one by one, launched c->adj_batch at a time
 struct AdjointBatch {
     lfts_ctx *c;
@@ -1438,7 +1473,7 @@ struct AdjointBatch {
     int n = 0;
     explicit AdjointBatch(lfts_ctx *ctx) : c(ctx)
     {
-        f.spec = static_cast<cpx<double> *>(c->adj_spec);
+        f.spec = static_cast<cpx<double> *>(c->adj_spec ? c->adj_spec : c->field);
         f.twy = static_cast<const cpx<double> *>(c->tw[1]);
         f.twz = static_cast<const cpx<double> *>(c->tw[2]);
     }
@@ -1848,45 +1883,22 @@ int lfts_backward(lfts_ctx *c, int ckpt_every, double *dH_dL, double *dH_dXbN, d
     CK(cudaFuncSetAttribute(c->adj.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->adj.smem));
     const long long M = c->M;
     const int nblk = (c->my * c->KZ + c->adj.cw - 1) / c->adj.cw;
-    if (!c->adj_spec) {
-        // terms per launch: about four CTAs per SM of 2 mx planes a term
-        // (one, if the device has no room for more)
-        c->adj_batch = std::max(1, std::min(kFwdBatch, (4 * c->sms + 2 * c->mx - 1) / (2 * c->mx)));
-        const size_t term = sizeof(cpx<double>) * 2 * (size_t)c->Mk;
-        if (cudaMalloc(&c->adj_spec, term * c->adj_batch) != cudaSuccess) {
-            cudaGetLastError();
-            c->adj_spec = nullptr;
-            c->adj_batch = 1;
-            CK(cudaMalloc(&c->adj_spec, term));
-        }
-    }
+    const int K = std::min(ckpt_every, c->N);
+    int segs = 1 + K < c->N ? 2 : 1;  // segments side by side; one alone if there is no second or no room
+    int rc = adjoint_scratch(c, nblk, K, &segs);
+    if (rc) return rc;
+    CK(cudaMemsetAsync(c->adj_partial, 0, sizeof(double) * 3 * nblk * c->adj_batch, c->st));
     const int nrows = nblk * c->adj_batch;
-    if (!c->adj_partial) CK(cudaMalloc(&c->adj_partial, sizeof(double) * 3 * nrows));
-    CK(cudaMemsetAsync(c->adj_partial, 0, sizeof(double) * 3 * nrows, c->st));
     double *q = static_cast<double *>(c->q);
     const int N = c->N;
     // q_i is the first half of slot i, q^_{i+1} the second half of slot N-i
     auto qh = [&](int i1) { return q + (long long)(N - i1) * 2 * M + M; };  // q^_{i1}
     AdjointBatch terms(c);
-    if (ckpt_every == 0) {
-        int rc = calc_concs_sync(c, nullptr);
+    if (K == 0) {
+        rc = calc_concs_sync(c, nullptr);
         if (rc) return rc;
         for (int i = 1; i < N; i++) terms.add(q + (long long)(i - 1) * 2 * M, qh(i + 1));
     } else {
-        const int K = std::min(ckpt_every, N);
-        int segs = 1 + K < N ? 2 : 1;  // segments side by side; one alone if there is no second or no room
-        if (c->adj_buf_slots < segs * K) {
-            cudaFree(c->adj_buf);
-            c->adj_buf = nullptr;
-            c->adj_buf_slots = 0;
-            if (segs == 2 && cudaMalloc(&c->adj_buf, sizeof(double) * 2 * (size_t)K * M) != cudaSuccess) {
-                cudaGetLastError();
-                c->adj_buf = nullptr;
-                segs = 1;
-            }
-            if (!c->adj_buf) CK(cudaMalloc(&c->adj_buf, sizeof(double) * (size_t)K * M));
-            c->adj_buf_slots = segs * K;
-        }
         chain_checkpointed(c, K);
         // `segs` segments (terms i = c0 .. c0 + n) at a time
         for (int c1 = 1; c1 < N; c1 += segs * K) {
