@@ -24,7 +24,7 @@ namespace lfts {
 struct AdjArgs {
     const cpx<double> *spec;  // per term: chain 0 at spec, chain 1 at spec + mx*ncol
     const cpx<double> *twx;
-    const double *gx, *gy, *gz;  // factorised g (1/M in gz)
+    const double *gx, *gy, *gz;  // factorised g (1/M in the product)
     int ncol, KZ, mx, my, mz;
     double *partial;  // [term][gridDim.x][3], accumulated over launches
 };

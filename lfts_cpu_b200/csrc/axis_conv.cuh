@@ -48,11 +48,23 @@ enum AxisMode : int {
 };
 constexpr int kAxisModes = 8;
 
+// The share of 1/M in an axis's weights: the largest power of two up to its length on
+// x and y, the rest on z, so that every convolution leaves values of the size that it
+// found.  With all of it on z an FP32 field was 1/(mx my) of itself between the axes,
+// and propagators below exp(-80) lost digits there (128^3, w+ shifted by 86: q_N 8.4e-5
+// off, 5.8e-7 so).  Powers of two change no other value.
+__host__ __device__ constexpr int axis_scale(int n)
+{
+    int s = 1;
+    while (2 * s <= n) s *= 2;
+    return s;
+}
+
 template <typename T>
 struct AxisArgs {
     T *S;                      // the field: FP32 M pairs (chain 1, chain 2); FP64 two fields of M
     const cpx<T> *twx, *twy, *twz;  // exp(-2 pi i t/n)
-    const T *gx, *gy, *gz;     // axis weights over signed wavenumbers, 1/M folded into gz
+    const T *gx, *gy, *gz;     // axis weights over signed wavenumbers, 1/M in their product (axis_scale)
     int mx, my, mz;
     int cbase;                 // chain of the grid's first chain index (FP64)
     long long M;
@@ -467,7 +479,7 @@ __device__ __forceinline__ void strided_body(const AxisArgs<T> &a, const int c, 
     const int tid = threadIdx.x, col0 = tile * CW;
     typename C::Tables tab{smem_raw + C::TILE};
     if constexpr (SELF)
-        tab.make(a.L[AXIS], (int)a.Nd, 1.0, tid, C::NT);
+        tab.make(a.L[AXIS], (int)a.Nd, (double)axis_scale(N), tid, C::NT);
     else
         tab.load(AXIS == 0 ? a.twx : a.twy, AXIS == 0 ? a.gx : a.gy, tid, C::NT);
     pdl_wait();
@@ -612,7 +624,7 @@ __device__ __forceinline__ void zline_body(const AxisArgs<T> &a, const int cta, 
     const int line0 = (cta * C::NW + wid) * C::LPW;
     typename C::Tables tab{smem_raw + C::TILE};
     if constexpr (SELF)
-        tab.make(a.L[2], (int)a.Nd, (double)a.M, threadIdx.x, C::NT);
+        tab.make(a.L[2], (int)a.Nd, (double)a.M / (axis_scale(a.mx) * axis_scale(a.my)), threadIdx.x, C::NT);
     else
         tab.load(a.twz, a.gz, threadIdx.x, C::NT);
     pdl_wait();
@@ -746,8 +758,8 @@ __device__ __forceinline__ void planeax_body(const AxisArgs<T> &a, const int x, 
     typename C::TabZ tabz{smem_raw + C::TILE + C::TabY::BYTES};
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     if constexpr (SELF) {
-        taby.make(a.L[1], (int)a.Nd, 1.0, threadIdx.x, C::NT);
-        tabz.make(a.L[2], (int)a.Nd, (double)a.M, threadIdx.x, C::NT);
+        taby.make(a.L[1], (int)a.Nd, (double)axis_scale(NY), threadIdx.x, C::NT);
+        tabz.make(a.L[2], (int)a.Nd, (double)a.M / (axis_scale(a.mx) * axis_scale(NY)), threadIdx.x, C::NT);
     } else {
         taby.load(a.twy, a.gy, threadIdx.x, C::NT);
         tabz.load(a.twz, a.gz, threadIdx.x, C::NT);

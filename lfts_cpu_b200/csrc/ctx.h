@@ -33,7 +33,7 @@ struct lfts_ctx {
     void *q = nullptr;         // N slots x 2M, slot i at (i-1)*2M
     void *field = nullptr;     // the contour chain's field (2M); half spectra of the adjoint and FP64 S(k)
     void *tw[3] = {};          // exp(-2 pi i t/m) per dimension
-    void *gtab[3] = {};        // gx[mx], gy[my], gz[KZ] (gz carries 1/M)
+    void *gtab[3] = {};        // gx[mx], gy[my], gz[mz], 1/M in the product
     double *qpart = nullptr;   // per-CTA sums of q_N
     unsigned *ticket = nullptr;  // CTAs of the chain's last kernel that are done
     double *Qd = nullptr;      // Q, ln Q

@@ -55,7 +55,7 @@ struct PlaneArgs {
     double *qpart;        // LAST: per-plane sums of chain 0
     int hsel0, hsel1;     // h half used by chain 0 / chain 1 (0 = hA, 1 = hB)
     double Nd;            // N as a double (h = exp(-w/N))
-    const T *gx, *gy, *gz;  // PLANE_G: separable Boltzmann weight, 1/M folded into gz
+    const T *gx, *gy, *gz;  // PLANE_G: separable Boltzmann weight, 1/M in the product
     const T *pf;          // PLANE_G: (chain 1, chain 2) slot that the next x-pencil reads, pulled into L2
     int pf_ctas;          // PLANE_G with pf: CTAs past the planes that pull pf into L2 (0: each plane CTA its plane)
 };
@@ -367,7 +367,7 @@ template <typename T>
 struct PencilArgs {
     cpx<T> *spec;             // chain c at spec + c*mx*ncol
     const cpx<T> *twx;        // exp(-2 pi i t/mx)
-    const T *gx, *gy, *gz;    // separable Boltzmann weight, 1/M folded into gz
+    const T *gx, *gy, *gz;    // separable Boltzmann weight, 1/M in the product
     double *S;                // POWER: accumulator (mx*ncol)
     int ncol;                 // my*KZ
     int KZ;

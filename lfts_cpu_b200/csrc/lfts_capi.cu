@@ -151,15 +151,15 @@ int upload_tables(lfts_ctx *c, void **tw, void **gt)
     }
     if (!gt) return LFTS_OK;
     // g = exp(-(2 pi)^2 (kx^2/Lx^2 + ky^2/Ly^2 + kz^2/Lz^2)/(6N)) / M, factorised;
-    // over each axis's signed wavenumbers
+    // over each axis's signed wavenumbers, 1/M shared out by axis_scale
+    const int sx = axis_scale(c->mx), sy = axis_scale(c->my);
+    const double share[3] = {(double)sx, (double)sy, (double)c->M / (sx * sy)};
     for (int d = 0; d < 3; d++) {
         std::vector<T> g(m[d]);
         for (int K = 0; K < m[d]; K++) {
             const int k = signed_k(K, m[d]);
             const double ksq = (double)k * k / (c->p.L[d] * c->p.L[d]);
-            double v = std::exp(-kTwoPi * kTwoPi * ksq / (6.0 * c->N));
-            if (d == 2) v /= (double)c->M;
-            g[K] = (T)v;
+            g[K] = (T)(std::exp(-kTwoPi * kTwoPi * ksq / (6.0 * c->N)) / share[d]);
         }
         CK(cudaMalloc(&gt[d], sizeof(T) * m[d]));
         CK(cudaMemcpy(gt[d], g.data(), sizeof(T) * m[d], cudaMemcpyHostToDevice));
