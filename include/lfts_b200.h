@@ -199,8 +199,9 @@ typedef struct lfts_tiles {
 } lfts_tiles;
 /* lfts_create picks the tiles by timing the whole contour chain for every
  * combination on the context's own buffers and keeping the fastest, once per
- * precision and mesh in a process (the counterpart of the reference's
- * FFTW_PATIENT planning, src/step.cc:15-16); lfts_get_tiles gives them, with
+ * precision, mesh, N (within a factor of two) and environment in a process (the
+ * counterpart of the reference's FFTW_PATIENT planning, src/step.cc:15-16);
+ * lfts_get_tiles gives them, with
  * plane_stages, h_in_pencil and plane_split of a transform chain that has such
  * tiles.  Environment: LFTS_AUTOTUNE=0 skips the timing (built-in choice);
  * LFTS_PENCIL_CW=8|16|32, LFTS_PHI_IN_CHAIN=0|1 and LFTS_ONE_STREAM=1 fix one
@@ -266,7 +267,7 @@ int lfts_ensemble_replica_status(const lfts_ensemble *ens, int r, int *status);
 int lfts_ensemble_tuning(const lfts_ensemble *ens, int r, int *pencil_cw);
 /* The tiles replica r computes with: picked per mesh group by timing the
  * group's batched contour chain (x-pencil width, yz-plane stages), once per
- * mesh, group size and N in a process.  A single FP32-mixed context given
+ * mesh, group size, N and environment in a process.  A single FP32-mixed context given
  * these tiles (lfts_set_tiles) computes exactly what the replica computes. */
 int lfts_ensemble_tiles(const lfts_ensemble *ens, int r, lfts_tiles *out);
 /* The CUDA stream the ensemble's graphs run on (a cudaStream_t). */

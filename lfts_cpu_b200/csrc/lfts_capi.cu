@@ -571,9 +571,10 @@ void enqueue_concs_any(lfts_ctx *c, void *Dh0, int nh, const HistPtrs &hist)
 //   two_streams   FP64: each chain on its own stream, or both chains per launch
 // autotune() times the whole chain for every combination on the context's own
 // buffers (a tile's cost depends on how it overlaps its neighbours in the chain,
-// so it is timed in place) and keeps the fastest, once per (precision, mesh) per
-// process -- the reference's analogue is planning its FFTs with FFTW_PATIENT
-// (src/step.cc:15-16).
+// so it is timed in place) and keeps the fastest, once per precision, mesh, chain
+// length within a factor of two (it decides how much of the slots stays in L2) and
+// candidates (which the environment restricts) per process -- the reference's
+// analogue is planning its FFTs with FFTW_PATIENT (src/step.cc:15-16).
 // lfts_set_tiles on an FP32-mixed context installs the transform chain instead,
 // whose choices change how values are rounded:
 //   plane_stages  yz-plane transform stages per axis: 3 (fft_plane3.cuh, 64 / 96 /
@@ -582,7 +583,7 @@ void enqueue_concs_any(lfts_ctx *c, void *Dh0, int nh, const HistPtrs &hist)
 //                 yz-plane kernel (96- and 128-point x lines, three-stage planes),
 //                 or both in the yz-plane kernel
 std::mutex g_tune_mu;
-std::map<std::tuple<int, int, int, int>, lfts_tiles> g_tuned;
+std::map<std::tuple<int, int, int, int, int, std::vector<int>>, lfts_tiles> g_tuned;
 
 // the captured chain and the Anderson-loop graph that holds it (rebuilt on
 // the next use with the new tiles)
@@ -797,7 +798,11 @@ int autotune(lfts_ctx *c)
     lfts_tiles t = default_tiles(c);
     const char *e = std::getenv("LFTS_AUTOTUNE");
     if (!(e && e[0] == '0')) {
-        const auto key = std::make_tuple(c->prec, c->mx, c->my, c->mz);
+        std::vector<int> cand;
+        for (const lfts_tiles &a : tile_candidates(c))
+            cand.insert(cand.end(), {a.pencil_cw, a.plane_stages, a.h_in_pencil, a.two_streams, a.phi_in_chain,
+                                     a.plane_split});
+        const auto key = std::make_tuple(c->prec, c->mx, c->my, c->mz, (int)std::log2(c->N), cand);
         std::lock_guard<std::mutex> lk(g_tune_mu);
         auto it = g_tuned.find(key);
         if (it != g_tuned.end()) {

@@ -493,7 +493,8 @@ struct GroupTiles {
     int cw, stages, xh, phi;
 };
 std::mutex g_ens_tune_mu;
-std::map<std::tuple<int, int, int, int, int>, GroupTiles> g_ens_tuned;
+// by mesh, replicas, chain length and candidates (which the environment restricts)
+std::map<std::tuple<int, int, int, int, int, std::vector<int>>, GroupTiles> g_ens_tuned;
 
 int set_group_tiles(Group &g, const GroupTiles &t)
 {
@@ -578,12 +579,14 @@ int tune_groups(lfts_ensemble *e)
     EK(cudaEventCreate(&e1));
     int rc = LFTS_OK;
     for (Group &g : e->groups) {
-        const auto key = std::make_tuple(g.mx, g.my, g.mz, (int)g.members.size(), e->N);
         const std::vector<GroupTiles> cand = group_candidates(g);
         if (cand.empty()) {
             rc = LFTS_ERR_UNSUPPORTED;
             break;
         }
+        std::vector<int> flat;
+        for (const GroupTiles &t : cand) flat.insert(flat.end(), {t.cw, t.stages, t.xh, t.phi});
+        const auto key = std::make_tuple(g.mx, g.my, g.mz, (int)g.members.size(), e->N, flat);
         // without timing: 16 columns (or the forced width), three stages where
         // they exist, h in the plane
         const char *fcw = std::getenv("LFTS_PENCIL_CW");
