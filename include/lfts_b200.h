@@ -205,7 +205,9 @@ typedef struct lfts_tiles {
  * plane_stages, h_in_pencil and plane_split of a transform chain that has such
  * tiles.  Environment: LFTS_AUTOTUNE=0 skips the timing (built-in choice);
  * LFTS_PENCIL_CW=8|16|32, LFTS_PHI_IN_CHAIN=0|1 and LFTS_ONE_STREAM=1 fix one
- * choice each, LFTS_XH_CHAIN=0 leaves the sums to the separate pass. */
+ * choice each; LFTS_XH_CHAIN=0|1 and LFTS_PLANE_SPLIT=8, on FP32-mixed meshes
+ * that have these choices, run the chain by 3-D transforms with h_in_pencil or
+ * plane_split so. */
 int lfts_get_tiles(const lfts_ctx *ctx, lfts_tiles *out);
 /* Installs a tile choice (LFTS_ERR_ARG / LFTS_ERR_UNSUPPORTED for an
  * invalid one), e.g. to make a context compute exactly what an ensemble

@@ -75,8 +75,9 @@ struct lfts_ctx {
     PlaneKernel fwd_yz{};      // FP64 forward transforms: S(k), the adjoint
     PencilKernel power_x{};
     lfts_tiles tiles{};        // the choice in use
-    // FP32: the chain by 3-D transforms, once lfts_set_tiles asked for it
-    bool transform_chain = false;
+    // FP32: the chain by 3-D transforms: in use (by default, or once lfts_set_tiles
+    // asked for it), and by default
+    bool transform_chain = false, default_transform = false;
     PlaneKernels<float> pl32{};
     PencilKernels<float> pe32{};
     int plane_split = 1;      // CTAs per x-plane of PLANE_G (8: the cluster kernel, fft_plane3c.cuh)

@@ -573,8 +573,8 @@ void enqueue_concs_any(lfts_ctx *c, void *Dh0, int nh, const HistPtrs &hist)
 // buffers (a tile's cost depends on how it overlaps its neighbours in the chain,
 // so it is timed in place) and keeps the fastest, once per precision, mesh, chain
 // length within a factor of two (it decides how much of the slots stays in L2) and
-// candidates (which the environment restricts) per process -- the reference's
-// analogue is planning its FFTs with FFTW_PATIENT (src/step.cc:15-16).
+// candidates (chain and tiles, which the environment restricts) per process -- the
+// reference's analogue is planning its FFTs with FFTW_PATIENT (src/step.cc:15-16).
 // lfts_set_tiles on an FP32-mixed context installs the transform chain instead,
 // whose choices change how values are rounded:
 //   plane_stages  yz-plane transform stages per axis: 3 (fft_plane3.cuh, 64 / 96 /
@@ -616,10 +616,25 @@ bool transform_by_default(const lfts_ctx *c)
            (c->M <= 16384 || (c->my == c->mz && ens(c->my) && (ens(c->mx) || c->mx == 64 || c->mx == 96)));
 }
 
+// square planes with a three-stage kernel
 bool has_three_stages(const lfts_ctx *c) { return c->my == c->mz && (c->my == 64 || c->my == 96 || c->my == 128); }
 bool has_h_in_pencil(const lfts_ctx *c)
 {
     return has_three_stages(c) && c->my != 64 && (c->mx == 96 || c->mx == 128);
+}
+bool has_plane_split(const lfts_ctx *c)
+{
+    PlaneSplitKernel ps{};
+    return has_h_in_pencil(c) && plane_split_kernel(c->my, c->mz, &ps) && ps.cl == 8;
+}
+
+// LFTS_XH_CHAIN=0|1 and LFTS_PLANE_SPLIT=8 name a layout of the transform chain: where
+// it has that layout, they select that chain
+bool transform_by_environment(const lfts_ctx *c)
+{
+    const char *split = std::getenv("LFTS_PLANE_SPLIT");
+    return c->prec == LFTS_FP32_MIXED && ((std::getenv("LFTS_XH_CHAIN") && has_h_in_pencil(c)) ||
+                                          (split && std::atoi(split) == 8 && has_plane_split(c)));
 }
 
 // the (A, B) concentration sums, FP32 pairs per mesh point
@@ -701,13 +716,13 @@ int apply_tiles(lfts_ctx *c, const lfts_tiles &t)
 // a choice of tile_candidates, for the chain that the context runs by default
 int apply_default_tiles(lfts_ctx *c, const lfts_tiles &t)
 {
-    return transform_by_default(c) ? apply_tiles(c, t) : apply_axis_tiles(c, t);
+    return c->default_transform ? apply_tiles(c, t) : apply_axis_tiles(c, t);
 }
 
 // every combination of the default chain, restricted by the environment
-// (LFTS_PENCIL_CW, LFTS_ONE_STREAM, LFTS_PHI_IN_CHAIN fix one choice each;
-// LFTS_XH_CHAIN=0 leaves the sums out).  plane_stages and h_in_pencil name the
-// transform chain that such a choice belongs to.
+// (LFTS_PENCIL_CW, LFTS_ONE_STREAM, LFTS_PHI_IN_CHAIN, and of the transform chain
+// LFTS_XH_CHAIN and LFTS_PLANE_SPLIT, fix one choice each).  For the axis-by-axis
+// chain plane_stages and h_in_pencil are those of a transform chain with such tiles.
 // The width that was the fastest on none of the cubic meshes is not tried: FP64 32
 // (64^3 460 us a call against 423, 128^3 2562 against 2223), FP32 8 (354 against 326,
 // 1405 against 1273); it costs a context's first creation as much as the others.
@@ -718,7 +733,9 @@ std::vector<lfts_tiles> tile_candidates(const lfts_ctx *c)
     const char *fxh = std::getenv("LFTS_XH_CHAIN");
     const char *fone = std::getenv("LFTS_ONE_STREAM");
     const char *fphi = std::getenv("LFTS_PHI_IN_CHAIN");
-    const int cw_forced = fcw ? std::atoi(fcw) : 0;
+    const char *fsplit = std::getenv("LFTS_PLANE_SPLIT");
+    const int cw_forced = fcw ? std::atoi(fcw) : 0, split_forced = fsplit ? std::atoi(fsplit) : 0;
+    const bool by_env = transform_by_environment(c);
     for (int cw : {8, 16, 32}) {
         if (cw_forced > 0 ? cw != cw_forced : cw == (c->prec == LFTS_FP64 ? 32 : 8)) continue;
         if (c->prec == LFTS_FP64) {
@@ -729,10 +746,19 @@ std::vector<lfts_tiles> tile_candidates(const lfts_ctx *c)
             continue;
         }
         const int xh = has_h_in_pencil(c) && !(fxh && fxh[0] == '0') ? 1 : 0;
-        for (int phi : {0, 1}) {
-            if (phi && !xh) continue;
-            if (fphi && xh && ((fphi[0] != '0') != (phi == 1))) continue;
-            out.push_back({cw, has_three_stages(c) ? 3 : 2, xh, 0, phi, 1});
+        const bool splits = by_env && xh && has_plane_split(c);
+        for (int stages : {3, 2}) {
+            // two stages where there are three: h in the plane kernel, as asked for
+            if (stages == 3 ? !has_three_stages(c) : has_three_stages(c) && !(by_env && !xh)) continue;
+            for (int phi : {0, 1}) {
+                if (phi && !xh) continue;
+                if (fphi && xh && ((fphi[0] != '0') != (phi == 1))) continue;
+                for (int split : {1, 8}) {
+                    if (split == 8 && !splits) continue;
+                    if (splits && split_forced > 0 && split != split_forced) continue;
+                    out.push_back({cw, stages, xh, 0, phi, split});
+                }
+            }
         }
     }
     return out;
@@ -802,6 +828,7 @@ int autotune(lfts_ctx *c)
         for (const lfts_tiles &a : tile_candidates(c))
             cand.insert(cand.end(), {a.pencil_cw, a.plane_stages, a.h_in_pencil, a.two_streams, a.phi_in_chain,
                                      a.plane_split});
+        cand.push_back(c->default_transform);
         const auto key = std::make_tuple(c->prec, c->mx, c->my, c->mz, (int)std::log2(c->N), cand);
         std::lock_guard<std::mutex> lk(g_tune_mu);
         auto it = g_tuned.find(key);
@@ -1637,6 +1664,7 @@ int lfts_create(const lfts_params *p, int precision, int device, lfts_ctx **out)
     }
     if (rc) return fail(rc);
     if (precision == LFTS_FP32_MIXED && (rc = set_axis<float>(c, kDefaultCwFp32))) return fail(rc);  // step_fwd
+    c->default_transform = transform_by_default(c) || transform_by_environment(c);
     if ((rc = autotune(c))) return fail(rc);
     *out = c;
     return LFTS_OK;
