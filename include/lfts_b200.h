@@ -176,10 +176,12 @@ int lfts_profile_chain(lfts_ctx *ctx, double *ms_plane, double *ms_pencil, doubl
 int lfts_profile_iteration(lfts_ctx *ctx, int reps, double *ms_chain, double *ms_concs, double *ms_update);
 /* Number of kernels this context has launched so far. */
 long long lfts_kernel_launches(const lfts_ctx *ctx);
-/* The free choices of a context's contour chain.  A context applies the bond
- * one axis at a time; lfts_create picks its pencil_cw, two_streams and
- * phi_in_chain by timing.  FP64: these change no value at all.  FP32-mixed: a
- * choice installed by lfts_set_tiles selects the chain by 3-D transforms, the
+/* The free choices of a context's contour chain.  FP64 contexts apply the bond
+ * one axis at a time, FP32-mixed ones too, except by 3-D transforms on meshes
+ * of up to 16384 points and on square yz planes of 16, 24, 32 or 48 points with
+ * 16, 24, 32, 48, 64 or 96 along x.  lfts_create picks pencil_cw, two_streams
+ * and phi_in_chain by timing.  FP64: these change no value at all.  FP32-mixed:
+ * a choice installed by lfts_set_tiles selects the chain by 3-D transforms, the
  * one that ensemble replicas run, with these tiles; its results agree with
  * the axis-by-axis chain's within that path's stated error. */
 typedef struct lfts_tiles {
@@ -211,8 +213,15 @@ typedef struct lfts_tiles {
 int lfts_get_tiles(const lfts_ctx *ctx, lfts_tiles *out);
 /* Installs a tile choice (LFTS_ERR_ARG / LFTS_ERR_UNSUPPORTED for an
  * invalid one), e.g. to make a context compute exactly what an ensemble
- * replica with those tiles computes. */
+ * replica with those tiles computes.  On an FP32-mixed context the choice is
+ * one of the chain by 3-D transforms, the tiles that lfts_get_tiles gives for
+ * the axis-by-axis chain included: lfts_reset_tiles takes the context back. */
 int lfts_set_tiles(lfts_ctx *ctx, const lfts_tiles *tiles);
+/* Installs the chain and the tiles that lfts_create picked. */
+int lfts_reset_tiles(lfts_ctx *ctx);
+/* 1 if the contour chain in use is the one by 3-D transforms, 0 if it applies
+ * the bond one axis at a time. */
+int lfts_chain_by_transforms(const lfts_ctx *ctx, int *by_transforms);
 /* pencil_cw and plane_stages of the current tiles */
 int lfts_tuning(const lfts_ctx *ctx, int *pencil_cw, int *plane_stages);
 /* Mean Anderson iteration count of all lfts_anderson_mix calls so far. */

@@ -236,6 +236,18 @@ class System:
                   int(plane_split))
         check(lib().lfts_set_tiles(self._h, C.byref(t)), "lfts_set_tiles")
 
+    def reset_tiles(self) -> None:
+        """back to the chain and the tiles that the system was created with (FP32-mixed:
+        set_tiles selects the chain by 3-D transforms)"""
+        check(lib().lfts_reset_tiles(self._h), "lfts_reset_tiles")
+
+    @property
+    def by_transforms(self) -> bool:
+        """whether the contour chain in use is the one by 3-D transforms"""
+        a = C.c_int()
+        check(lib().lfts_chain_by_transforms(self._h, C.byref(a)), "lfts_chain_by_transforms")
+        return bool(a.value)
+
     def profile_chain(self):
         """(ms per yz-plane step kernel, ms per x-pencil kernel, ms per chain)"""
         a, b, c = C.c_double(), C.c_double(), C.c_double()

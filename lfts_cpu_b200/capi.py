@@ -93,6 +93,8 @@ SIGNATURES = {
     "lfts_tuning": (C.c_int, [_P, C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     "lfts_get_tiles": (C.c_int, [_P, C.POINTER(Tiles)]),
     "lfts_set_tiles": (C.c_int, [_P, C.POINTER(Tiles)]),
+    "lfts_reset_tiles": (C.c_int, [_P]),
+    "lfts_chain_by_transforms": (C.c_int, [_P, C.POINTER(C.c_int)]),
     "lfts_ensemble_tiles": (C.c_int, [_P, C.c_int, C.POINTER(Tiles)]),
     "lfts_profile_chain": (C.c_int, [_P, C.POINTER(C.c_double), C.POINTER(C.c_double), C.POINTER(C.c_double)]),
     "lfts_profile_iteration": (C.c_int, [_P, C.c_int, C.POINTER(C.c_double), C.POINTER(C.c_double),

@@ -75,6 +75,7 @@ struct lfts_ctx {
     PlaneKernel fwd_yz{};      // FP64 forward transforms: S(k), the adjoint
     PencilKernel power_x{};
     lfts_tiles tiles{};        // the choice in use
+    lfts_tiles default_tiles{};  // lfts_create's
     // FP32: the chain by 3-D transforms: in use (by default, or once lfts_set_tiles
     // asked for it), and by default
     bool transform_chain = false, default_transform = false;

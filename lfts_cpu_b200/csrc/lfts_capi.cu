@@ -1666,6 +1666,7 @@ int lfts_create(const lfts_params *p, int precision, int device, lfts_ctx **out)
     if (precision == LFTS_FP32_MIXED && (rc = set_axis<float>(c, kDefaultCwFp32))) return fail(rc);  // step_fwd
     c->default_transform = transform_by_default(c) || transform_by_environment(c);
     if ((rc = autotune(c))) return fail(rc);
+    c->default_tiles = c->tiles;
     *out = c;
     return LFTS_OK;
 }
@@ -2060,6 +2061,22 @@ int lfts_set_tiles(lfts_ctx *c, const lfts_tiles *t)
     int rc = apply_tiles(c, *t);  // an invalid choice leaves the context as it was
     if (rc) g_last_error = "tile choice not valid for this context's precision and mesh";
     return rc;
+}
+
+int lfts_reset_tiles(lfts_ctx *c)
+{
+    if (!c) return LFTS_ERR_ARG;
+    DeviceGuard g(c->dev);
+    CK(cudaStreamSynchronize(c->st));
+    CK(cudaStreamSynchronize(c->st1));
+    return apply_default_tiles(c, c->default_tiles);
+}
+
+int lfts_chain_by_transforms(const lfts_ctx *c, int *by_transforms)
+{
+    if (!c || !by_transforms) return LFTS_ERR_ARG;
+    *by_transforms = c->transform_chain ? 1 : 0;
+    return LFTS_OK;
 }
 
 int lfts_tuning(const lfts_ctx *c, int *pencil_cw, int *plane_stages)
