@@ -432,6 +432,10 @@ __device__ __forceinline__ void pencil_body(const PencilArgs<T> &a, const int ti
         const int col = col0 + threadIdx.x % CW;
         if (col < ncol) gyz = a.gy[col / a.KZ] * a.gz[col % a.KZ];
     }
+    // With the sums the dependent goes out at once, as the plane kernel behind takes one CTA
+    // an SM: calc_concs with 16 columns, N = 64, 96^3 904 -> 896 us, 128^3 with split planes
+    // 1905 -> 1879; at 128^3 the two are level.
+    if (MODE == PENCIL_HA) pdl_launch_dependents();
     pdl_wait();
 
     // X1: forward stage A from global (strided rows), twiddles, to smem.  At
@@ -479,8 +483,10 @@ __device__ __forceinline__ void pencil_body(const PencilArgs<T> &a, const int ti
                 av[k2] = a.acc_init ? make_float2(0.f, 0.f) : ap[o];
             }
         }
-        // the (hA, hB) pairs (L2), for the same reason
-        constexpr bool kH = kAcc || MODE == PENCIL_H || MODE == PENCIL_H_LAST;
+        // the (hA, hB) pairs (L2), for the same reason; not beside the partner slot and the
+        // sums, where the registers they take cost CTAs (16 columns: 80 a thread and 96^3
+        // 993 us a calc_concs, 64 and 904 with h loaded where it is used; 128^3 1551 and 1504)
+        constexpr bool kH = MODE == PENCIL_H || MODE == PENCIL_H_LAST;
         float2 hv[kH ? R2 : 1];
         if constexpr (kH) {
 #pragma unroll
@@ -526,7 +532,7 @@ __device__ __forceinline__ void pencil_body(const PencilArgs<T> &a, const int ti
 #pragma unroll
             for (int k2 = 0; k2 < R2; k2++) {
                 const long long o = (long long)(k1 + R1 * k2) * ncol + col;
-                const float2 h = hv[k2];
+                const float2 h = __ldg(reinterpret_cast<const float2 *>(a.h) + o);
                 const float va = v[k2].x * (hs0 ? h.y : h.x);
                 const float vb = v[k2].y * (hs1 ? h.y : h.x);
                 if (MODE == PENCIL_HA_LAST) __stcs(reinterpret_cast<float2 *>(a.qout) + o, make_float2(va, vb));
@@ -574,7 +580,7 @@ __device__ __forceinline__ void pencil_body(const PencilArgs<T> &a, const int ti
     }
     if (MODE == PENCIL_POWER || MODE == PENCIL_H_LAST || MODE == PENCIL_HA_LAST) return;
     __syncthreads();
-    pdl_launch_dependents();
+    if (MODE != PENCIL_HA) pdl_launch_dependents();
 
     // X3: inverse stage A (strided) -> natural order, to global
     for (int t = threadIdx.x; t < CW * R2; t += C::NT) {
