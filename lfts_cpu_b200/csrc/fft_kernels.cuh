@@ -26,7 +26,8 @@
 
 namespace lfts {
 
-// Programmatic dependent launch: the contour chain's kernels (axis_conv.cuh) are
+// Programmatic dependent launch: the kernels of both contour chains (axis_conv.cuh;
+// here, fft_packed.cuh, fft_plane3.cuh, the ensemble's) and of the allocation-free step are
 // launched with programmatic stream serialisation, so a kernel's CTAs may start
 // while the previous kernel drains.  Each kernel loads its constant tables
 // first, then waits for the previous grid's results (griddepcontrol.wait) before

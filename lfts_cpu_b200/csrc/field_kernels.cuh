@@ -130,7 +130,9 @@ __device__ __forceinline__ void dot_partials(const double (&acc)[kRedWidth], int
 // serial chain of loads; split over up to 32 threads, the pass and its reduction
 // went from 18.7 to 12.4 us at 16^3, 39.5 to 31 at 48^3 (N = 64, ten history
 // vectors).  Where the mesh fills the grid one thread sums, in its own
-// instantiation: the split's shared memory cost 80^3 and larger meshes 1-2 %.
+// instantiation: the split's shared memory cost 80^3 and larger meshes 1-2 % of the pass
+// (the device-side Anderson loop has the split one for all: six iterations at 80^3 4477 us
+// against 4470, at 96^3 the same).
 // FP32-mixed sums stay with one thread: another order of the FP64 sum moved the
 // fields of a short ensemble run by 2.6e-5 through its replicas' Anderson loops.
 template <typename T>

@@ -603,7 +603,8 @@ void drop_chain_graph(lfts_ctx *c)
 // FP32-mixed meshes whose default chain is the one by transforms:
 //  * what an ensemble runs with one layout of it only, so that a replica computes
 //    what a context of its mesh does (16^3 ... 48^3: as replicas' Anderson loops
-//    amplify rounding, the ensemble keeps the arithmetic of its chain);
+//    amplify rounding, the ensemble keeps the arithmetic of its chain; 64^3 and 96^3 have
+//    several layouts there, and a context equals a replica only with set_tiles anyway);
 //  * meshes of up to 16384 points, where a Langevin step with a capped Anderson loop
 //    moves by up to 6e-5 with any change of rounding (20^3 3.6e-5, 80 x 12 x 12 5.9e-5;
 //    of 52 systems of 17 to 66 thousand points three moved by 2.3e-5 to 4.0e-5, the
