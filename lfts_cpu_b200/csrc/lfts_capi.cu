@@ -839,6 +839,8 @@ int autotune(lfts_ctx *c)
             int rc = tune_tiles(c, &t);
             if (rc) return rc;
             g_tuned[key] = t;
+            // the timed calls left their concentrations: back to a new context's
+            CK(cudaMemsetAsync(c->w + 2 * c->M, 0, sizeof(double) * 2 * c->M, c->st));
         }
     }
     return apply_default_tiles(c, t);

@@ -646,7 +646,11 @@ int tune_groups(lfts_ensemble *e)
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    return rc;
+    if (rc) return rc;
+    // the timed calls left their concentrations: back to a new replica's
+    for (const lfts_ctx *c : e->rep) EK(cudaMemsetAsync(c->w + 2 * c->M, 0, sizeof(double) * 2 * c->M, e->s0));
+    EK(cudaStreamSynchronize(e->s0));
+    return LFTS_OK;
 }
 
 int read_back(lfts_ensemble *e, int *k_out, double *lnQ_out)
